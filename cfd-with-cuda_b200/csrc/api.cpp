@@ -2473,9 +2473,8 @@ int cfd_unet_forward(cfd_unet* u, const int dims[3], const float* x, float* y, i
   if (rc) return rc;
   UnetNet& n = u->net;
   cudaStream_t s = n.own_stream;
-  DevBuf<float> tmp;
-  if (!on_device && tmp.alloc(2 * (size_t)nv)) return CFD_E_NOMEM;
-  rc = unet_load_input(u, x, nv, on_device, tmp.p);
+  if (!on_device && n.host_buffer(2 * nv)) return CFD_E_NOMEM;
+  rc = unet_load_input(u, x, nv, on_device, n.host_io);
   if (rc) return rc;
   // the output stays in the network's FP32 buffer too (cfd_unet_tensor)
   if (n.forward(s, nullptr) != cudaSuccess) return CFD_E_CUDA;
@@ -2515,11 +2514,10 @@ int cfd_unet_gradient(cfd_unet* u, const int dims[3], const float* x, const floa
   if (rc) return rc;
   UnetNet& n = u->net;
   cudaStream_t s = n.own_stream;
-  DevBuf<float> tmp;
-  if (!on_device && tmp.alloc(2 * (size_t)nv)) return CFD_E_NOMEM;
+  if (!on_device && n.host_buffer(2 * nv)) return CFD_E_NOMEM;
   if (cudaMemsetAsync(n.G, 0, n.nparam * sizeof(float), s) || cudaMemsetAsync(n.lossv, 0, sizeof(float), s))
     return CFD_E_CUDA;
-  rc = unet_sample(u, x, t, nv, on_device, tmp.p);
+  rc = unet_sample(u, x, t, nv, on_device, n.host_io);
   if (rc) return rc;
   if (cudaMemcpyAsync(n.h_pinned, n.lossv, sizeof(float), cudaMemcpyDeviceToHost, s)) return CFD_E_CUDA;
   if (grad && cudaMemcpyAsync(grad, n.G, n.nparam * sizeof(float), cudaMemcpyDeviceToHost, s)) return CFD_E_CUDA;
@@ -2585,12 +2583,11 @@ int cfd_unet_train_batch(cfd_unet* u, const int dims[3], int nb, const float* x,
   if (rc) return rc;
   UnetNet& n = u->net;
   cudaStream_t s = n.own_stream;
-  DevBuf<float> tmp;
-  if (!on_device && tmp.alloc(2 * (size_t)nv)) return CFD_E_NOMEM;
+  if (!on_device && n.host_buffer(2 * nv)) return CFD_E_NOMEM;
   if (cudaMemsetAsync(n.G, 0, n.nparam * sizeof(float), s) || cudaMemsetAsync(n.lossv, 0, sizeof(float), s))
     return CFD_E_CUDA;
   for (int i = 0; i < nb; i++) {
-    rc = unet_sample(u, x + (size_t)i * nv, t + (size_t)i * nv, nv, on_device, tmp.p);
+    rc = unet_sample(u, x + (size_t)i * nv, t + (size_t)i * nv, nv, on_device, n.host_io);
     if (rc) return rc;
   }
   if (n.adam(s, lr, 1.0f / nb) != cudaSuccess) return CFD_E_CUDA;

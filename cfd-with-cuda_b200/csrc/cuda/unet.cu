@@ -1,9 +1,9 @@
 // U-Net preconditioner kernels: 3x3x3 convolutions (stride 1 or 2) on
 // channels-last BF16 activations with BF16 weights and FP32 accumulation,
-// their data- and weight-gradients, vertex-centred prolongation and its
-// transpose, input scaling, MSE loss and Adam.  These are the training and
-// reference kernels; the inference hot path uses the tensor-core forward
-// convolution in unet_tc.cu where the layer shape allows.
+// vertex-centred prolongation and its transpose, input scaling, MSE loss and
+// Adam.  The forward convolutions here are the reference kernels; the hot path
+// uses the tensor-core forward convolution in unet_tc.cu where the layer
+// shape allows.  The data and weight gradients are in unet_bwd.cu.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -245,141 +245,6 @@ __global__ void __launch_bounds__(256) k_up_fwd_v(Dims3 g, const __nv_bfloat16* 
   }
 }
 
-// One thread per input voxel, CIB input channels per blockIdx.y chunk;
-// weights staged as [27][cout][CIB].
-template <int CIB>
-__global__ void __launch_bounds__(128) k_conv_dgrad(ConvDesc d, const float* __restrict__ dout, float* dA, int accA,
-                                                    float* dB, int accB) {
-  extern __shared__ float sw[];
-  const int cin = d.ca + d.cb, ci0 = blockIdx.y * CIB;
-  for (int i = threadIdx.x; i < 27 * d.cout * CIB; i += blockDim.x) {
-    const int c = i % CIB, co = (i / CIB) % d.cout, k = i / (CIB * d.cout);
-    sw[i] = (ci0 + c < cin) ? bf(d.w[((size_t)k * cin + ci0 + c) * d.cout + co]) : 0.f;
-  }
-  __syncthreads();
-  const long long nu = (long long)d.in_dims[0] * d.in_dims[1] * d.in_dims[2];
-  for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < nu;
-       u += (long long)gridDim.x * blockDim.x) {
-    int ix, iy, iz;
-    vox3(u, d.in_dims, ix, iy, iz);
-    float acc[CIB];
-#pragma unroll
-    for (int c = 0; c < CIB; c++) acc[c] = 0.f;
-    for (int k = 0; k < 27; k++) {
-      int X = ix - ((k % 3) - 1), Y = iy - ((k / 3) % 3 - 1), Z = iz - (k / 9 - 1);
-      if (d.stride == 2) {
-        if ((X | Y | Z) & 1) continue;
-        X >>= 1;
-        Y >>= 1;
-        Z >>= 1;
-      }
-      if (X < 0 || Y < 0 || Z < 0 || X >= d.out_dims[0] || Y >= d.out_dims[1] || Z >= d.out_dims[2]) continue;
-      const long long v = X + (long long)d.out_dims[0] * (Y + (long long)d.out_dims[1] * Z);
-      const float* g = dout + v * d.cout;
-      const float* wk = sw + (size_t)k * d.cout * CIB;
-      for (int co = 0; co < d.cout; co++) {
-        const float gv = g[co];
-#pragma unroll
-        for (int c = 0; c < CIB; c++) acc[c] += gv * wk[co * CIB + c];
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < CIB; c++) {
-      const int ci = ci0 + c;
-      if (ci >= cin) break;
-      if (ci < d.ca) {
-        if (dA) {
-          float* p = dA + u * d.ca + ci;
-          *p = accA ? *p + acc[c] : acc[c];
-        }
-      } else if (dB) {
-        float* p = dB + u * d.cb + (ci - d.ca);
-        *p = accB ? *p + acc[c] : acc[c];
-      }
-    }
-  }
-}
-
-// Weight gradient: blockIdx.x = voxel chunk, blockIdx.y = tap k, blockIdx.z =
-// input-channel chunk of CIB; a tile of TV output voxels of the input values
-// and output gradients is staged in shared memory; thread t accumulates the
-// (ci, co) pairs t, t + blockDim, ...; partial sums are added atomically.
-constexpr int kTV = 32;
-constexpr int kWgJ = 2;  // (ci, co) pairs per thread: CIB * cout <= kWgJ * 256
-template <int CIB>
-__global__ void __launch_bounds__(256) k_conv_wgrad(ConvDesc d, const float* __restrict__ dout, float* dw,
-                                                    long long vchunk) {
-  __shared__ float s_in[kTV][CIB];
-  extern __shared__ float s_g[];  // [kTV][cout]
-  const int cin = d.ca + d.cb, k = blockIdx.y, ci0 = blockIdx.z * CIB;
-  const long long nv = (long long)d.out_dims[0] * d.out_dims[1] * d.out_dims[2];
-  const long long v0 = blockIdx.x * vchunk, v1 = v0 + vchunk < nv ? v0 + vchunk : nv;
-  const int npair = CIB * d.cout;
-  float acc[kWgJ];
-#pragma unroll
-  for (int j = 0; j < kWgJ; j++) acc[j] = 0.f;
-  const int dx = (k % 3) - 1, dy = (k / 3) % 3 - 1, dz = k / 9 - 1;
-  for (long long t0 = v0; t0 < v1; t0 += kTV) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < kTV * CIB; i += blockDim.x) {
-      const int tv = i / CIB, c = i % CIB;
-      const long long v = t0 + tv;
-      float val = 0.f;
-      if (v < v1 && ci0 + c < cin) {
-        int X, Y, Z;
-        vox3(v, d.out_dims, X, Y, Z);
-        const int ix = X * d.stride + dx, iy = Y * d.stride + dy, iz = Z * d.stride + dz;
-        if (ix >= 0 && iy >= 0 && iz >= 0 && ix < d.in_dims[0] && iy < d.in_dims[1] && iz < d.in_dims[2]) {
-          const long long u = ix + (long long)d.in_dims[0] * (iy + (long long)d.in_dims[1] * iz);
-          const int ci = ci0 + c;
-          val = ci < d.ca ? bf(d.inA[u * d.ca + ci]) : bf(d.inB[u * d.cb + (ci - d.ca)]);
-        }
-      }
-      s_in[tv][c] = val;
-    }
-    for (int i = threadIdx.x; i < kTV * d.cout; i += blockDim.x) {
-      const int tv = i / d.cout, co = i % d.cout;
-      const long long v = t0 + tv;
-      s_g[i] = v < v1 ? dout[v * d.cout + co] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kWgJ; j++) {
-      const int pr = threadIdx.x + j * blockDim.x;
-      if (pr < npair) {
-        const int c = pr / d.cout, co = pr % d.cout;
-        float a = 0.f;
-#pragma unroll 8
-        for (int tv = 0; tv < kTV; tv++) a += s_in[tv][c] * s_g[tv * d.cout + co];
-        acc[j] += a;
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < kWgJ; j++) {
-    const int pr = threadIdx.x + j * blockDim.x;
-    if (pr < npair) {
-      const int c = pr / d.cout, co = pr % d.cout;
-      if (ci0 + c < cin) atomicAdd(dw + ((size_t)k * cin + ci0 + c) * d.cout + co, acc[j]);
-    }
-  }
-}
-
-__global__ void k_bias_grad(long long nv, int cout, const float* __restrict__ dout, float* db, long long vchunk) {
-  const long long v0 = blockIdx.x * vchunk, v1 = v0 + vchunk < nv ? v0 + vchunk : nv;
-  for (int co = threadIdx.x; co < cout; co += blockDim.x) {
-    float a = 0.f;
-    for (long long v = v0; v < v1; v++) a += dout[v * cout + co];
-    atomicAdd(db + co, a);
-  }
-}
-
-__global__ void k_act_bwd(long long n, const __nv_bfloat16* __restrict__ y, float* dy) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    if (bf(y[i]) <= 0.f) dy[i] *= kLeaky;
-}
-
-
 __global__ void k_up_fwd(Dims3 g, int ch, const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* skip,
                          __nv_bfloat16* out, const int* skipflag) {
   if (skipflag && *skipflag) return;
@@ -405,32 +270,27 @@ __global__ void k_up_fwd(Dims3 g, int ch, const __nv_bfloat16* __restrict__ in, 
   }
 }
 
-__global__ void k_up_bwd(Dims3 g, int ch, const float* __restrict__ dfine, float* dcoarse) {
-  const long long nc = (long long)g.c[0] * g.c[1] * g.c[2];
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nc * ch;
-       v += (long long)gridDim.x * blockDim.x) {
-    const long long cv = v / ch;
-    const int c = (int)(v % ch);
+// Four channels of a coarse voxel per thread: its 27 fine neighbours,
+// weight 1/2 per odd offset.
+__global__ void k_up_bwd(Dims3 g, int ch4, const float4* __restrict__ dfine, float4* dcoarse) {
+  const long long n = (long long)g.c[0] * g.c[1] * g.c[2] * ch4;
+  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)(v % ch4);
     int x, y, z;
-    vox3(cv, g.c, x, y, z);
-    float s = 0.f;
-    for (int dz = -1; dz <= 1; dz++) {
-      const int Z = 2 * z + dz;
-      if (Z < 0 || Z >= g.f[2]) continue;
-      const float wz = dz ? 0.5f : 1.f;
-      for (int dy = -1; dy <= 1; dy++) {
-        const int Y = 2 * y + dy;
-        if (Y < 0 || Y >= g.f[1]) continue;
-        const float wy = dy ? 0.5f : 1.f;
-        for (int dx = -1; dx <= 1; dx++) {
-          const int X = 2 * x + dx;
-          if (X < 0 || X >= g.f[0]) continue;
-          const float wx = dx ? 0.5f : 1.f;
-          s += wx * wy * wz * dfine[((long long)X + (long long)g.f[0] * (Y + (long long)g.f[1] * Z)) * ch + c];
-        }
-      }
+    vox3(v / ch4, g.c, x, y, z);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 27; k++) {
+      const int X = 2 * x + k % 3 - 1, Y = 2 * y + (k / 3) % 3 - 1, Z = 2 * z + k / 9 - 1;
+      if (X < 0 || Y < 0 || Z < 0 || X >= g.f[0] || Y >= g.f[1] || Z >= g.f[2]) continue;
+      const float w = (k % 3 == 1 ? 1.f : 0.5f) * ((k / 3) % 3 == 1 ? 1.f : 0.5f) * (k / 9 == 1 ? 1.f : 0.5f);
+      const float4 d = __ldg(dfine + (X + (long long)g.f[0] * (Y + (long long)g.f[1] * Z)) * ch4 + c);
+      s.x += w * d.x;
+      s.y += w * d.y;
+      s.z += w * d.z;
+      s.w += w * d.w;
     }
-    dcoarse[v] += s;
+    dcoarse[v] = s;
   }
 }
 
@@ -443,10 +303,6 @@ __global__ void k_input(int nv, const T* __restrict__ r, const int* __restrict__
   const float cf = (float)c;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += gridDim.x * blockDim.x)
     x[i] = __float2bfloat16((float)r[pmap ? pmap[i] : i] * cf);
-}
-__global__ void k_add(long long n, const float* __restrict__ a, float* b) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    b[i] += a[i];
 }
 
 __global__ void k_loss(Dims3 g, const float* __restrict__ out, const float* __restrict__ t, float* dout,
@@ -548,55 +404,6 @@ cudaError_t conv3_forward(const ConvDesc& d, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t conv3_dgrad(const ConvDesc& d, const float* dout, float* dA, int accA, float* dB, int accB,
-                        cudaStream_t s) {
-  const int cin = d.ca + d.cb;
-  const long long nu = (long long)d.in_dims[0] * d.in_dims[1] * d.in_dims[2];
-  const int gx = grid1(nu, 128);
-  if (d.cout <= 32) {
-    const size_t sm = (size_t)27 * d.cout * 16 * sizeof(float);
-    cudaError_t e = with_smem(k_conv_dgrad<16>, sm);
-    if (e != cudaSuccess) return e;
-    k_conv_dgrad<16><<<dim3(gx, (cin + 15) / 16), 128, sm, s>>>(d, dout, dA, accA, dB, accB);
-  } else {
-    const size_t sm = (size_t)27 * d.cout * 8 * sizeof(float);
-    cudaError_t e = with_smem(k_conv_dgrad<8>, sm);
-    if (e != cudaSuccess) return e;
-    k_conv_dgrad<8><<<dim3(gx, (cin + 7) / 8), 128, sm, s>>>(d, dout, dA, accA, dB, accB);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t conv3_wgrad(const ConvDesc& d, const float* dout, float* dw, float* db, cudaStream_t s) {
-  const int cin = d.ca + d.cb;
-  const long long nv = (long long)d.out_dims[0] * d.out_dims[1] * d.out_dims[2];
-  const long long vchunk = 2048;
-  const int nchunk = (int)((nv + vchunk - 1) / vchunk);
-  // CIB chosen so that CIB * cout <= kWgJ * 256
-  const size_t sm = (size_t)kTV * d.cout * sizeof(float);
-  if (d.cout <= 64) {
-    if (d.cout <= 32) {
-      k_conv_wgrad<16><<<dim3(nchunk, 27, (cin + 15) / 16), 256, sm, s>>>(d, dout, dw, vchunk);
-    } else {
-      k_conv_wgrad<8><<<dim3(nchunk, 27, (cin + 7) / 8), 256, sm, s>>>(d, dout, dw, vchunk);
-    }
-  } else {
-    return cudaErrorInvalidValue;
-  }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  if (db) {
-    const long long bchunk = 1024;
-    k_bias_grad<<<(int)((nv + bchunk - 1) / bchunk), 64, 0, s>>>(nv, d.cout, dout, db, bchunk);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t act_backward(long long n, const __nv_bfloat16* y, float* dy, cudaStream_t s) {
-  k_act_bwd<<<grid1(n), 256, 0, s>>>(n, y, dy);
-  return cudaGetLastError();
-}
-
 cudaError_t upsample_forward(const int* cdims, const int* fdims, int ch, const __nv_bfloat16* in,
                              const __nv_bfloat16* skip, __nv_bfloat16* out, const int* skipflag, cudaStream_t s) {
   Dims3 g;
@@ -624,13 +431,10 @@ cudaError_t upsample_backward(const int* cdims, const int* fdims, int ch, const 
     g.c[i] = cdims[i];
     g.f[i] = fdims[i];
   }
-  const long long n = (long long)cdims[0] * cdims[1] * cdims[2] * ch;
-  k_up_bwd<<<grid1(n), 256, 0, s>>>(g, ch, dfine, dcoarse);
-  return cudaGetLastError();
-}
-
-cudaError_t add_f32(long long n, const float* src, float* dst, cudaStream_t s) {
-  k_add<<<grid1(n), 256, 0, s>>>(n, src, dst);
+  if (ch % 4) return cudaErrorInvalidValue;
+  const long long n = (long long)cdims[0] * cdims[1] * cdims[2] * (ch / 4);
+  k_up_bwd<<<grid1(n), 256, 0, s>>>(g, ch / 4, reinterpret_cast<const float4*>(dfine),
+                                    reinterpret_cast<float4*>(dcoarse));
   return cudaGetLastError();
 }
 

@@ -35,26 +35,27 @@ struct ConvDesc {
 
 cudaError_t conv3_forward(const ConvDesc& d, cudaStream_t s);
 
-// dIn = conv^T(dOut, W): writes FP32 gradients of inA (dA, ca channels) and inB
-// (dB, cb channels); accumulate into existing values when acc* != 0.
-cudaError_t conv3_dgrad(const ConvDesc& d, const float* dout, float* dA, int accA, float* dB, int accB,
-                        cudaStream_t s);
-// dW[k][ci][co] += sum_v in[s v + off_k][ci] dOut[v][co],  db[co] += sum_v dOut[v][co]
-cudaError_t conv3_wgrad(const ConvDesc& d, const float* dout, float* dw, float* db, cudaStream_t s);
-
-// dy *= leaky'(y) (derivative from the sign of the stored output y)
-cudaError_t act_backward(long long n, const __nv_bfloat16* y, float* dy, cudaStream_t s);
+// Data gradient: dx = add + conv^T(dOut, W) in FP32 (add may be null), and
+// weight gradients dW[k][ci][co] += sum_v in[s v + off_k][ci] dOut[v][co],
+// db[co] += sum_v dOut[v][co] (unet_bwd.cu).  dOut is the gradient of the
+// stored output y when y is given (the leaky ReLU's derivative, from the
+// sign of y, is applied on the way in).  Layer shapes of the network only
+// (one input; cin and cout of 1, 16, 32 or 64 as listed in unet_net.h).
+cudaError_t conv3_dgrad(const ConvDesc& d, const float* dout, const __nv_bfloat16* y, const float* add, float* dx,
+                        int num_sms, cudaStream_t s);
+// work: conv3_wgrad_words(num_sms) floats for the blocks' partial sums (one
+// launch's contents at a time).
+long long conv3_wgrad_words(int num_sms);
+cudaError_t conv3_wgrad(const ConvDesc& d, const float* dout, const __nv_bfloat16* y, float* dw, float* db,
+                        float* work, int num_sms, cudaStream_t s);
 
 // out = P(in) + skip: vertex-centred trilinear prolongation from coarse dims c
 // to fine dims f = 2c - 1 (ch channels), plus an optional fine skip tensor.
 cudaError_t upsample_forward(const int* cdims, const int* fdims, int ch, const __nv_bfloat16* in,
                              const __nv_bfloat16* skip, __nv_bfloat16* out, const int* skipflag, cudaStream_t s);
-// transpose of upsample_forward: coarse gradient += R(fine gradient)
+// transpose of upsample_forward: coarse gradient = R(fine gradient), ch a multiple of 4
 cudaError_t upsample_backward(const int* cdims, const int* fdims, int ch, const float* dfine, float* dcoarse,
                               cudaStream_t s);
-
-// dst += src (FP32)
-cudaError_t add_f32(long long n, const float* src, float* dst, cudaStream_t s);
 
 // Network input x[v] = bf16(r[p(v)] * c), v over the nv grid voxels, p(v) =
 // p_of_vox[v] (identity when null).  c = sqrt(nv / rr[0]) when rr is given

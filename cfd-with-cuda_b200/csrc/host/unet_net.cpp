@@ -73,6 +73,8 @@ UnetNet::~UnetNet() {
   }
   cudaFree(out);
   cudaFree(lossv);
+  cudaFree(wg_work);
+  cudaFree(host_io);
   cudaFree(tc_err);
   for (int l = 0; l < kUnetConvs; l++) {
     cudaFree(wpack[l]);
@@ -165,11 +167,18 @@ int UnetNet::set_grid(const int d[3], bool train) {
   if (e == cudaSuccess) e = grow(out, out_cap, nvox[0], &gen);
   for (int t = 1; train && t < kUnetTensors && e == cudaSuccess; t++)
     e = grow(grad[t], gcap[t], nvox[kUnetTensor[t].level] * kUnetTensor[t].ch);
+  if (train && e == cudaSuccess) e = grow(wg_work, wg_cap, conv3_wgrad_words(num_sms));
   if (e != cudaSuccess) {
     err = std::string("U-Net activation allocation: ") + cudaGetErrorString(e);
     return -1;
   }
   return 0;
+}
+
+int UnetNet::host_buffer(long long n) {
+  if (grow(host_io, host_io_cap, n) == cudaSuccess) return 0;
+  err = "U-Net input allocation failed";
+  return -1;
 }
 
 namespace {
@@ -256,34 +265,29 @@ cudaError_t UnetNet::forward(cudaStream_t s, float* out_f32, const int* skip) {
 
 cudaError_t UnetNet::backward(cudaStream_t s) {
   cudaError_t e = cudaSuccess;
-  for (int t = 1; t < kUnetTensors - 1 && e == cudaSuccess; t++)
-    e = cudaMemsetAsync(grad[t], 0, (size_t)nvox[kUnetTensor[t].level] * kUnetTensor[t].ch * sizeof(float), s);
   for (int i = kUnetConvs + 1; i >= 0 && e == cudaSuccess; i--) {
     const int op = kOrder[i];
     if (op >= 0) {
       const UnetConvSpec& c = kUnetConv[op];
-      ConvDesc d = conv_desc(*this, op, out);
-      float* g = grad[c.out];
-      if (c.act) {
-        e = act_backward(nvox[kUnetTensor[c.out].level] * kUnetTensor[c.out].ch, act[c.out], g, s);
-        launches++;
-        if (e != cudaSuccess) break;
-      }
+      const ConvDesc d = conv_desc(*this, op, out);
+      const __nv_bfloat16* y = c.act ? act[c.out] : nullptr;
       if (c.in != 0) {
-        e = conv3_dgrad(d, g, grad[c.in], 1, nullptr, 0, s);
+        // a tensor that also feeds a skip connection gets that gradient too
+        const float* add = nullptr;
+        for (const UnetUpSpec& u : kUnetUp)
+          if (u.skip == c.in) add = grad[u.out];
+        e = conv3_dgrad(d, grad[c.out], y, add, grad[c.in], num_sms, s);
         launches++;
         if (e != cudaSuccess) break;
       }
-      e = conv3_wgrad(d, g, G + unet_weight_offset(op), G + unet_bias_offset(op), s);
-      launches += 2;
+      e = conv3_wgrad(d, grad[c.out], y, G + unet_weight_offset(op), G + unet_bias_offset(op), wg_work, num_sms, s);
+      launches++;  // with the sum of its records
     } else {
       const UnetUpSpec& u = kUnetUp[-1 - op];
-      const int lc = kUnetTensor[u.in].level, lf = kUnetTensor[u.out].level;
-      const int ch = kUnetTensor[u.out].ch;
-      e = upsample_backward(dims[lc], dims[lf], ch, grad[u.out], grad[u.in], s);
-      if (e == cudaSuccess) e = add_f32(nvox[lf] * ch, grad[u.out], grad[u.skip], s);
-      launches += 2;
+      e = upsample_backward(dims[kUnetTensor[u.in].level], dims[kUnetTensor[u.out].level], kUnetTensor[u.out].ch,
+                            grad[u.out], grad[u.in], s);
     }
+    launches++;
   }
   return e;
 }

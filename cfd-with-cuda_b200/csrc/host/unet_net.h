@@ -75,6 +75,10 @@ struct UnetNet {
   float* grad[kUnetTensors] = {};
   long long gcap[kUnetTensors] = {};
   float* lossv = nullptr;
+  float* wg_work = nullptr;  // partial sums of one layer's weight gradient
+  long long wg_cap = 0;
+  float* host_io = nullptr;  // device copies of host-side inputs and targets
+  long long host_io_cap = 0;
   float* h_pinned = nullptr;
   int gen = 0;  // bumped whenever an activation buffer moves
 
@@ -107,6 +111,8 @@ struct UnetNet {
   int get_params(float* h, long long n);
   // Sets the grid and (re)allocates activations; train != 0 also gradients.
   int set_grid(const int d[3], bool train);
+  // Room for n floats of host-side inputs on the device (kept).
+  int host_buffer(long long n);
   // Packs weights and builds plans for the tensor-core layers when needed.
   cudaError_t prepare_tc(cudaStream_t s);
   // Forward pass of the grid set by set_grid: act[0] must hold the input;
