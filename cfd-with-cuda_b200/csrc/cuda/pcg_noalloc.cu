@@ -7,26 +7,45 @@
 // application that reserves all of its device memory up front through its
 // own pool allocator cannot let a library allocate at solve time, where an
 // allocation could fail in the middle of a run.  Such callers own the matrix,
-// right-hand side and solution buffers and pass them in; the Krylov work
-// vectors, per-block partial sums, the barrier words and the result live in
+// right-hand side and solution buffers and pass them in; the published work
+// vector, per-block partial sums, the barrier words and the result live in
 // one file-scope static device array of fixed size.
 //
 // Limits and rules:
 //   - n <= CFD_NOALLOC_MAX_N (524288 rows, a 80^3 pressure grid); larger
 //     systems are rejected with CFD_E_BADARG and a message.
-//   - every GPU that loads this library holds the array (16.1 MiB) until the
+//   - every GPU that loads this library holds the array (4.1 MiB) until the
 //     process exits;
 //   - the first call on a device looks the array's device address up
 //     (cudaGetSymbolAddress, once per device, with that device current); make
 //     that first call before any stream capture;
 //   - all calls share the array and it keeps the last call's contents; the
 //     barrier words and the error flag are cleared on every call, the work
-//     vectors are fully rewritten before use.  Calls that overlap on the GPU
+//     vector is fully rewritten before use.  Calls that overlap on the GPU
 //     (two streams, or two host threads) race on the array and must not be
 //     issued.
 // The algorithm is the solver's FP64 Jacobi-PCG: x0 = 0, stop when
 // ||r||_2 <= rtol ||b||_2, one persistent cooperative kernel with bounded
 // grid barriers.
+//
+// The iteration is Chronopoulos and Gear's form of CG (1989; the same
+// iterates as the textbook form): with u = D^-1 r and w = A u, the step
+// lengths come from (r, u) and (w, u) of the same iteration, so one reduction
+// and one publication of u are the only grid-wide waits.  Everything but u
+// is used by the block that owns the rows only and stays in its shared
+// memory: r, p, s, w and x.
+//
+// What bounds it: the matrix stream (12 bytes per non-zero; up to about 9 M
+// non-zeros it stays in L2 between iterations) and the two waits.  One block
+// of 1024 threads per SM keeps the waits short (148 arrivals, 148 partial
+// sums).  A block owns a contiguous range of rows, so the gathers of u stay
+// in its L1; a row is summed by a group of G lanes, G chosen from the mean row
+// length so that a row takes about four loads per lane, all in flight at
+// once.  Measured on a 27-point operator with 65 x 63 x 61 rows (rtol 1e-8,
+// 273 iterations): 82 us per iteration with a warp per row, 1184 blocks, all
+// vectors in L2 and three waits; 34 us with the row groups and 148 blocks; 31
+// us in this form; 27 us with two rows per group at once and the row extents
+// read ahead.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -38,119 +57,236 @@
 namespace cfd {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 1024;
 constexpr int kMaxN = CFD_NOALLOC_MAX_N;
 constexpr int kMaxBlocks = 2048;
 constexpr int kMaxDevices = 64;
 // layout of the scratch array (bytes)
 constexpr size_t kVecBytes = (size_t)kMaxN * sizeof(double);
-constexpr size_t kOffR = 0, kOffZ = kVecBytes, kOffP = 2 * kVecBytes, kOffQ = 3 * kVecBytes;
-constexpr size_t kOffPart = 4 * kVecBytes;                                    // 6 x kMaxBlocks doubles
+constexpr size_t kOffU = 0;  // u; the other vectors live in shared memory
+constexpr size_t kOffPart = kVecBytes;                                    // 6 x kMaxBlocks doubles
 constexpr size_t kOffCtl = kOffPart + 6 * (size_t)kMaxBlocks * sizeof(double);  // barrier[2], err, pad
 constexpr size_t kOffRes = kOffCtl + 256;                                       // 4 doubles
 constexpr size_t kScratchBytes = kOffRes + 256;
+constexpr int kMaxDynSmem = 200 * 1024;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-template <int NV>
-__device__ __forceinline__ bool reduce_all(double (&v)[NV], double* part, int phase, unsigned* bar, int* err) {
-  __shared__ double res[NV];
-  const int G = gridDim.x;
-  double* buf = part + (size_t)(phase & 1) * 3 * G;
-  block_sum<NV>(v);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < NV; k++) buf[(size_t)k * G + blockIdx.x] = v[k];
-  if (!grid_barrier(bar, err, 2000000000ULL)) return false;
-  if (threadIdx.x < 32) {
-    for (int k = 0; k < NV; k++) {
-      double s = 0;
-      for (int i = threadIdx.x; i < G; i += 32) s += __ldcg(buf + (size_t)k * G + i);
-      s = warp_sum(s);
-      if (threadIdx.x == 0) res[k] = s;
+// Grid-wide wait number k (1, 2, ...) of the launch on a monotonic arrival
+// counter (host-zeroed): every block has arrived k times.  Returns false in
+// every thread of the block when the bounded wait gives up or another block
+// has raised *err.  With NV > 0 also sums NV values over the grid: v in, the
+// total out, every block adding the posted partials in the same order.
+struct GridSync {
+  unsigned* cnt;
+  int* err;
+  double* part;
+  unsigned k;
+  template <int NV>
+  __device__ __forceinline__ bool wait(double (&v)[NV > 0 ? NV : 1]) {
+    __shared__ double res[NV > 0 ? NV : 1];
+    __shared__ int s_ok;
+    const int G = gridDim.x;
+    if (G == 1) {  // one block: no one to wait for
+      if constexpr (NV > 0) {
+        block_sum<NV>(v);
+        if (threadIdx.x == 0)
+          for (int i = 0; i < NV; i++) res[i] = v[i];
+      }
+      __syncthreads();
+      if constexpr (NV > 0)
+        for (int i = 0; i < NV; i++) v[i] = res[i];
+      __syncthreads();
+      return true;
     }
-  }
-  __syncthreads();
-  for (int k = 0; k < NV; k++) v[k] = res[k];
-  __syncthreads();
-  return true;
-}
-
-__global__ void __launch_bounds__(kThreads) k_pcg_noalloc(int n, const int* __restrict__ rp,
-                                                           const int* __restrict__ col,
-                                                           const double* __restrict__ val,
-                                                           const double* __restrict__ dinv,
-                                                           const double* __restrict__ b, double* x, double rtol,
-                                                           int maxit, unsigned char* scratch) {
-  double* r = reinterpret_cast<double*>(scratch + kOffR);
-  double* z = reinterpret_cast<double*>(scratch + kOffZ);
-  double* p = reinterpret_cast<double*>(scratch + kOffP);
-  double* q = reinterpret_cast<double*>(scratch + kOffQ);
-  double* part = reinterpret_cast<double*>(scratch + kOffPart);
-  unsigned* bar = reinterpret_cast<unsigned*>(scratch + kOffCtl);
-  int* err = reinterpret_cast<int*>(scratch + kOffCtl + 8);
-  double* result = reinterpret_cast<double*>(scratch + kOffRes);
-  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  const long long gw = (long long)blockIdx.x * wpb + (threadIdx.x >> 5), nw = (long long)gridDim.x * wpb;
-  const int r0 = (int)(n * gw / nw), r1 = (int)(n * (gw + 1) / nw);
-  int phase = 0;
-  double v3[3] = {0, 0, 0};
-  for (int i = r0 + lane; i < r1; i += 32) {
-    double bi = b[i], zi = bi * dinv[i];
-    x[i] = 0.0;
-    r[i] = bi;
-    z[i] = zi;
-    p[i] = zi;
-    v3[0] += bi * bi;
-    v3[1] += bi * zi;
-    v3[2] += bi * bi;
-  }
-  bool alive = reduce_all<3>(v3, part, phase++, bar, err);
-  const double bnorm = sqrt(v3[0]);
-  double rz = v3[1], rn = sqrt(v3[2]);
-  const double tol = rtol * bnorm;
-  int its = 0, status = 1;
-  if (!alive) {
-    status = 3;
-  } else if (!isfinite(bnorm)) {
-    status = 2;
-  } else if (bnorm == 0.0 || rn <= tol) {
-    status = 0;
-  } else {
-    while (its < maxit) {
-      double pq = 0;
-      for (int i = r0; i < r1; i++) {
-        double s = 0;
-        for (int j = __ldg(rp + i) + lane; j < __ldg(rp + i + 1); j += 32) s += __ldg(val + j) * __ldcg(p + __ldg(col + j));
-        s = warp_sum(s);
-        if (lane == 0) {
-          q[i] = s;
-          pq += p[i] * s;
+    k++;
+    double* buf = part + (size_t)(k & 1) * 3 * G;
+    if constexpr (NV > 0) {
+      block_sum<NV>(v);
+      if (threadIdx.x == 0)
+        for (int i = 0; i < NV; i++) buf[(size_t)i * G + blockIdx.x] = v[i];
+    } else {
+      __syncthreads();
+    }
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
+        __threadfence();
+        red_add_release_u32(cnt, 1u);
+      }
+      __syncwarp();
+      const unsigned target = k * (unsigned)G;
+      int ok = 1;
+      if (ld_acquire_u32(cnt) < target) {
+        const unsigned long long t0 = global_ns();
+        while (ld_acquire_u32(cnt) < target) {
+          if (ld_volatile_i32(err) || global_ns() - t0 > 2000000000ULL) {
+            ok = 0;
+            break;
+          }
         }
       }
-      double v1[1] = {pq};
-      if (!reduce_all<1>(v1, part, phase++, bar, err)) { status = 3; break; }
-      const double alpha = rz / v1[0];
-      double v2[2] = {0, 0};
-      for (int i = r0 + lane; i < r1; i += 32) {
-        x[i] += alpha * p[i];
-        double ri = r[i] - alpha * __ldcg(q + i);
-        double zi = ri * dinv[i];
-        r[i] = ri;
-        z[i] = zi;
-        v2[0] += ri * ri;
-        v2[1] += ri * zi;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok && threadIdx.x == 0) atomicExch(err, 1);
+      __threadfence();
+      if constexpr (NV > 0) {
+        for (int i = 0; i < NV; i++) {
+          double s = 0;
+          for (int b = threadIdx.x; b < G; b += 32) s += __ldcg(buf + (size_t)i * G + b);
+          s = warp_sum(s);
+          if (threadIdx.x == 0) res[i] = s;
+        }
       }
-      if (!reduce_all<2>(v2, part, phase++, bar, err)) { status = 3; break; }
-      its++;
-      rn = sqrt(v2[0]);
-      if (!isfinite(rn)) { status = 2; break; }
-      if (rn <= tol) { status = 0; break; }
-      const double beta = v2[1] / rz;
-      rz = v2[1];
-      for (int i = r0 + lane; i < r1; i += 32) p[i] = z[i] + beta * p[i];
-      if (!grid_barrier(bar, err, 2000000000ULL)) { status = 3; break; }
+      if (threadIdx.x == 0) s_ok = ok;
+    }
+    __syncthreads();
+    if constexpr (NV > 0)
+      for (int i = 0; i < NV; i++) v[i] = res[i];
+    const bool r = s_ok != 0;
+    __syncthreads();
+    return r;
+  }
+};
+
+// read-once loads that leave the L1 to the gathered vector
+__device__ __forceinline__ int ldg_stream(const int* p) {
+  int v;
+  asm volatile("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ldg_stream(const double* p) {
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+
+// w = A u on the block's rows r0 .. r0 + nr, G lanes per row (w in shared
+// memory); returns the thread's part of (w, u).  u is read with plain loads:
+// other blocks' parts of it are visible after the grid-wide wait before.
+template <int G>
+__device__ __forceinline__ double spmv_rows(int r0, int nr, const int* __restrict__ rp, const int* __restrict__ col,
+                                            const double* __restrict__ val, const double* u, double* w) {
+  constexpr int R = 2, STEP = kThreads / G;  // rows per group at once, rows of a pass
+  const int lane = threadIdx.x % G;
+  double wu = 0;
+  // the groups of a warp stay together (the sums below are warp-wide); the
+  // next rows' extents are read ahead of this pass's entries
+  const int base0 = (int)(threadIdx.x & ~31) / G, sub = (int)(threadIdx.x & 31) / G;
+  int nb[R], ne[R];
+#pragma unroll
+  for (int k = 0; k < R; k++) {
+    const int i = base0 + sub + k * STEP;
+    nb[k] = i < nr ? __ldg(rp + r0 + i) : 0;
+    ne[k] = i < nr ? __ldg(rp + r0 + i + 1) : 0;
+  }
+  for (int base = base0; base < nr; base += R * STEP) {
+    int b[R], e[R], c[R][4];
+    double v[R][4], s[R];
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      b[k] = nb[k] + lane;
+      e[k] = ne[k];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int j = b[k] + q * G;
+        c[k][q] = j < e[k] ? ldg_stream(col + j) : -1;
+        v[k][q] = j < e[k] ? ldg_stream(val + j) : 0.0;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      const int i = base + sub + (R + k) * STEP;
+      nb[k] = i < nr ? __ldg(rp + r0 + i) : 0;
+      ne[k] = i < nr ? __ldg(rp + r0 + i + 1) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < R; k++) {
+      s[k] = 0;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (c[k][q] >= 0) s[k] += v[k][q] * u[c[k][q]];
+      for (int j = b[k] + 4 * G; j < e[k]; j += G) s[k] += ldg_stream(val + j) * u[ldg_stream(col + j)];
+      s[k] = group_sum<G>(s[k]);
+      const int i = base + sub + k * STEP;
+      if (i < nr && lane == 0) {
+        w[i] = s[k];
+        wu += u[r0 + i] * s[k];
+      }
     }
   }
+  return wu;
+}
+
+__global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* __restrict__ rp,
+                                                              const int* __restrict__ col,
+                                                              const double* __restrict__ val,
+                                                              const double* __restrict__ dinv,
+                                                              const double* __restrict__ b, double* xout, double rtol,
+                                                              int maxit, unsigned char* scratch) {
+  extern __shared__ double sv[];
+  const int r0 = (int)((long long)n * blockIdx.x / gridDim.x);
+  const int nr = (int)((long long)n * (blockIdx.x + 1) / gridDim.x) - r0;
+  double *r = sv, *p = r + nr, *s = p + nr, *w = s + nr, *x = w + nr;
+  double* u = reinterpret_cast<double*>(scratch + kOffU);
+  double* result = reinterpret_cast<double*>(scratch + kOffRes);
+  GridSync gs{reinterpret_cast<unsigned*>(scratch + kOffCtl), reinterpret_cast<int*>(scratch + kOffCtl + 8),
+              reinterpret_cast<double*>(scratch + kOffPart), 0u};
+  // lanes per row: about four loads per lane for a row of the mean length
+  const int mean = (int)(((long long)__ldg(rp + n) - __ldg(rp)) / n);
+  double ru = 0, rr = 0, none[1];
+  for (int i = threadIdx.x; i < nr; i += kThreads) {
+    const double bi = b[r0 + i], ui = bi * dinv[r0 + i];
+    r[i] = bi;
+    p[i] = s[i] = x[i] = 0.0;
+    u[r0 + i] = ui;
+    ru += bi * ui;
+    rr += bi * bi;
+  }
+  bool alive = gs.wait<0>(none);
+  double bnorm = 0, tol = 0, rn = 0, gamma_old = 1, alpha_old = 1;
+  int its = 0, status = 1;
+  while (true) {
+    if (!alive) { status = 3; break; }
+    double v[3] = {ru, 0.0, rr};
+    if (mean <= 8)
+      v[1] = spmv_rows<2>(r0, nr, rp, col, val, u, w);
+    else if (mean <= 16)
+      v[1] = spmv_rows<4>(r0, nr, rp, col, val, u, w);
+    else if (mean <= 32)
+      v[1] = spmv_rows<8>(r0, nr, rp, col, val, u, w);
+    else if (mean <= 64)
+      v[1] = spmv_rows<16>(r0, nr, rp, col, val, u, w);
+    else
+      v[1] = spmv_rows<32>(r0, nr, rp, col, val, u, w);
+    if (!gs.wait<3>(v)) { status = 3; break; }
+    const double gamma = v[0], delta = v[1];
+    rn = sqrt(v[2]);
+    if (its == 0) {
+      bnorm = rn;
+      tol = rtol * bnorm;
+    }
+    if (!isfinite(rn)) { status = 2; break; }
+    if (rn <= tol) { status = 0; break; }
+    if (its >= maxit) break;
+    const double beta = its > 0 ? gamma / gamma_old : 0.0;
+    const double alpha = its > 0 ? gamma / (delta - beta * gamma / alpha_old) : gamma / delta;
+    gamma_old = gamma;
+    alpha_old = alpha;
+    ru = rr = 0;
+    for (int i = threadIdx.x; i < nr; i += kThreads) {
+      const double pi = u[r0 + i] + beta * p[i], si = w[i] + beta * s[i];
+      const double ri = r[i] - alpha * si, ui = ri * dinv[r0 + i];
+      p[i] = pi;
+      s[i] = si;
+      x[i] += alpha * pi;
+      r[i] = ri;
+      u[r0 + i] = ui;
+      ru += ri * ui;
+      rr += ri * ri;
+    }
+    its++;
+    alive = gs.wait<0>(none);
+  }
+  for (int i = threadIdx.x; i < nr; i += kThreads) xout[r0 + i] = x[i];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     result[0] = its;
     result[1] = bnorm > 0 ? rn / bnorm : 0.0;
@@ -206,18 +342,26 @@ extern "C" int cfd_pcg_solve_noalloc(const int* rowptr, const int* col, const do
     scratch = g_scratch_addr[dev];
   }
   cudaStream_t s = (cudaStream_t)stream;
-  int sms = 0, per_sm = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_noalloc, kThreads, 0) != cudaSuccess ||
-      per_sm < 1) {
-    put_err(errbuf, errlen, "cfd_pcg_solve_noalloc: occupancy query failed");
+  // one block per SM, at least 256 rows each: a small system waits on fewer
+  // arrivals, and one block on none, so up to 512 rows stay on one (512 rows
+  // of 27: 6.8 us per iteration, two blocks 9.2; 8000 rows: 9.5 us on 32
+  // blocks, 11.3 on 16)
+  int sms = 0;
+  long long grid = 0;
+  size_t smem = 0;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) {
+    grid = n <= 512 ? 1 : ((long long)n + 255) / 256;
+    if (grid > sms) grid = sms;
+    if (grid > kMaxBlocks) grid = kMaxBlocks;
+    if (grid < 1) grid = 1;
+    smem = 5 * sizeof(double) * (size_t)((n + grid - 1) / grid);
+    e = cudaFuncSetAttribute(k_pcg_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+  }
+  if (e != cudaSuccess || smem > kMaxDynSmem) {
+    put_err(errbuf, errlen, "cfd_pcg_solve_noalloc: the device cannot hold the block vectors");
     return CFD_E_CUDA;
   }
-  long long grid = (long long)sms * per_sm;
-  long long want = ((long long)n + (kThreads / 32) * 8 - 1) / ((kThreads / 32) * 8);
-  if (grid > want) grid = want;
-  if (grid > kMaxBlocks) grid = kMaxBlocks;
-  if (grid < 1) grid = 1;
   unsigned char* base = static_cast<unsigned char*>(scratch);
   e = cudaMemsetAsync(base + kOffCtl, 0, 256, s);  // barrier words and error flag start at zero
   if (e == cudaSuccess) {
@@ -225,7 +369,7 @@ extern "C" int cfd_pcg_solve_noalloc(const int* rowptr, const int* col, const do
     double rt = rtol;
     unsigned char* sp = base;
     void* params[] = {&nn, (void*)&rowptr, (void*)&col, (void*)&val, (void*)&dinv, (void*)&b, (void*)&x, &rt, &mi, &sp};
-    e = cudaLaunchCooperativeKernel((const void*)k_pcg_noalloc, dim3((unsigned)grid), dim3(kThreads), params, 0, s);
+    e = cudaLaunchCooperativeKernel((const void*)k_pcg_noalloc, dim3((unsigned)grid), dim3(kThreads), params, smem, s);
   }
   double res[4] = {0, 0, 0, 0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(res, base + kOffRes, sizeof(res), cudaMemcpyDeviceToHost, s);
