@@ -679,7 +679,7 @@ int upload_problem(cfd_ctx* c) {
   c->res_blocks = residual_blocks((int)NNp, c->num_sms);
   CU(c->ir_part.alloc(c->res_blocks));
   CU(c->ir_sum.alloc(2));
-  c->nub = step3_blocks((int)NN, c->num_sms);
+  c->nub = mixed(c) ? step3_blocks<float>((int)NN) : step3_blocks<double>((int)NN);
   c->npb = pupdate_blocks((int)NNp, c->num_sms);
   CU(c->upart.alloc(3 * (size_t)c->nub));
   CU(c->ppart.alloc(2 * (size_t)c->npb));

@@ -151,7 +151,8 @@ struct Step3Args {
 };
 template <class VT>
 cudaError_t launch_step3(const Step3Args<VT>& a, cudaStream_t s);
-int step3_blocks(int NN, int num_sms);
+template <class VT>
+int step3_blocks(int NN);  // blocks of launch_step3 (its partial sums)
 
 template <class VT>
 struct SpmvK3Args {

@@ -5,9 +5,18 @@
 // library SpMVs plus 2-4 elementwise kernels and the temporary
 // cudaMalloc/cudaFree of every call.
 //
-// One thread owns one row; a warp owns one 32-row slice, so the entry loop
-// has a warp-uniform trip count, needs no shuffles, and every load of the
-// matrix is a contiguous warp-wide segment.  Matrix values and columns are
+// A warp owns a 32-row slice, lane = row, so the entry loop has a
+// warp-uniform trip count, needs no shuffles, and every load of the matrix is
+// a contiguous warp-wide segment.  With few slices that leaves most of the
+// chip idle and each warp a serial chain of up to 125 dependent rounds of
+// loads, so SPLIT warps (one block) share a slice.  FP64: warp k sums entries
+// k, k + SPLIT, ..., and the partial sums are added in warp order.  FP32: the
+// warps load entries and gather vector values side by side into shared
+// memory, and the first warp runs the multiply-adds in entry order from
+// there, so that the FP32 sums keep every bit of the unsplit row (the pressure
+// of a step is sensitive to their rounding: a reordered G^T d moved it by
+// 1e-6).  row_split below has the rule and the measurements.  Matrix values
+// and columns are
 // read with streaming (evict-first) loads so the gathered vectors stay in
 // L2.  Matrix values are VT (double or float, accumulated in VT); vectors
 // stay FP64.
@@ -24,41 +33,163 @@ inline int rows_grid(long long rows) {
   return (int)(g < 1 ? 1 : g);
 }
 
+// Warps per slice: the largest of 1, 2, 4, 8 with at most `warps` warps over
+// all slices.  Splitting pays while the chip is short of warps (a wave is 148
+// x 64) or a few long rows are its tail; it costs where the epilogue, which
+// one warp of the SPLIT runs, weighs as much as the row, and in FP32 where the
+// trip through shared memory does.  Measured in us at SPLIT 1 / 2 / 4 / 8 on
+// cavities of n^3 elements (velocity slices: 154, 1123, 3676, 8582, 16 600,
+// 22 000 and 67 000 for n = 8, 16, 24, 32, 40, 44, 64; pressure slices: 23,
+// 154, 489, 1124, 2154, 2848, 8583):
+//              n = 8                n = 16           n = 24           n = 32 (40 FP32)    n = 44 (64 FP32)
+//   FP64
+//   k_step1    31 / 28 / 17 / 10    74/62/34/21      81/70/45/50      97 / 89 / 93 / 107  205/217/230/273
+//   k_spmv_k3  32 / 18 / 10 / 6.3   71/37/20/14      74/43/30/30      89 / 61 / 59 / 63   144/144/146/152
+//   k_step3    7.6/ 7.1/ 5.2/ 4.3   23/13/7.9/6.5    30/19/15/20      32 / 32 / 34 / 46   72/70/80/107
+//   k_gt       57 / 30 / 17 / 9.6   114/59/31/17     146/72/38/22     142 / 73 / 41 / 28  148/84/87/72
+//   FP32
+//   k_step1    18 / 16 / 11 / 8.2   37/33/20/21      43/43/47/67      93 / 163 / 192 / 297
+//   k_spmv_k3  16 / 14 / 9.2 / 7.0  36/30/17/13      39/33/29/40      59 / 108 / 118 / 170
+//   k_step3    8.7/ 6.1/ 4.8/ 4.3   17/9.8/7.0/10    20/14/18/25      40 / 52 / 67 / 107
+//   k_gt       30 / 24 / 13 / 8.3   60/46/25/14      72/55/30/17      75 / 58 / 37 / 37   114/130/122/131
+// and k_gt in FP64 at n = 64 193 / 188 / 191 / 187, in FP32 on the duct of 24
+// x 24 x 160 (3145 slices) 78 / 63 / 63 / 53.
+struct SplitRule {
+  long long fp64, fp32;  // warps
+  int least32;           // least FP32 split that pays (below it: 1)
+};
+constexpr SplitRule kStep1Rule{148 * 128, 148 * 32, 2}, kSpmvK3Rule{148 * 256, 148 * 100, 2},
+    kStep3Rule{148 * 128, 148 * 50, 2}, kGtRule{148 * 512, 148 * 192, 8};
+template <class VT>
+inline int row_split(long long rows, const SplitRule& rule) {
+  const long long ns = (rows + 31) / 32, warps = sizeof(VT) == 8 ? rule.fp64 : rule.fp32;
+  int sp = 1;
+  while (sp < 8 && 2 * sp * ns <= warps) sp *= 2;
+  return sizeof(VT) == 4 && sp < rule.least32 ? 1 : sp;
+}
+constexpr int block_threads(int split) { return split == 1 ? kRowThreads : 32 * split; }
+inline int split_grid(long long rows, int sp) { return sp == 1 ? rows_grid(rows) : (int)((rows + 31) / 32); }
+
+// One entry of a row and the vector values it multiplies.
+template <class T>
+struct alignas(4 * sizeof(T)) Entry {
+  T a, b, c, d;
+};
+// Shared memory of a split slice: FP32 entries on their way to the first
+// warp, or NV FP64 partial sums of every warp.
+template <class VT, class E, int NV, int SPLIT>
+struct SplitBuf {
+  static constexpr bool ordered = sizeof(VT) == 4;
+  union {
+    E e[ordered ? 4 * SPLIT : 1][32];
+    VT v[ordered ? 1 : SPLIT][NV][32];
+  };
+};
+// Entries of a slice's rows, w of them: load(j) fetches entry j of the
+// thread's row, use(e) consumes it.  FP32 with SPLIT > 1: each of the block's
+// warps loads four of the next 4 SPLIT entries (the loads of the next group
+// are in flight while the first warp consumes the current one).
+template <int SPLIT, class B, class L, class U>
+__device__ __forceinline__ void for_entries(B& buf, int w, L load, U use) {
+  if constexpr (SPLIT == 1) {
+#pragma unroll 4
+    for (int j = 0; j < w; j++) use(load(j));
+  } else if constexpr (!B::ordered) {
+#pragma unroll 4
+    for (int j = threadIdx.x >> 5; j < w; j += SPLIT) use(load(j));
+  } else {
+    const int k = threadIdx.x >> 5, l = threadIdx.x & 31;
+    decltype(load(0)) e[4];
+    auto fetch = [&](int c0) {
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (c0 + 4 * k + i < w) e[i] = load(c0 + 4 * k + i);
+    };
+    fetch(0);
+    for (int c0 = 0; c0 < w; c0 += 4 * SPLIT) {
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; i++) buf.e[4 * k + i][l] = e[i];
+      __syncthreads();
+      fetch(c0 + 4 * SPLIT);
+      if (k == 0) {
+        const int n = min(4 * SPLIT, w - c0);
+#pragma unroll 4
+        for (int j = 0; j < n; j++) use(buf.e[j][l]);
+      }
+    }
+  }
+}
+// FP64 with SPLIT > 1: the warps' partial sums, added in warp order in the
+// first warp.  Called by every thread of the block.
+template <int SPLIT, class B, class VT, int NV>
+__device__ __forceinline__ void split_sum(B& buf, VT (&v)[NV]) {
+  if constexpr (SPLIT > 1 && !B::ordered) {
+    const int k = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (k != 0)
+#pragma unroll
+      for (int i = 0; i < NV; i++) buf.v[k][i][l] = v[i];
+    __syncthreads();
+    if (k == 0)
+#pragma unroll
+      for (int j = 1; j < SPLIT; j++)
+#pragma unroll
+        for (int i = 0; i < NV; i++) v[i] += buf.v[j][i][l];
+  }
+}
+
 // step1: R1 = R1conv - K UnpHalf_prev - G Pn (blascoCodinaHuerta.cpp:
 // 3745-3758), R1 = 0 at Dirichlet nodes (applyBC_Step1(2)),
 // UnpHalf = Un + dt R1 MdInv (:3781-3783) -- the Dirichlet zeroing is the
 // zero in minv_free.  Also writes d = UnpHalf/dt^2 - [iter>1] MdOrigInv KAcc,
 // the input of step2 (blascoCodinaHuerta.cpp:3821-3832).
-template <class VT>
-__global__ void __launch_bounds__(kRowThreads) k_step1(Step1Args<VT> a) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= a.NN) return;
-  const int s = row >> 5, l = row & 31;
+template <class VT, int SPLIT>
+__global__ void __launch_bounds__(block_threads(SPLIT)) k_step1(Step1Args<VT> a) {
+  __shared__ SplitBuf<VT, Entry<VT>, 6, SPLIT> buf;
+  const int l = threadIdx.x & 31;
+  const int row = SPLIT == 1 ? blockIdx.x * blockDim.x + threadIdx.x : 32 * blockIdx.x + l;
+  if (SPLIT == 1 && row >= a.NN) return;
+  const int s = row >> 5;
   const double inv_dt2 = 1.0000000000000000 / (a.dt * a.dt);
   VT kx = 0, ky = 0, kz = 0, gx = 0, gy = 0, gz = 0;
   {
     const int b = __ldg(a.k_off + s), w = (__ldg(a.k_off + s + 1) - b) >> 5;
     const int* col = a.k_col + b + l;
     const VT* val = a.kval + b + l;
-#pragma unroll 4
-    for (int j = 0; j < w; j++) {
-      const VT v = __ldcs(val + 32 * j);
-      const auto x = ldgv(a.uprev + __ldcs(col + 32 * j));
-      kx += v * (VT)x.x;
-      ky += v * (VT)x.y;
-      kz += v * (VT)x.z;
-    }
+    for_entries<SPLIT>(
+        buf, w,
+        [&](int j) {
+          const VT v = __ldcs(val + 32 * j);
+          const auto x = ldgv(a.uprev + __ldcs(col + 32 * j));
+          return Entry<VT>{v, (VT)x.x, (VT)x.y, (VT)x.z};
+        },
+        [&](const Entry<VT>& e) {
+          kx += e.a * e.b;
+          ky += e.a * e.c;
+          kz += e.a * e.d;
+        });
   }
   {
     const int b = __ldg(a.g_off + s), w = (__ldg(a.g_off + s + 1) - b) >> 5;
     const int* col = a.g_col + b + l;
-#pragma unroll 4
-    for (int j = 0; j < w; j++) {
-      const VT p = (VT)__ldg(a.pn + __ldcs(col + 32 * j));
-      gx += __ldcs(a.g1 + b + l + 32 * j) * p;
-      gy += __ldcs(a.g2 + b + l + 32 * j) * p;
-      gz += __ldcs(a.g3 + b + l + 32 * j) * p;
-    }
+    for_entries<SPLIT>(
+        buf, w,
+        [&](int j) {
+          const VT p = (VT)__ldg(a.pn + __ldcs(col + 32 * j));
+          return Entry<VT>{__ldcs(a.g1 + b + l + 32 * j), __ldcs(a.g2 + b + l + 32 * j),
+                           __ldcs(a.g3 + b + l + 32 * j), p};
+        },
+        [&](const Entry<VT>& e) {
+          gx += e.a * e.d;
+          gy += e.b * e.d;
+          gz += e.c * e.d;
+        });
+  }
+  if constexpr (SPLIT > 1) {
+    VT v[6] = {kx, ky, kz, gx, gy, gz};
+    split_sum<SPLIT>(buf, v);
+    if (threadIdx.x >= 32 || row >= a.NN) return;
+    kx = v[0], ky = v[1], kz = v[2], gx = v[3], gy = v[4], gz = v[5];
   }
   double4 rc;
   if (a.r1conv32) {
@@ -99,43 +230,57 @@ __global__ void __launch_bounds__(kRowThreads) k_step1(Step1Args<VT> a) {
 
 // out[p] = sum_d (G_d^T d_d)[p]; out[pin] = 0 when pin > 0
 // (step2GPU's three transposed csrmv calls + applyPresBC, CUDAcodes.cu:1006-1011).
-template <class VT>
-__global__ void __launch_bounds__(kRowThreads) k_gt(GtArgs<VT> a) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= a.NNp) return;
-  const int s = row >> 5, l = row & 31;
+template <class VT, int SPLIT>
+__global__ void __launch_bounds__(block_threads(SPLIT)) k_gt(GtArgs<VT> a) {
+  __shared__ SplitBuf<VT, VT, 1, SPLIT> buf;
+  const int l = threadIdx.x & 31;
+  const int row = SPLIT == 1 ? blockIdx.x * blockDim.x + threadIdx.x : 32 * blockIdx.x + l;
+  if (SPLIT == 1 && row >= a.NNp) return;
+  const int s = row >> 5;
   const int b = __ldg(a.gt_off + s) + l, w = (__ldg(a.gt_off + s + 1) - __ldg(a.gt_off + s)) >> 5;
-  VT acc = 0;
-#pragma unroll 4
-  for (int j = 0; j < w; j++) {
-    const int e = b + 32 * j;
-    const auto d = ldgv(a.d + __ldcs(a.gt_col + e));
-    acc += __ldcs(a.gt1 + e) * (VT)d.x + __ldcs(a.gt2 + e) * (VT)d.y + __ldcs(a.gt3 + e) * (VT)d.z;
-  }
-  a.out[row] = (a.pin > 0 && row == a.pin) ? 0.0 : (double)acc;
+  VT acc[1] = {0};
+  for_entries<SPLIT>(
+      buf, w,
+      [&](int j) {
+        const int e = b + 32 * j;
+        const auto d = ldgv(a.d + __ldcs(a.gt_col + e));
+        return __ldcs(a.gt1 + e) * (VT)d.x + __ldcs(a.gt2 + e) * (VT)d.y + __ldcs(a.gt3 + e) * (VT)d.z;
+      },
+      [&](VT t) { acc[0] += t; });
+  split_sum<SPLIT>(buf, acc);
+  if (SPLIT > 1 && (threadIdx.x >= 32 || row >= a.NNp)) return;
+  a.out[row] = (a.pin > 0 && row == a.pin) ? 0.0 : (double)acc[0];
 }
 
 // step3: R3 = -dt G Pdot - [iter>1] dt KAcc, R3 = 0 at Dirichlet nodes,
 // Acc = R3 MdInv, Unp1 = UnpHalf + dt Acc (blascoCodinaHuerta.cpp:3920-3967)
 // plus the partial sums of the convergence test (:2936-2961) and of the
 // steady-state test (:3052-3057).
-template <class VT>
-__global__ void __launch_bounds__(kRowThreads) k_step3(Step3Args<VT> a) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+template <class VT, int SPLIT>
+__global__ void __launch_bounds__(block_threads(SPLIT)) k_step3(Step3Args<VT> a) {
+  __shared__ SplitBuf<VT, Entry<VT>, 3, SPLIT> buf;
+  const int l = threadIdx.x & 31;
+  const int row = SPLIT == 1 ? blockIdx.x * blockDim.x + threadIdx.x : 32 * blockIdx.x + l;
   const double inv_dt = 1.0000000000000000 / a.dt;
   double s_u2 = 0, s_du2 = 0, m_acc = 0;
-  if (row < a.NN) {
-    const int s = row >> 5, l = row & 31;
+  VT gx = 0, gy = 0, gz = 0;
+  auto products = [&]() {
+    const int s = row >> 5;
     const int b = __ldg(a.g_off + s) + l, w = (__ldg(a.g_off + s + 1) - __ldg(a.g_off + s)) >> 5;
-    VT gx = 0, gy = 0, gz = 0;
-#pragma unroll 4
-    for (int j = 0; j < w; j++) {
-      const int e = b + 32 * j;
-      const VT p = (VT)__ldg(a.pdot + __ldcs(a.g_col + e));
-      gx += __ldcs(a.g1 + e) * p;
-      gy += __ldcs(a.g2 + e) * p;
-      gz += __ldcs(a.g3 + e) * p;
-    }
+    for_entries<SPLIT>(
+        buf, w,
+        [&](int j) {
+          const int e = b + 32 * j;
+          const VT p = (VT)__ldg(a.pdot + __ldcs(a.g_col + e));
+          return Entry<VT>{__ldcs(a.g1 + e), __ldcs(a.g2 + e), __ldcs(a.g3 + e), p};
+        },
+        [&](const Entry<VT>& e) {
+          gx += e.a * e.d;
+          gy += e.b * e.d;
+          gz += e.c * e.d;
+        });
+  };
+  auto epilogue = [&]() {
     double rx = -a.dt * (double)gx, ry = -a.dt * (double)gy, rz = -a.dt * (double)gz;
     if (a.iter != 1) {
       const double4 ka = a.kacc[row];
@@ -158,6 +303,18 @@ __global__ void __launch_bounds__(kRowThreads) k_step3(Step3Args<VT> a) {
     const double dx = u1.x - pv.x, dy = u1.y - pv.y, dz = u1.z - pv.z;
     s_du2 = dx * dx + dy * dy + dz * dz;
     m_acc = fmax(fabs((u1.x - un.x) * inv_dt), fmax(fabs((u1.y - un.y) * inv_dt), fabs((u1.z - un.z) * inv_dt)));
+  };
+  if constexpr (SPLIT == 1) {
+    if (row < a.NN) {
+      products();
+      epilogue();
+    }
+  } else {
+    products();
+    VT v[3] = {gx, gy, gz};
+    split_sum<SPLIT>(buf, v);
+    gx = v[0], gy = v[1], gz = v[2];
+    if (threadIdx.x < 32 && row < a.NN) epilogue();
   }
   double v[2] = {s_u2, s_du2};
   m_acc = warp_max(m_acc);
@@ -173,23 +330,32 @@ __global__ void __launch_bounds__(kRowThreads) k_step3(Step3Args<VT> a) {
   }
 }
 
-template <class VT>
-__global__ void __launch_bounds__(kRowThreads) k_spmv_k3(SpmvK3Args<VT> a) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= a.NN) return;
-  const int s = row >> 5, l = row & 31;
+template <class VT, int SPLIT>
+__global__ void __launch_bounds__(block_threads(SPLIT)) k_spmv_k3(SpmvK3Args<VT> a) {
+  __shared__ SplitBuf<VT, Entry<VT>, 3, SPLIT> buf;
+  const int l = threadIdx.x & 31;
+  const int row = SPLIT == 1 ? blockIdx.x * blockDim.x + threadIdx.x : 32 * blockIdx.x + l;
+  if (SPLIT == 1 && row >= a.NN) return;
+  const int s = row >> 5;
   const int b = __ldg(a.off + s) + l, w = (__ldg(a.off + s + 1) - __ldg(a.off + s)) >> 5;
   VT sx = 0, sy = 0, sz = 0;
-#pragma unroll 4
-  for (int j = 0; j < w; j++) {
-    const int e = b + 32 * j;
-    const VT v = __ldcs(a.val + e);
-    const auto x = ldgv(a.x + __ldcs(a.col + e));
-    sx += v * (VT)x.x;
-    sy += v * (VT)x.y;
-    sz += v * (VT)x.z;
-  }
-  a.y[row] = make_double4((double)sx, (double)sy, (double)sz, 0.0);
+  for_entries<SPLIT>(
+      buf, w,
+      [&](int j) {
+        const int e = b + 32 * j;
+        const VT v = __ldcs(a.val + e);
+        const auto x = ldgv(a.x + __ldcs(a.col + e));
+        return Entry<VT>{v, (VT)x.x, (VT)x.y, (VT)x.z};
+      },
+      [&](const Entry<VT>& e) {
+        sx += e.a * e.b;
+        sy += e.a * e.c;
+        sz += e.a * e.d;
+      });
+  VT v[3] = {sx, sy, sz};
+  split_sum<SPLIT>(buf, v);
+  if (SPLIT > 1 && (threadIdx.x >= 32 || row >= a.NN)) return;
+  a.y[row] = make_double4((double)v[0], (double)v[1], (double)v[2], 0.0);
 }
 
 __global__ void __launch_bounds__(kRowThreads) k_pressure_update(int n, double dt, const double* __restrict__ pn,
@@ -298,26 +464,40 @@ inline int ew_grid(long long n) {
 
 }  // namespace
 
+// Launches kernel<VT, SPLIT> with the SPLIT of the row count.
+#define SPLIT_LAUNCH(kernel, rows, rule)                                                  \
+  do {                                                                                    \
+    const int sp_ = row_split<VT>(rows, rule), g_ = split_grid(rows, sp_);                \
+    switch (sp_) {                                                                        \
+      case 1: kernel<VT, 1><<<g_, kRowThreads, 0, s>>>(a); break;                         \
+      case 2: kernel<VT, 2><<<g_, block_threads(2), 0, s>>>(a); break;                         \
+      case 4: kernel<VT, 4><<<g_, block_threads(4), 0, s>>>(a); break;                         \
+      default: kernel<VT, 8><<<g_, block_threads(8), 0, s>>>(a); break;                        \
+    }                                                                                     \
+    return cudaGetLastError();                                                            \
+  } while (0)
+
 template <class VT>
 cudaError_t launch_step1(const Step1Args<VT>& a, int, cudaStream_t s) {
-  k_step1<VT><<<rows_grid(a.NN), kRowThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  SPLIT_LAUNCH(k_step1, a.NN, kStep1Rule);
 }
 template <class VT>
 cudaError_t launch_gt(const GtArgs<VT>& a, int, cudaStream_t s) {
-  k_gt<VT><<<rows_grid(a.NNp), kRowThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  SPLIT_LAUNCH(k_gt, a.NNp, kGtRule);
 }
-int step3_blocks(int NN, int) { return rows_grid(NN); }
+template <class VT>
+int step3_blocks(int NN) {
+  return split_grid(NN, row_split<VT>(NN, kStep3Rule));
+}
+template int step3_blocks<double>(int);
+template int step3_blocks<float>(int);
 template <class VT>
 cudaError_t launch_step3(const Step3Args<VT>& a, cudaStream_t s) {
-  k_step3<VT><<<a.nblocks, kRowThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  SPLIT_LAUNCH(k_step3, a.NN, kStep3Rule);
 }
 template <class VT>
 cudaError_t launch_spmv_k3(const SpmvK3Args<VT>& a, int, cudaStream_t s) {
-  k_spmv_k3<VT><<<rows_grid(a.NN), kRowThreads, 0, s>>>(a);
-  return cudaGetLastError();
+  SPLIT_LAUNCH(k_spmv_k3, a.NN, kSpmvK3Rule);
 }
 int pupdate_blocks(int NNp, int num_sms) { return ew_grid(NNp) < num_sms * 4 ? ew_grid(NNp) : num_sms * 4; }
 cudaError_t launch_pressure_update(int NNp, double dt, const double* pn, const double* pdot, const double* pprev,
