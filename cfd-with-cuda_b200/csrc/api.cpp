@@ -148,6 +148,11 @@ struct cfd_ctx {
   DevBuf<double> cg_work, cg_part, cg_res, ir_r, ir_part, ir_sum;
   DevBuf<float> f_b, f_x, f_work;
   DevBuf<unsigned> cg_sync;
+  // Z by offsets (pcg_dia.cu) when its entries lie on few diagonals: offsets
+  // on the device, the largest |offset|, coefficients; dia_grid = 0: not used
+  DevBuf<int> zd_off;
+  DevBuf<double> zd_coef;
+  int zd_ntap = 0, zd_reach = 0, dia_grid = 0;
   DevBuf<int> nb64, nb32;  // per PCG block: [lo..., hi...] neighbour block ranges
   DevBuf<int> cg_err;
   int pcg_grid64 = 1, pcg_grid32 = 1, res_blocks = 1;
@@ -552,6 +557,8 @@ int klaunch(cfd_ctx* c, int cls, F&& f) {
 // Allocates every device buffer and uploads mesh, patterns, BC data and the
 // initial condition (initializeAndAllocateGPU, CUDAcodes.cu:161-274, and
 // applyBC_initial, blascoCodinaHuerta.cpp:4062-4110).
+int find_diagonals(cfd_ctx* c);
+
 int upload_problem(cfd_ctx* c) {
   HostProblem& P = c->P;
   cudaStream_t s = c->stream;
@@ -664,7 +671,11 @@ int upload_problem(cfd_ctx* c) {
   CU(c->cg_work.alloc(10 * NNp));
   c->pcg_grid64 = pcg_max_grid<double>((int)NNp, c->device);
   c->pcg_grid32 = pcg_max_grid<float>((int)NNp, c->device);
-  const int gmax = std::max(c->pcg_grid64, c->pcg_grid32);
+  {
+    int rc = find_diagonals(c);
+    if (rc) return rc;
+  }
+  const int gmax = std::max({c->pcg_grid64, c->pcg_grid32, c->dia_grid});
   CU(c->cg_part.alloc(8 * (size_t)gmax));
   CU(c->cg_sync.alloc(1 + (size_t)gmax));
   for (int pass = 0; pass < 2; pass++) {
@@ -697,21 +708,65 @@ int upload_problem(cfd_ctx* c) {
   return CFD_OK;
 }
 
+// The diagonals of Z's pattern (column - row), kept when they are few enough
+// for the stored-by-offsets form: at most kDiaMaxTaps of them and at most 1.2
+// times the bytes of value and column (small matrices, which the latency of an
+// iteration bounds and not its bytes, at any fill).
+int find_diagonals(cfd_ctx* c) {
+  const int n = (int)c->P.NNp;
+  c->zd_ntap = c->dia_grid = 0;
+  c->zd_off.reset();
+  c->zd_coef.reset();
+  const int grid = pcg_dia_grid(n, c->device);
+  if (grid == 0) return CFD_OK;
+  DevBuf<unsigned char> mark;
+  CU(mark.alloc(2 * (size_t)n));
+  CU(cudaMemsetAsync(mark.p, 0, mark.bytes(), c->stream));
+  CU(launch_dia_mark(n, c->z_rp.p, c->z_col.p, mark.p, c->stream));
+  std::vector<unsigned char> h(2 * (size_t)n - 1);
+  CU(cudaMemcpyAsync(h.data(), mark.p, h.size(), cudaMemcpyDeviceToHost, c->stream));
+  CU(cudaStreamSynchronize(c->stream));
+  std::vector<int> off;
+  for (size_t k = 0; k < h.size() && (int)off.size() <= kDiaMaxTaps; k++)
+    if (h[k]) off.push_back((int)k - (n - 1));
+  const int ntap = (int)off.size();
+  if (ntap < 1 || ntap > kDiaMaxTaps) return CFD_OK;
+  if (n > 4096 && 8.0 * ntap * n > 1.2 * 12.0 * (double)c->P.nnzZ) return CFD_OK;
+  CU(upload(c->zd_off, off, c->stream));
+  CU(c->zd_coef.alloc(dia_elems(n, ntap)));
+  CU(cudaStreamSynchronize(c->stream));
+  c->zd_ntap = ntap;
+  c->zd_reach = std::max(-off.front(), off.back());
+  c->dia_grid = grid;
+  return CFD_OK;
+}
+
 // ---- pressure solves ----------------------------------------------------
 
 int run_pcg64(cfd_ctx* c, const double* b, double* x, int warm, double rtol, int maxit, double* res) {
   cudaStream_t s = c->stream;
   CU(cudaMemsetAsync(c->cg_sync.p, 0, c->cg_sync.bytes(), s));
   CU(cudaMemsetAsync(c->cg_err.p, 0, sizeof(int), s));
-  PcgArgs<double> a{};
-  a.n = c->P.NNp;
-  a.off = c->zs_off.p; a.col = c->zs_col.p; a.val = c->zs_val.p; a.dinv = c->zdinv.p;
-  a.b = b; a.x = x; a.work = c->cg_work.p;
-  a.part = c->cg_part.p; a.sync = c->cg_sync.p; a.err = c->cg_err.p;
-  a.nb_lo = c->nb64.p; a.nb_hi = c->nb64.p + c->pcg_grid64;
-  a.rtol = rtol; a.maxit = maxit; a.warm = warm; a.result = c->cg_res.p;
-  a.timeout_ns = 2000000000ULL;
-  KL(CFD_K_PCG64, launch_pcg<double>(a, c->pcg_grid64, s));
+  if (c->dia_grid > 0) {
+    PcgDiaArgs a{};
+    a.d = DiaArgs{(int)c->P.NNp, c->zd_ntap, c->zd_off.p, c->zd_coef.p};
+    a.reach = c->zd_reach;
+    a.dinv = c->zdinv.p; a.b = b; a.x = x; a.mb = c->cg_work.p;
+    a.part = c->cg_part.p; a.sync = c->cg_sync.p; a.err = c->cg_err.p;
+    a.rtol = rtol; a.maxit = maxit; a.warm = warm; a.result = c->cg_res.p;
+    a.timeout_ns = 2000000000ULL;
+    KL(CFD_K_PCG64, launch_pcg_dia(a, c->dia_grid, s));
+  } else {
+    PcgArgs<double> a{};
+    a.n = c->P.NNp;
+    a.off = c->zs_off.p; a.col = c->zs_col.p; a.val = c->zs_val.p; a.dinv = c->zdinv.p;
+    a.b = b; a.x = x; a.work = c->cg_work.p;
+    a.part = c->cg_part.p; a.sync = c->cg_sync.p; a.err = c->cg_err.p;
+    a.nb_lo = c->nb64.p; a.nb_hi = c->nb64.p + c->pcg_grid64;
+    a.rtol = rtol; a.maxit = maxit; a.warm = warm; a.result = c->cg_res.p;
+    a.timeout_ns = 2000000000ULL;
+    KL(CFD_K_PCG64, launch_pcg<double>(a, c->pcg_grid64, s));
+  }
   CU(cudaMemcpyAsync(c->h_small, c->cg_res.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
   for (int i = 0; i < 4; i++) res[i] = c->h_small[i];
@@ -1751,6 +1806,9 @@ int cfd_step0(cfd_ctx* c) {
   z.minv_orig = c->minv_orig.p;
   CU(launch_build_z(z, s));
   CU(launch_recip(P.NNp, c->zdiag.p, c->zdinv.p, mixed(c) ? c->zdinv32.p : nullptr, s));
+  if (c->dia_grid > 0)
+    CU(launch_dia_fill(DiaArgs{P.NNp, c->zd_ntap, c->zd_off.p, nullptr}, c->z_rp.p, c->z_col.p, c->zval.p,
+                       c->zd_coef.p, s));
   // SELL-32 copies of the assembled operators (FP64, and FP32 in CFD_MIXED)
   CU(launch_csr_to_sell<double>(P.NN, c->k_rp.p, c->kval.p, c->ks_off.p, c->ks_val.p, s));
   CU(launch_csr_to_sell<double>(P.NN, c->g_rp.p, c->g1.p, c->gs_off.p, c->gs1.p, s));

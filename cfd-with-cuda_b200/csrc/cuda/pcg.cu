@@ -16,123 +16,13 @@
 #include <algorithm>
 #include <vector>
 
+#include "block_sync.cuh"
 #include "kernels.h"
 #include "sell_stream.cuh"
 
 namespace cfd {
 
 namespace {
-
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) { return ld_acquire_u32(p); }
-__device__ __forceinline__ void st_release_gpu(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void red_release_add(unsigned* p, unsigned v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Block-level synchronisation of the pipelined solve (all waits bounded):
-//   publish(k)        this block's own rows of phase k are written
-//   wait_nb(k)        every block owning a row this block gathers reached k
-//   arrive/wait_red   monotonic arrival counter of the per-iteration reduction
-struct BlockSync {
-  unsigned* cnt;
-  unsigned* prog;
-  int lo, hi;
-  int* err;
-  unsigned long long timeout_ns;
-
-  __device__ void publish(unsigned k) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_release_gpu(prog + blockIdx.x, k);
-    }
-  }
-  __device__ bool wait_nb(unsigned k) {
-    __shared__ int ok;
-    if (threadIdx.x < 32) {
-      // one lane per neighbour block, all polled at once
-      int good = 1;
-      const unsigned long long t0 = global_ns();
-      for (int j0 = lo; j0 <= hi; j0 += 32) {
-        const int j = j0 + (int)threadIdx.x;
-        bool done = j > hi;
-        while (true) {
-          if (!done) done = ld_acquire_gpu(prog + j) >= k;
-          if (__all_sync(0xffffffffu, done)) break;
-          // the whole warp gives up together: every lane takes the same
-          // sequence of warp-wide votes
-          if (__any_sync(0xffffffffu, ld_volatile_i32(err) != 0 || global_ns() - t0 > timeout_ns)) {
-            good = 0;
-            break;
-          }
-        }
-        if (!good) break;
-      }
-      __threadfence();
-      if (threadIdx.x == 0) {
-        if (!good) atomicExch(err, 1);
-        ok = good;
-      }
-    }
-    __syncthreads();
-    return ok != 0;
-  }
-  // partials already written by thread 0 of this block
-  __device__ void arrive() {
-    if (threadIdx.x == 0) {
-      __threadfence();
-      red_release_add(cnt, 1u);
-    }
-  }
-  // Waits until `target` arrivals, then every block sums the partials in the
-  // same fixed order (FP64): all blocks see identical values.
-  template <int NV>
-  __device__ bool wait_red(unsigned target, const double* buf, double (&v)[NV]) {
-    __shared__ double res[NV];
-    __shared__ int ok;
-    const int G = gridDim.x;
-    if (threadIdx.x < 32) {
-      int good = 1;
-      const unsigned long long t0 = global_ns();
-      while (ld_acquire_gpu(cnt) < target) {
-        if (ld_volatile_i32(err) || global_ns() - t0 > timeout_ns) {
-          good = 0;
-          break;
-        }
-      }
-      good = __all_sync(0xffffffffu, good);
-      if (good) {
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-          double sum = 0;
-          for (int i = threadIdx.x; i < G; i += 32) sum += __ldcg(buf + (size_t)k * G + i);
-          sum = warp_sum(sum);
-          if (threadIdx.x == 0) res[k] = sum;
-        }
-      } else if (threadIdx.x == 0) {
-        atomicExch(err, 1);
-      }
-      if (threadIdx.x == 0) ok = good;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NV; k++) v[k] = res[k];
-    const bool r = ok != 0;
-    __syncthreads();
-    return r;
-  }
-};
-
-// Writes this block's partial sums of NV values into buf (thread 0).
-template <int NV>
-__device__ __forceinline__ void block_partials(double (&v)[NV], double* buf) {
-  block_sum<NV>(v);
-  if (threadIdx.x == 0)
-#pragma unroll
-    for (int k = 0; k < NV; k++) buf[(size_t)k * gridDim.x + blockIdx.x] = v[k];
-}
 
 // Pipelined Jacobi-PCG (Ghysels & Vanroose 2014) with M = diag(Z)^-1:
 //   g_i = (r_i,u_i), d_i = (w_i,u_i), m_i = M w_i, n_i = Z m_i
@@ -240,8 +130,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg(PcgArgs<VT> a) {
     }
   }
   block_partials<4>(v, a.part);
-  bs.publish(2);
-  bs.arrive();
+  bs.publish_arrive(2);
 
   double bnorm = 0, tol = 0, rn = 0, gam_old = 1, alpha_old = 1;
   int its = 0, status = 1;
@@ -315,8 +204,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg(PcgArgs<VT> a) {
     }
     its++;
     block_partials<4>(d, a.part + (size_t)((i + 1) & 1) * 4 * G);
-    bs.publish((unsigned)i + 3);
-    bs.arrive();
+    bs.publish_arrive((unsigned)i + 3);
   }
   st.drain(a.timeout_ns);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
