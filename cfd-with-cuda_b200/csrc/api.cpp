@@ -148,11 +148,13 @@ struct cfd_ctx {
   DevBuf<double> cg_work, cg_part, cg_res, ir_r, ir_part, ir_sum;
   DevBuf<float> f_b, f_x, f_work;
   DevBuf<unsigned> cg_sync;
-  // Z by offsets (pcg_dia.cu) when its entries lie on few diagonals: offsets
-  // on the device, the largest |offset|, coefficients; dia_grid = 0: not used
+  // Z by offsets (pcg_dia.cu) when its entries lie on few diagonals (ntap >
+  // 0): offsets on the device, the largest |offset|, coefficients; blocks of
+  // the persistent PCG (0: too many rows for it) and of the one-pass kernels
   DevBuf<int> zd_off;
   DevBuf<double> zd_coef;
-  int zd_ntap = 0, zd_reach = 0, dia_grid = 0;
+  int zd_ntap = 0, zd_reach = 0, dia_grid = 0, dia_apply = 0;
+  DiaArgs dia() const { return DiaArgs{(int)P.NNp, zd_ntap, zd_reach, zd_off.p, zd_coef.p}; }
   DevBuf<int> nb64, nb32;  // per PCG block: [lo..., hi...] neighbour block ranges
   DevBuf<int> cg_err;
   int pcg_grid64 = 1, pcg_grid32 = 1, res_blocks = 1;
@@ -688,7 +690,7 @@ int upload_problem(cfd_ctx* c) {
 
   CU(c->cg_err.alloc(1));
   c->res_blocks = residual_blocks((int)NNp, c->num_sms);
-  CU(c->ir_part.alloc(c->res_blocks));
+  CU(c->ir_part.alloc(std::max(c->res_blocks, c->dia_apply)));
   CU(c->ir_sum.alloc(2));
   c->nub = mixed(c) ? step3_blocks<float>((int)NN) : step3_blocks<double>((int)NN);
   c->npb = pupdate_blocks((int)NNp, c->num_sms);
@@ -714,11 +716,11 @@ int upload_problem(cfd_ctx* c) {
 // iteration bounds and not its bytes, at any fill).
 int find_diagonals(cfd_ctx* c) {
   const int n = (int)c->P.NNp;
-  c->zd_ntap = c->dia_grid = 0;
+  c->zd_ntap = c->dia_grid = c->dia_apply = 0;
   c->zd_off.reset();
   c->zd_coef.reset();
-  const int grid = pcg_dia_grid(n, c->device);
-  if (grid == 0) return CFD_OK;
+  const int apply = dia_apply_grid(n, c->num_sms);
+  if (apply == 0) return CFD_OK;
   DevBuf<unsigned char> mark;
   CU(mark.alloc(2 * (size_t)n));
   CU(cudaMemsetAsync(mark.p, 0, mark.bytes(), c->stream));
@@ -737,7 +739,8 @@ int find_diagonals(cfd_ctx* c) {
   CU(cudaStreamSynchronize(c->stream));
   c->zd_ntap = ntap;
   c->zd_reach = std::max(-off.front(), off.back());
-  c->dia_grid = grid;
+  c->dia_grid = pcg_dia_grid(n, c->device);
+  c->dia_apply = apply;
   return CFD_OK;
 }
 
@@ -749,8 +752,7 @@ int run_pcg64(cfd_ctx* c, const double* b, double* x, int warm, double rtol, int
   CU(cudaMemsetAsync(c->cg_err.p, 0, sizeof(int), s));
   if (c->dia_grid > 0) {
     PcgDiaArgs a{};
-    a.d = DiaArgs{(int)c->P.NNp, c->zd_ntap, c->zd_off.p, c->zd_coef.p};
-    a.reach = c->zd_reach;
+    a.d = c->dia();
     a.dinv = c->zdinv.p; a.b = b; a.x = x; a.mb = c->cg_work.p;
     a.part = c->cg_part.p; a.sync = c->cg_sync.p; a.err = c->cg_err.p;
     a.rtol = rtol; a.maxit = maxit; a.warm = warm; a.result = c->cg_res.p;
@@ -1230,6 +1232,8 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
     work = c->fcg_work32.p;
   } else {
     a.val = c->zs_val.p;
+    if (c->dia_apply > 0) a.dia = c->dia();
+    a.dia_grid = c->dia_apply;
     if (!c->fcg_work64.p) CU(c->fcg_work64.alloc(nwork));
     work = c->fcg_work64.p;
   }
@@ -1488,9 +1492,15 @@ bool fcg_path(const cfd_ctx* c) { return learned(c) || twolevel(c); }
 // ||b - Z x||_2 in FP64 (also leaves r in ir_r and (float) r in f_b).
 int residual_norm(cfd_ctx* c, const double* b, const double* x, double* out) {
   cudaStream_t s = c->stream;
-  KL(CFD_K_RESID64, launch_residual64(c->P.NNp, c->zs_off.p, c->zs_col.p, c->zs_val.p, b, x, c->ir_r.p, c->f_b.p,
-                                      c->ir_part.p, c->res_blocks, s));
-  KL(CFD_K_OTHER, launch_sum_partials(c->ir_part.p, c->res_blocks, c->ir_sum.p, s));
+  int nparts = c->res_blocks;
+  if (x && c->dia_apply > 0) {
+    nparts = c->dia_apply;
+    KL(CFD_K_RESID64, launch_residual_dia(c->dia(), b, x, c->ir_r.p, c->f_b.p, c->ir_part.p, nparts, s));
+  } else {
+    KL(CFD_K_RESID64, launch_residual64(c->P.NNp, c->zs_off.p, c->zs_col.p, c->zs_val.p, b, x, c->ir_r.p, c->f_b.p,
+                                        c->ir_part.p, c->res_blocks, s));
+  }
+  KL(CFD_K_OTHER, launch_sum_partials(c->ir_part.p, nparts, c->ir_sum.p, s));
   CU(cudaMemcpyAsync(c->h_small, c->ir_sum.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
   *out = std::sqrt(c->h_small[0]);
@@ -1806,9 +1816,7 @@ int cfd_step0(cfd_ctx* c) {
   z.minv_orig = c->minv_orig.p;
   CU(launch_build_z(z, s));
   CU(launch_recip(P.NNp, c->zdiag.p, c->zdinv.p, mixed(c) ? c->zdinv32.p : nullptr, s));
-  if (c->dia_grid > 0)
-    CU(launch_dia_fill(DiaArgs{P.NNp, c->zd_ntap, c->zd_off.p, nullptr}, c->z_rp.p, c->z_col.p, c->zval.p,
-                       c->zd_coef.p, s));
+  if (c->zd_ntap > 0) CU(launch_dia_fill(c->dia(), c->z_rp.p, c->z_col.p, c->zval.p, c->zd_coef.p, s));
   // SELL-32 copies of the assembled operators (FP64, and FP32 in CFD_MIXED)
   CU(launch_csr_to_sell<double>(P.NN, c->k_rp.p, c->kval.p, c->ks_off.p, c->ks_val.p, s));
   CU(launch_csr_to_sell<double>(P.NN, c->g_rp.p, c->g1.p, c->gs_off.p, c->gs1.p, s));

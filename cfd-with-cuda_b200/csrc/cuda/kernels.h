@@ -176,6 +176,45 @@ cudaError_t launch_reduce_norms(const double* upart, int nub, const double* ppar
                                 cudaStream_t s);
 
 // ---- Krylov ----
+// Matrix by offsets (pcg_dia.cu): column - row takes only ntap values over
+// the whole matrix, as on a structured grid numbered along its axes; stored
+// per 32-row slice, tap-major (coef[slice][tap][lane], zero where a row has no
+// such entry), no column indices.  off: the ntap offsets, ascending.
+constexpr int kDiaMaxTaps = 160;
+struct DiaArgs {
+  int n, ntap, reach;  // reach: largest |offset|
+  const int* off;
+  const double* coef;
+};
+inline size_t dia_elems(int n, int ntap) { return (size_t)((n + 31) / 32) * ntap * 32; }
+// mark[col - row + n - 1] = 1 for every entry (mark: 2 n - 1 bytes, zeroed by
+// the caller)
+cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, cudaStream_t s);
+// Fills coef (zeroed first) from the CSR values.
+cudaError_t launch_dia_fill(const DiaArgs& d, const int* rp, const int* col, const double* val, double* coef,
+                            cudaStream_t s);
+// The pipelined Jacobi-PCG of pcg.cu on a matrix by offsets, FP64, with the
+// vectors in shared memory.  mb: 2 n work entries; part: 8 x blocks; sync: 1 +
+// blocks words, host-zeroed; result as in PcgArgs.  grid = 0 when n exceeds
+// what the blocks' shared memory holds.
+struct PcgDiaArgs {
+  DiaArgs d;
+  const double *dinv, *b;
+  double *x, *mb, *part;
+  unsigned* sync;
+  int* err;
+  double rtol;
+  int maxit, warm;
+  double* result;
+  unsigned long long timeout_ns;
+};
+int pcg_dia_grid(int n, int device);
+// Blocks of the one-pass kernels (0: n too large for them), and the residual
+// r = b - Z x with rf = (float) r (may be null) and per-block partials of r^2.
+int dia_apply_grid(int n, int num_sms);
+cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
+                                int grid, cudaStream_t s);
+cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s);
 template <class VT>
 struct PcgArgs {
   int n;
@@ -194,41 +233,6 @@ struct PcgArgs {
   double* result;  // its, relres, status, bnorm
   unsigned long long timeout_ns;
 };
-// Matrix by offsets (pcg_dia.cu): column - row takes only ntap values over
-// the whole matrix, as on a structured grid numbered along its axes; stored
-// per 32-row slice, tap-major (coef[slice][tap][lane], zero where a row has no
-// such entry), no column indices.  off: the ntap offsets, ascending.
-constexpr int kDiaMaxTaps = 160;
-struct DiaArgs {
-  int n, ntap;
-  const int* off;
-  const double* coef;
-};
-inline size_t dia_elems(int n, int ntap) { return (size_t)((n + 31) / 32) * ntap * 32; }
-// mark[col - row + n - 1] = 1 for every entry (mark: 2 n - 1 bytes, zeroed by
-// the caller)
-cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, cudaStream_t s);
-// Fills coef (zeroed first) from the CSR values.
-cudaError_t launch_dia_fill(const DiaArgs& d, const int* rp, const int* col, const double* val, double* coef,
-                            cudaStream_t s);
-// The pipelined Jacobi-PCG of pcg.cu on a matrix by offsets, FP64, with the
-// vectors in shared memory.  mb: 2 n work entries; part: 8 x blocks; sync: 1 +
-// blocks words, host-zeroed; result as in PcgArgs.  grid = 0 when n exceeds
-// what the blocks' shared memory holds.
-struct PcgDiaArgs {
-  DiaArgs d;
-  int reach;  // largest |offset|
-  const double *dinv, *b;
-  double *x, *mb, *part;
-  unsigned* sync;
-  int* err;
-  double rtol;
-  int maxit, warm;
-  double* result;
-  unsigned long long timeout_ns;
-};
-int pcg_dia_grid(int n, int device);
-cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s);
 // Block ranges each PCG block gathers from, for a given grid (host).
 // Truncated flexible CG, FCG(m), on the SELL-32 pressure matrix (fcg.cu).
 // State words in sc[]: indices below; status -1 running, 0 converged, 1
@@ -277,6 +281,8 @@ template <class VT> struct FcgArgs {
   VT* z1;
   const VT* dinv;
   int pdl;  // 1: the iteration kernels launch with programmatic dependent launch
+  DiaArgs dia;   // ntap > 0: the matrix by offsets, used by the FP64 SpMV instead of the SELL arrays
+  int dia_grid;  // blocks of that SpMV
   int upd_grid;  // > 0: blocks of the update kernel (default: one thread per entry, at most kFcgMaxBlocks)
 };
 struct Int3 {

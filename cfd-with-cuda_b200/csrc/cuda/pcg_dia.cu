@@ -34,118 +34,41 @@
 #include <algorithm>
 
 #include "block_sync.cuh"
+#include "dia.cuh"
 #include "kernels.h"
 
 namespace cfd {
 
 namespace {
 
-constexpr int kDiaWarps = 16, kDiaThreads = 32 * kDiaWarps;
-constexpr int kDiaGroup = 16;  // taps per group
 constexpr int kDiaVecs = 10;   // r u w z q s p x m dinv
 constexpr int kDiaMaxSmem = 224 * 1024;
 
 size_t dia_smem(int slices) {
-  return (size_t)slices * 32 * kDiaVecs * sizeof(double) + (size_t)(slices + kDiaWarps) * 32 * sizeof(double);
+  return (size_t)slices * 32 * kDiaVecs * sizeof(double) + dia_slot_bytes(slices);
 }
-
-__device__ __forceinline__ double ld_coef(const double* p) {
-  double v;
-  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
-// The block's share of the matrix: slices [s0, s0 + ns), ng groups per slice.
-// Warp w owns groups [g0, g1) of the ns ng; its part of slice s goes to
-// slot[s + w] (distinct for every warp and slice that meet).
-struct DiaRows {
-  DiaArgs d;
-  const int* off;  // shared memory
-  double (*slot)[32];
-  int s0, ns, ng, g0, g1, reach;
-
-  __device__ __forceinline__ int owner(int g) const { return (kDiaWarps * (g + 1) - 1) / (ns * ng); }
-  // The coefficients of group g of the block.
-  __device__ __forceinline__ void load(int g, int lane, double (&c)[kDiaGroup]) const {
-    const int sl = g / ng, t0 = (g - sl * ng) * kDiaGroup;
-    const double* p = d.coef + ((size_t)(s0 + sl) * d.ntap + t0) * 32 + lane;
-#pragma unroll
-    for (int k = 0; k < kDiaGroup; k++) c[k] = t0 + k < d.ntap ? ld_coef(p + 32 * k) : 0.0;
-  }
-  // Partial products of the warp's groups with v; c holds the first group on
-  // entry and (the stream being cyclic) again on return.
-  __device__ __forceinline__ void multiply(int warp, int lane, const double* v, double (&c)[kDiaGroup]) const {
-    if (g0 >= g1) return;
-    int sl = g0 / ng;
-    double acc[4] = {0, 0, 0, 0};
-    for (int g = g0; g < g1; g++) {
-      const int t0 = (g - sl * ng) * kDiaGroup;
-      double nxt[kDiaGroup];
-      load(g + 1 < g1 ? g + 1 : g0, lane, nxt);
-      const int row0 = (s0 + sl) * 32, row = row0 + lane;
-      double x[kDiaGroup];
-      if (row0 >= reach && row0 + 31 + reach < d.n) {
-#pragma unroll
-        for (int k = 0; k < kDiaGroup; k++) x[k] = v[row + off[t0 + k]];
-      } else {
-#pragma unroll
-        for (int k = 0; k < kDiaGroup; k++) x[k] = v[min(max(row + off[t0 + k], 0), d.n - 1)];
-      }
-#pragma unroll
-      for (int k = 0; k < kDiaGroup; k++) acc[k & 3] += c[k] * x[k];
-      const bool last = g + 1 == g1 || g + 1 == (sl + 1) * ng;
-      if (last) {
-        slot[sl + warp][lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-        acc[0] = acc[1] = acc[2] = acc[3] = 0;
-        sl++;
-      }
-#pragma unroll
-      for (int k = 0; k < kDiaGroup; k++) c[k] = nxt[k];
-    }
-  }
-  // The product of row 32 sl + l of the block, after a block barrier.
-  __device__ __forceinline__ double row(int sl, int l) const {
-    const int w1 = owner(sl * ng + ng - 1);
-    double y = 0;
-    for (int w = owner(sl * ng); w <= w1; w++) y += slot[sl + w][l];
-    return y;
-  }
-};
 
 __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   extern __shared__ double sv[];
   __shared__ int soff[kDiaMaxTaps + kDiaGroup];
   const int n = a.d.n, nslices = (n + 31) >> 5, G = gridDim.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // padding taps: coefficient 0 at offset 0
-  for (int k = threadIdx.x; k < kDiaMaxTaps + kDiaGroup; k += kDiaThreads) soff[k] = k < a.d.ntap ? a.d.off[k] : 0;
-  DiaRows M;
-  M.d = a.d;
-  M.off = soff;
-  M.reach = a.reach;
-  M.s0 = (int)((long long)nslices * blockIdx.x / G);
-  M.ns = (int)((long long)nslices * (blockIdx.x + 1) / G) - M.s0;
-  M.ng = (a.d.ntap + kDiaGroup - 1) / kDiaGroup;
-  const int T = M.ns * M.ng, R = 32 * M.ns, r0 = 32 * M.s0, nr = min(R, n - r0);
-  M.g0 = T * warp / kDiaWarps;
-  M.g1 = T * (warp + 1) / kDiaWarps;
+  const int R = 32 * ((int)((long long)nslices * (blockIdx.x + 1) / G) - (int)((long long)nslices * blockIdx.x / G));
   double *r = sv, *u = r + R, *w = u + R, *z = w + R, *q = z + R, *s = q + R, *p = s + R, *x = p + R, *m = x + R,
          *dinv = m + R;
-  M.slot = reinterpret_cast<double(*)[32]>(dinv + R);
+  const DiaRows M = dia_rows(a.d, soff, dinv + R);
+  const int r0 = 32 * M.s0, nr = min(R, n - r0), reach = a.d.reach;
 
   auto block_of = [&](int row) { return (int)(((long long)G * ((row >> 5) + 1) - 1) / nslices); };
   BlockSync bs;
   bs.cnt = a.sync;
   bs.prog = a.sync + 1;
-  bs.lo = block_of(max(r0 - a.reach, 0));
-  bs.hi = block_of(min(r0 + nr - 1 + a.reach, n - 1));
+  bs.lo = block_of(max(r0 - reach, 0));
+  bs.hi = block_of(min(r0 + nr - 1 + reach, n - 1));
   bs.err = a.err;
   bs.timeout_ns = a.timeout_ns;
   double* mb[2] = {a.mb, a.mb + n};
 
-  // with fewer groups than warps some slots between a slice's first and last
-  // warp are never written
-  for (int k = threadIdx.x; k < (M.ns + kDiaWarps) * 32; k += kDiaThreads) M.slot[k >> 5][k & 31] = 0.0;
   double c[kDiaGroup];
   if (M.g0 < M.g1) M.load(M.g0, lane, c);
   __syncthreads();  // soff, slots
@@ -255,6 +178,33 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   }
 }
 
+// r = b - Z x in FP64, rf = (float) r, per-block partial of r^2: one pass over
+// the coefficients, bound by their stream (us on the 64^3 cavity: 68 on the
+// SELL-32 form, 47 here).
+__global__ void __launch_bounds__(kDiaThreads, 1) k_residual_dia(DiaArgs d, const double* __restrict__ b,
+                                                                 const double* __restrict__ x, double* r, float* rf,
+                                                                 double* part) {
+  extern __shared__ double sv[];
+  __shared__ int soff[kDiaMaxTaps + kDiaGroup];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const DiaRows M = dia_rows(d, soff, sv);
+  double c[kDiaGroup];
+  if (M.g0 < M.g1) M.load(M.g0, lane, c);
+  __syncthreads();
+  M.multiply(warp, lane, x, c);
+  __syncthreads();
+  const int r0 = 32 * M.s0, nr = min(32 * M.ns, d.n - r0);
+  double v[1] = {0};
+  for (int i = threadIdx.x; i < nr; i += kDiaThreads) {
+    const double ri = b[r0 + i] - M.row(i >> 5, i & 31);
+    r[r0 + i] = ri;
+    if (rf) rf[r0 + i] = (float)ri;
+    v[0] += ri * ri;
+  }
+  block_sum<1>(v);
+  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+}
+
 __global__ void k_dia_mark(int n, const int* __restrict__ rp, const int* __restrict__ col, unsigned char* mark) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     for (int k = rp[i]; k < rp[i + 1]; k++) {
@@ -300,6 +250,18 @@ cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s) {
   void* params[] = {&args};
   return cudaLaunchCooperativeKernel((const void*)k_pcg_dia, dim3(grid), dim3(kDiaThreads), params,
                                      dia_smem((ns + grid - 1) / grid), s);
+}
+
+int dia_apply_grid(int n, int num_sms) { return dia_blocks(n, num_sms); }
+
+cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
+                                int grid, cudaStream_t s) {
+  const int ns = (d.n + 31) / 32;
+  if (grid < 1 || grid > ns || d.ntap < 1 || d.ntap > kDiaMaxTaps) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(k_residual_dia, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem);
+  if (e != cudaSuccess) return e;
+  k_residual_dia<<<grid, kDiaThreads, dia_slot_bytes((ns + grid - 1) / grid), s>>>(d, b, x, r, rf, part);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, cudaStream_t s) {

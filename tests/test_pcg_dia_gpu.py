@@ -1,5 +1,6 @@
-"""The FP64 Jacobi-PCG on the pressure matrix stored by offsets (pcg_dia.cu)
-against the general solver: the same mesh with its corner nodes renumbered at
+"""The FP64 solves on the pressure matrix stored by offsets (pcg_dia.cu: the
+Jacobi-PCG, the two-level flexible CG's SpMV, the residual) against the general
+kernels: the same mesh with its corner nodes renumbered at
 random has the same Z up to a permutation, but no few-diagonal form, so it takes
 the SELL-32 kernel.
 
@@ -69,3 +70,28 @@ def test_offsets_form_matches_general(kind, n, warm, tmp_path):
         s.close()
     assert abs(its[0] - its[1]) <= 2
     assert np.linalg.norm(xs[0] - xs[1]) <= 4e-7 * np.linalg.norm(xs[1])
+
+
+@pytest.mark.parametrize("kind,n", [("cavity", 4), ("graded", 12), ("duct", (8, 40)), ("cavity", 21)])
+def test_offsets_form_two_level(kind, n, tmp_path):
+    """FP64 two-level solves and a mixed solve's FP64 refinement on both forms."""
+    import cfdfs
+    from cfdfs import meshgen
+    pa, pb, perm = _decks(tmp_path, kind, n)
+    dims = meshgen.duct_grid_dims(*n) if kind == "duct" else (n + 1,) * 3
+    rhs = np.random.default_rng(4).standard_normal(len(perm))
+    b = np.empty_like(rhs)
+    b[perm] = rhs
+    for precision in (cfdfs.FP64, cfdfs.MIXED):
+        got = []
+        for path, f, pmap in ((pa, rhs, None), (pb, b, perm)):
+            s = cfdfs.Solver(device=0, precision=precision, precond=cfdfs.PC_TWOLEVEL, cg_rtol=1e-10)
+            s.load(path)
+            s.step0()
+            s.set_pressure_grid(dims, pmap)
+            x, st = s.pressure_solve(f)
+            assert st.status == 0 and st.fallback == 0 and st.relres <= 1e-10
+            got.append((x if pmap is None else x[perm], st.iterations))
+            s.close()
+        assert abs(got[0][1] - got[1][1]) <= 2 + (precision == cfdfs.MIXED) * 8
+        assert np.linalg.norm(got[0][0] - got[1][0]) <= 4e-7 * np.linalg.norm(got[1][0])
