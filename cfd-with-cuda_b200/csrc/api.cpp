@@ -25,6 +25,7 @@
 #include "../../include/cfdfs.h"
 #include "cuda/kernels.h"
 #include "cuda/unet.h"
+#include "dev_pool.h"
 #include "host/coarse.h"
 #include "host/problem.h"
 #include "host/unet_net.h"
@@ -81,19 +82,24 @@ template <class T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
+  DevPool* pool = nullptr;  // where p came from (null: cudaMalloc)
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { reset(); }
   void reset() {
-    if (p) cudaFree(p);
+    if (p && pool)
+      pool->put(p);
+    else if (p)
+      cudaFree(p);
     p = nullptr;
     n = 0;
   }
   cudaError_t alloc(size_t count) {
     reset();
     if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
+    pool = current_pool();
+    cudaError_t e = pool ? pool->get(count * sizeof(T), (void**)&p) : cudaMalloc((void**)&p, count * sizeof(T));
     if (e != cudaSuccess) {
       p = nullptr;
       return e;
@@ -107,6 +113,7 @@ struct DevBuf {
 }  // namespace
 
 struct cfd_ctx {
+  DevPool pool;  // first member: outlives every buffer taken from it
   int device = 0, num_sms = 148;
   cudaStream_t stream = nullptr;
   cfd_options opt{};
@@ -1648,6 +1655,7 @@ int cfd_create(cfd_ctx** out, int device) {
   if (cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess)
     return CFD_E_CUDA;
+  c->pool.streams(c->stream, c->stream2);
   if (cudaMallocHost((void**)&c->h_small, 64 * sizeof(double)) != cudaSuccess) return CFD_E_CUDA;
   if (const char* e = std::getenv("CFD_FCG_GRAPH")) c->fcg_use_graph = std::atoi(e) != 0;
   if (const char* e = std::getenv("CFD_FCG_PERSIST")) c->fcg_persist = std::atoi(e) != 0;
@@ -1670,6 +1678,7 @@ void cfd_destroy(cfd_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->stream2) cudaStreamSynchronize(c->stream2);
+  c->pool.streams(nullptr, nullptr);  // both idle
   if (c->h_small) cudaFreeHost(c->h_small);
   if (c->l2_window) {
     // release the persisting L2 lines and the set-aside this context took
@@ -1714,6 +1723,7 @@ int cfd_set_options(cfd_ctx* c, const cfd_options* o) {
 
 int cfd_load_inp(cfd_ctx* c, const char* path) {
   if (!c || !path) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   int rc = set_device(c);
   if (rc) return rc;
   c->P = HostProblem();
@@ -1728,6 +1738,7 @@ int cfd_load_mesh(cfd_ctx* c, const cfd_problem_info* info, const double* coords
                   const double* bcvals, int nVelFaces, const int* velfaces, const double* monitor) {
   if (!c || !info || !coords || !conn || (nBC > 0 && !bcvals) || (nVelFaces > 0 && !velfaces) || !monitor)
     return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   int rc = set_device(c);
   if (rc) return rc;
   HostProblem& P = c->P;
@@ -1779,6 +1790,7 @@ int cfd_info(const cfd_ctx* c, cfd_problem_info* i) {
 
 int cfd_step0(cfd_ctx* c) {
   if (!c) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->loaded, "cfd_step0 before cfd_load_inp");
   int rc = set_device(c);
   if (rc) return rc;
@@ -1862,6 +1874,7 @@ int cfd_begin_step(cfd_ctx* c) {
 
 int cfd_convect(cfd_ctx* c) {
   if (!c) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->assembled, "cfd_convect before cfd_step0");
   cudaStream_t s = c->stream;
   if (mixed(c))
@@ -1938,6 +1951,7 @@ int cfd_step1(cfd_ctx* c, int iter) {
 
 int cfd_step2(cfd_ctx* c, int iter, cfd_solve_stats* st) {
   if (!c) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->assembled && iter >= 1, "cfd_step2: bad state or iter");
   cudaStream_t s = c->stream;
   const int pin = c->P.zeroP;
@@ -2054,6 +2068,7 @@ int cfd_end_step(cfd_ctx* c) {
 
 int cfd_run(cfd_ctx* c, int nsteps, cfd_run_stats* st) {
   if (!c) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->assembled, "cfd_run before cfd_step0");
   cfd_run_stats r{};
   int rc = set_device(c);
@@ -2229,6 +2244,7 @@ int cfd_download_matrix(cfd_ctx* c, int which, long long* nnz, int* rowptr, int*
 
 int cfd_pressure_solve(cfd_ctx* c, const double* rhs, double* x, cfd_solve_stats* st) {
   if (!c || !rhs || !x) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->assembled, "cfd_pressure_solve before cfd_step0");
   cudaStream_t s = c->stream;
   const size_t NNp = c->P.NNp;
@@ -2262,6 +2278,7 @@ int cfd_read_restart(cfd_ctx* c, const char* path) {
 
 int cfd_set_bc_values(cfd_ctx* c, int n, const int* nodes, const double* uvw) {
   if (!c || !c->loaded || n < 0 || (n > 0 && (!nodes || !uvw))) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   for (int i = 0; i < n; i++) NEED(nodes[i] >= 0 && nodes[i] < c->P.NN, "BC node out of range");
   DevBuf<int> dn;
   DevBuf<double> dv;
@@ -2417,6 +2434,7 @@ int cfd_coarse_matrix(int device, const int dims[3], const int* rowptr, const in
 
 int cfd_selftest_wait_timeout(cfd_ctx* c, int timeout_ms) {
   if (!c || timeout_ms <= 0 || timeout_ms > 10000) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   int rc = set_device(c);
   if (rc) return rc;
   cudaStream_t s = c->stream;
@@ -2665,6 +2683,7 @@ int cfd_unet_train_batch(cfd_unet* u, const int dims[3], int nb, const float* x,
 
 int cfd_unet_attach(cfd_ctx* c, cfd_unet* u, const int dims[3], const int* p_of_vox) {
   if (!c) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   if (!u) {
     c->reset_fcg_graphs();
     c->unet = nullptr;
@@ -2725,6 +2744,7 @@ int cfd_unet_load(cfd_ctx* c, const char* path, const int dims[3]) {
 
 int cfd_pressure_residual(cfd_ctx* c, const double* rhs, const double* x, double* r, double* norm) {
   if (!c || !rhs || !x || !r) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->assembled, "cfd_pressure_residual before cfd_step0");
   cudaStream_t s = c->stream;
   const size_t NNp = c->P.NNp;
@@ -2744,12 +2764,14 @@ int cfd_pressure_residual(cfd_ctx* c, const double* rhs, const double* x, double
 
 int cfd_set_pressure_grid(cfd_ctx* c, const int dims[3], const int* p_of_vox) {
   if (!c || !dims) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->loaded, "cfd_set_pressure_grid before cfd_load_inp");
   return set_grid(c, dims, p_of_vox);
 }
 
 int cfd_precond_apply(cfd_ctx* c, const double* r, double* z) {
   if (!c || !r || !z) return CFD_E_BADARG;
+  PoolScope scope(&c->pool);
   NEED(c->assembled, "cfd_precond_apply before cfd_step0");
   cudaStream_t s = c->stream;
   const bool with_coarse = c->opt.precond == CFD_PC_TWOLEVEL || c->opt.precond == CFD_PC_LEARNED;
