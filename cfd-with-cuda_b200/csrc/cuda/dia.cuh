@@ -22,9 +22,9 @@ inline int dia_blocks(int n, int num_sms) {
   return g > 0 && dia_slot_bytes((ns + g - 1) / g) <= 200 * 1024 ? g : 0;
 }
 
-__device__ __forceinline__ double ld_coef(const double* p) {
+__device__ __forceinline__ double ld_coef(const double* p, unsigned long long policy) {
   double v;
-  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(policy));
   return v;
 }
 
@@ -36,14 +36,19 @@ struct DiaRows {
   const int* off;  // shared memory
   double (*slot)[32];
   int s0, ns, ng, g0, g1;
+  // the first groups of every warp, keep_bytes over the whole matrix, stay
+  // in L2 from one iteration of a solve to the next; the rest passes through
+  int gk;
+  unsigned long long keep, once;
 
   __device__ __forceinline__ int owner(int g) const { return (kDiaWarps * (g + 1) - 1) / (ns * ng); }
   // The coefficients of group g of the block.
   __device__ __forceinline__ void load(int g, int lane, double (&c)[kDiaGroup]) const {
     const int sl = g / ng, t0 = (g - sl * ng) * kDiaGroup;
+    const unsigned long long policy = g < gk ? keep : once;
     const double* p = d.coef + ((size_t)(s0 + sl) * d.ntap + t0) * 32 + lane;
 #pragma unroll
-    for (int k = 0; k < kDiaGroup; k++) c[k] = t0 + k < d.ntap ? ld_coef(p + 32 * k) : 0.0;
+    for (int k = 0; k < kDiaGroup; k++) c[k] = t0 + k < d.ntap ? ld_coef(p + 32 * k, policy) : 0.0;
   }
   // Partial products of the warp's groups with v; c holds the first group on
   // entry and (the stream being cyclic) again on return.
@@ -85,10 +90,19 @@ struct DiaRows {
   }
 };
 
+// Part of a matrix's coefficients that a persistent solve asks to stay in L2
+// (126 MB, shared with the vectors; kernels that pass over the matrix once, or
+// between reads of the coarse inverse, ask for none: 2 us slower with it).  Measured per iteration of
+// the persistent PCG at 0 / 0.1 / 0.25 / 0.35 / 0.5 of the coefficients: 46.2 /
+// 45.2 / 43.5 / 44.1 / 47.1 us for 275 MB (64^3), 22.5 / 21.8 / 21.2 / 20.8 /
+// 20.2 for 118 MB (48^3; 19.8 at 0.6, 23.0 at 1): the L2's own rate is not much
+// above the copy rate, and past about 70 MB it starts to lose lines.
+constexpr double kPcgKeepBytes = 70e6;
+
 // Sets up the block's share and its offsets table (kDiaMaxTaps + kDiaGroup ints
 // of shared memory); slot: dia_slot_bytes(its slices).  The caller
 // synchronises the block before the first product.
-__device__ __forceinline__ DiaRows dia_rows(const DiaArgs& d, int* soff, double* slot) {
+__device__ __forceinline__ DiaRows dia_rows(const DiaArgs& d, int* soff, double* slot, double keep_bytes) {
   const int nslices = (d.n + 31) >> 5, G = gridDim.x, warp = threadIdx.x >> 5;
   // padding taps: coefficient 0 at offset 0
   for (int k = threadIdx.x; k < kDiaMaxTaps + kDiaGroup; k += kDiaThreads) soff[k] = k < d.ntap ? d.off[k] : 0;
@@ -102,6 +116,10 @@ __device__ __forceinline__ DiaRows dia_rows(const DiaArgs& d, int* soff, double*
   M.g0 = T * warp / kDiaWarps;
   M.g1 = T * (warp + 1) / kDiaWarps;
   M.slot = reinterpret_cast<double(*)[32]>(slot);
+  M.keep = l2_evict_last();
+  M.once = l2_evict_first();
+  const double bytes = 256.0 * (double)nslices * d.ntap;
+  M.gk = M.g0 + (bytes <= keep_bytes ? M.g1 - M.g0 : (int)((M.g1 - M.g0) * (keep_bytes / bytes)));
   // with fewer groups than warps some slots between a slice's first and last
   // warp are never written
   for (int k = threadIdx.x; k < (M.ns + kDiaWarps) * 32; k += kDiaThreads) slot[k] = 0.0;

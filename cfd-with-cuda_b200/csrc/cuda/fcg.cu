@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_fcg_spmv_dia(FcgArgs<double>
   const int m = (int)sc[kFcgM], it = (int)sc[kFcgIt];
   const int nd = it < m ? it : m;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const DiaRows M = dia_rows(a.dia, soff, slots);
+  const DiaRows M = dia_rows(a.dia, soff, slots, 0.0);
   double c[kDiaGroup];
   if (M.g0 < M.g1) M.load(M.g0, lane, c);
   __syncthreads();

@@ -25,8 +25,9 @@
 // iteration on cavities of n^3 elements, against k_pcg on the SELL-32 form (us):
 //   n          4     8     16    24    32    48    64
 //   k_pcg      15.8  17.0  19.9  20.4  21.2  42    77.5
-//   k_pcg_dia  4.7   5.1   6.7   8.6   13.0  23.4  46
-// 46 us at n = 64 is 0.93 of the copy rate on the 275 MB of coefficients.  Half
+//   k_pcg_dia  4.7   5.1   6.5   8.4   10.6  19.6  43.7
+// of which L2 residence of part of the coefficients (dia.cuh) gave 13.0 -> 10.6
+// at n = 32 and 46 -> 43.7 at 64: 0.98 of the copy rate on the 275 MB.  Half
 // the coefficients (Z is symmetric) would halve that, but the mirror reads of
 // other blocks' rows come from L2 at about the same rate.  Keeping the
 // coefficients of small grids in the L1 changed nothing there and cost the
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   const int R = 32 * ((int)((long long)nslices * (blockIdx.x + 1) / G) - (int)((long long)nslices * blockIdx.x / G));
   double *r = sv, *u = r + R, *w = u + R, *z = w + R, *q = z + R, *s = q + R, *p = s + R, *x = p + R, *m = x + R,
          *dinv = m + R;
-  const DiaRows M = dia_rows(a.d, soff, dinv + R);
+  const DiaRows M = dia_rows(a.d, soff, dinv + R, kPcgKeepBytes);
   const int r0 = 32 * M.s0, nr = min(R, n - r0), reach = a.d.reach;
 
   auto block_of = [&](int row) { return (int)(((long long)G * ((row >> 5) + 1) - 1) / nslices); };
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_residual_dia(DiaArgs d, cons
   extern __shared__ double sv[];
   __shared__ int soff[kDiaMaxTaps + kDiaGroup];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const DiaRows M = dia_rows(d, soff, sv);
+  const DiaRows M = dia_rows(d, soff, sv, 0.0);
   double c[kDiaGroup];
   if (M.g0 < M.g1) M.load(M.g0, lane, c);
   __syncthreads();
