@@ -222,9 +222,11 @@ struct cfd_ctx {
   bool fcg_persist = false;
   // CFD_COARSE_HOST=1: factor and invert the coarse matrix on the host
   bool coarse_on_host = false;
-  // CFD_PDL=1: the flexible-CG iteration kernels use programmatic dependent
-  // launch (each may start while the one before it drains)
-  bool pdl = false;
+  // the flexible-CG iteration kernels use programmatic dependent launch: each
+  // starts while the one before it drains, and requests what does not depend
+  // on it (the matrix, the coarse inverse, tables) meanwhile; CFD_PDL=0 turns
+  // it off
+  bool pdl = true;
   // CFD_L2_PERSIST=1: a persisting L2 window over the coarse inverse
   bool l2_persist = false, l2_window = false;
   // CFD_COARSE_SPACING=<s>: coarse-lattice spacing in voxels (default 4)
@@ -1295,7 +1297,8 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
   // the sequential form: its correction would need a second SpMV.
   const bool split = sizeof(VT) == 4 && a.stencil && c->cs_zp_ok && !pmap && c->fcg_split;
   a.dinv = dinv;
-  a.pdl = c->pdl ? 1 : 0;
+  a.pdl = c->pdl && !split ? 1 : 0;  // the split form forks to a second stream
+  a.keep_l2 = stencil_keep_fraction(n, (double)c->cs_nc * c->cs_ld * sizeof(__half));
   a.upd_grid = c->upd_grid >= 0 ? c->upd_grid : 4 * c->num_sms;
   if (split) {
     if (!c->fcg_z1.p) CU(c->fcg_z1.alloc(n));

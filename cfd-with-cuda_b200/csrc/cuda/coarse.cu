@@ -19,9 +19,10 @@ namespace cfd {
 
 namespace {
 
-// c = P^T r, separably: one block per coarse (iy, iz) pair.  The block's
-// fine x-lines (the y-z support of the pair, weights wy wz kept in shared
-// memory) are summed by G groups of fd[0] threads, each thread one fine x
+// c = P^T r, separably: one block per coarse (iy, iz) pair and range of coarse
+// x-nodes (blockIdx.y of nxs ranges).  The block's fine x-lines (the y-z support of
+// the pair, weights wy wz kept in shared memory, set up before the wait for the
+// previous kernel) are summed by G groups of threads, each thread one fine x
 // over every G-th line (independent loads), the group partials are added,
 // and warps restrict the resulting fine x-line onto the coarse x-nodes.
 constexpr int kRestrictThreads = 512;
@@ -29,14 +30,14 @@ constexpr int kRestrictLines = 1024;  // y-z support lines per coarse pair at mo
 template <class VT>
 __global__ void __launch_bounds__(kRestrictThreads) k_restrict(CoarseArgs<VT> a, const VT* __restrict__ r,
                                                                float* __restrict__ c, const int* done) {
-  pdl_wait();
-  pdl_trigger();
-  if (done && *done) return;
-  extern __shared__ double sline[];  // G x fd[0] partial sums
+  pdl_trigger();  // the coarse solve reads only constants before its wait
+  extern __shared__ double sline[];  // G x W partial sums
   __shared__ double swt[kRestrictLines];
   __shared__ int sbase[kRestrictLines];
   const int cx = a.cd[0], cy = a.cd[1];
   const int iy = blockIdx.x % cy, iz = blockIdx.x / cy;
+  const int ix0 = cx * blockIdx.y / gridDim.y, ix1 = cx * (blockIdx.y + 1) / gridDim.y;
+  const int xb = a.rx[2 * ix0], W = a.rx[2 * (ix1 - 1) + 1] - xb + 1;  // fine x-range
   const int y0 = a.ry[2 * iy], ny = a.ry[2 * iy + 1] - y0 + 1;
   const int z0 = a.rz[2 * iz], nz = a.rz[2 * iz + 1] - z0 + 1;
   const int fx = a.fd[0], fxy = a.fd[0] * a.fd[1];
@@ -46,30 +47,32 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(CoarseArgs<VT> a,
     const double wy = a.i0y[y] == iy ? 1.0 - a.fy[y] : (a.i0y[y] + 1 == iy ? a.fy[y] : 0.0);
     const double wz = a.i0z[z] == iz ? 1.0 - a.fz[z] : (a.i0z[z] + 1 == iz ? a.fz[z] : 0.0);
     swt[l] = wy * wz;
-    sbase[l] = fx * y + fxy * z;
+    sbase[l] = xb + fx * y + fxy * z;
   }
+  pdl_wait();
+  if (done && *done) return;
   __syncthreads();
-  const int G = fx <= (int)blockDim.x ? (int)blockDim.x / fx : 1;
-  const int g = threadIdx.x / fx;
-  for (int x = threadIdx.x % fx; g < G && x < fx; x += (G == 1 ? (int)blockDim.x : fx)) {
+  const int G = W <= (int)blockDim.x ? (int)blockDim.x / W : 1;
+  const int g = threadIdx.x / W;
+  for (int x = threadIdx.x % W; g < G && x < W; x += (G == 1 ? (int)blockDim.x : W)) {
     double acc = 0.0;
 #pragma unroll 4
     for (int l = g; l < nl; l += G) {
       const int v = sbase[l] + x;
       acc += swt[l] * (double)r[a.pmap ? a.pmap[v] : v];
     }
-    sline[g * fx + x] = acc;
+    sline[g * W + x] = acc;
     if (G != 1) break;
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int ix = warp; ix < cx; ix += blockDim.x >> 5) {
+  for (int ix = ix0 + warp; ix < ix1; ix += blockDim.x >> 5) {
     const int x0 = a.rx[2 * ix], x1 = a.rx[2 * ix + 1];
     double acc = 0.0;
     for (int x = x0 + lane; x <= x1; x += 32) {
       const double wx = a.i0x[x] == ix ? 1.0 - a.fx[x] : (a.i0x[x] + 1 == ix ? a.fx[x] : 0.0);
       double sx = 0.0;
-      for (int gg = 0; gg < G; gg++) sx += sline[gg * fx + x];
+      for (int gg = 0; gg < G; gg++) sx += sline[gg * W + x - xb];
       acc += wx * sx;
     }
     acc = warp_sum(acc);
@@ -87,32 +90,36 @@ __device__ __forceinline__ float dot8(const uint4& q, const float* c) {
 }
 
 // e = inv c: one block of four warps per row, every thread with its share
-// of the row's 16-byte loads (8 FP16 entries each) in flight at once, FP32
-// products with c (read through L1), block sum.  The inverse is read with
-// an evict-last L2 policy (the SpMV's matrix stream is evict-first), so it
-// stays in L2 from one flexible-CG iteration to the next.
-constexpr int kMvThreads = 128;
+// of the row's 16-byte loads (8 FP16 entries each) in flight at once and
+// requested before the wait for c, FP32 products with c (read through L1),
+// block sum.  The inverse is read with an evict-last L2 policy (the SpMV's
+// matrix stream is evict-first), so it stays in L2 from one flexible-CG
+// iteration to the next.
+constexpr int kMvThreads = 128, kMvLoads = 6;  // 6 x 128 x 8 entries >= kCoarseMaxNodes of the solver
 template <class VT>
 __global__ void __launch_bounds__(kMvThreads) k_coarse_mv(int nc, int ld, const __half* __restrict__ inv, float rscale,
                                                           const float* __restrict__ c, VT* __restrict__ e,
                                                           const int* done) {
-  pdl_wait();
-  pdl_trigger();
-  if (done && *done) return;
   const int row = blockIdx.x;
   const int nv8 = nc >> 3, tail = nc & 7;  // whole 8-entry groups inside the row, then a tail
   const uint4* ir = reinterpret_cast<const uint4*>(inv + (size_t)row * ld);
   const unsigned long long keep = l2_evict_last();
+  const int k = threadIdx.x;
+  uint4 q[kMvLoads];
+#pragma unroll
+  for (int u = 0; u < kMvLoads; u++)
+    if (k + u * kMvThreads < nv8) q[u] = ldg_hint(ir + k + u * kMvThreads, keep);
+  pdl_wait();
+  pdl_trigger();
+  if (done && *done) return;
+  // four chains over the first four loads where a thread has them all, one
+  // chain otherwise and for the rest
   float s[4] = {0.f, 0.f, 0.f, 0.f};
-  int k = threadIdx.x;
-  for (; k + 3 * kMvThreads < nv8; k += 4 * kMvThreads) {
-    uint4 q[4];
+  const bool four = k + 3 * kMvThreads < nv8;
 #pragma unroll
-    for (int u = 0; u < 4; u++) q[u] = ldg_hint(ir + k + u * kMvThreads, keep);
-#pragma unroll
-    for (int u = 0; u < 4; u++) s[u] += dot8(q[u], c + 8 * (k + u * kMvThreads));
-  }
-  for (; k < nv8; k += kMvThreads) s[0] += dot8(ldg_hint(ir + k, keep), c + 8 * k);
+  for (int u = 0; u < kMvLoads; u++)
+    if (k + u * kMvThreads < nv8) s[four && u < 4 ? u : 0] += dot8(q[u], c + 8 * (k + u * kMvThreads));
+  for (int kk = k + kMvLoads * kMvThreads; kk < nv8; kk += kMvThreads) s[0] += dot8(ldg_hint(ir + kk, keep), c + 8 * kk);
   if (threadIdx.x < tail) s[1] += __half2float(inv[(size_t)row * ld + 8 * nv8 + threadIdx.x]) * c[8 * nv8 + threadIdx.x];
   float t = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
   __shared__ float sw[kMvThreads / 32];
@@ -126,37 +133,51 @@ __global__ void __launch_bounds__(kMvThreads) k_coarse_mv(int nc, int ld, const 
   }
 }
 
+// z from r, dinv, e and y.  Only e is written by the kernel before, so all
+// the rest of a thread's first voxel is loaded before the wait for it.
 template <class VT>
 __global__ void __launch_bounds__(256) k_precond(CoarseArgs<VT> a, int nv, const VT* __restrict__ r,
                                                  const VT* __restrict__ dinv, const VT* __restrict__ e,
                                                  const float* __restrict__ y, const double* rr, double dscale,
                                                  VT* __restrict__ z, const int* done) {
+  pdl_trigger();  // the SpMV reads only the matrix before its wait
+  const int cx = a.cd[0], cxy = a.cd[0] * a.cd[1];
+  const int bx = a.cd[0] > 1, by = a.cd[1] > 1, bz = a.cd[2] > 1;
+  int p = 0, e0 = 0;
+  VT jac = 0, fx = 0, fy = 0, fz = 0, net = 0;
+  auto load = [&](int v) {
+    p = a.pmap ? a.pmap[v] : v;
+    jac = dinv[p] * r[p];
+    if (e) {
+      const int x = v % a.fd[0], yy = (v / a.fd[0]) % a.fd[1], zz = v / (a.fd[0] * a.fd[1]);
+      e0 = a.i0x[x] + cx * a.i0y[yy] + cxy * a.i0z[zz];
+      fx = (VT)a.fx[x], fy = (VT)a.fy[yy], fz = (VT)a.fz[zz];
+    }
+    if (y) net = (VT)y[v];
+  };
+  int v = blockIdx.x * blockDim.x + threadIdx.x;
+  bool loaded = v < nv;
+  if (loaded) load(v);
   pdl_wait();
-  pdl_trigger();
   if (done && *done) return;
   VT ys = 0;
   if (y) ys = (VT)(rr[0] > 0.0 ? sqrt(rr[0] / (double)nv) / dscale : 0.0);
-  const int cx = a.cd[0], cxy = a.cd[0] * a.cd[1];
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    const int p = a.pmap ? a.pmap[v] : v;
-    VT zi = dinv[p] * r[p];
+  for (; v < nv; v += gridDim.x * blockDim.x) {
+    if (!loaded) load(v);
+    loaded = false;
+    VT zi = jac;
     if (e) {
-      const int x = v % a.fd[0], yy = (v / a.fd[0]) % a.fd[1], zz = v / (a.fd[0] * a.fd[1]);
-      const int ix = a.i0x[x], iy = a.i0y[yy], iz = a.i0z[zz];
-      const VT fx = (VT)a.fx[x], fy = (VT)a.fy[yy], fz = (VT)a.fz[zz];
-      const int bx = a.cd[0] > 1, by = a.cd[1] > 1, bz = a.cd[2] > 1;
-      const VT* e0 = e + ix + cx * iy + cxy * iz;
       VT s = 0;
 #pragma unroll
       for (int cnr = 0; cnr < 8; cnr++) {
         const int dx = cnr & 1, dy = (cnr >> 1) & 1, dz = cnr >> 2;
         if ((dx && !bx) || (dy && !by) || (dz && !bz)) continue;
         const VT w = (dx ? fx : 1 - fx) * (dy ? fy : 1 - fy) * (dz ? fz : 1 - fz);
-        s += w * e0[dx + cx * dy + cxy * dz];
+        s += w * e[e0 + dx + cx * dy + cxy * dz];
       }
       zi += s;
     }
-    if (y) zi += (VT)y[v] * ys;
+    if (y) zi += net * ys;
     z[p] = zi;
   }
 }
@@ -170,15 +191,19 @@ int grid_of(long long n, int threads) {
 
 template <class VT>
 cudaError_t launch_coarse_restrict(const CoarseArgs<VT>& a, const VT* r, float* c, const int* done, cudaStream_t s) {
-  // shared memory: G groups x fd[0] partials (G = 1 once fd[0] exceeds the block)
+  // shared memory: G groups x W partials (G = 1 once the range exceeds the block)
   if (a.fd[0] > 4096) return cudaErrorInvalidValue;
   for (int ax = 1; ax < 3; ax++) {  // support lines of a coarse pair: at most (2 h + 1)^2
     const double h = a.cd[ax] > 1 ? (double)(a.fd[ax] - 1) / (a.cd[ax] - 1) : 1.0;
     if (h > 15.0) return cudaErrorInvalidValue;
   }
-  const int G = a.fd[0] <= kRestrictThreads ? kRestrictThreads / a.fd[0] : 1;
-  const size_t sm = (size_t)G * a.fd[0] * sizeof(double);
-  return launch_k(a.pdl != 0, k_restrict<VT>, dim3(a.cd[1] * a.cd[2]), dim3(kRestrictThreads), sm, s, a, r, c, done);
+  // ranges of coarse x-nodes: two blocks per SM, at least eight nodes each (the
+  // fine ranges of neighbours overlap by a support); 49 pairs of the 24 x 24 x 160
+  // duct: 10.3 us in one range, 5.3 in five
+  const int pairs = a.cd[1] * a.cd[2];
+  const int nxs = std::max(1, std::min((2 * 148 + pairs - 1) / pairs, a.cd[0] / 8));
+  const size_t sm = (size_t)std::max(kRestrictThreads, a.fd[0]) * sizeof(double);
+  return launch_k(a.pdl != 0, k_restrict<VT>, dim3(pairs, nxs), dim3(kRestrictThreads), sm, s, a, r, c, done);
 }
 
 template <class VT>

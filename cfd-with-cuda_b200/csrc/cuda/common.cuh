@@ -129,7 +129,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, int* err, unsigned l
 // stream is still running: pdl_wait() returns once that kernel has finished
 // and its writes are visible (at once for a launch without the attribute),
 // and pdl_trigger() lets the kernel after this one launch as soon as every
-// block of this one has reached it.
+// block of this one has reached it.  A kernel that triggers after its own wait
+// promises its successor that everything before this kernel is complete, so
+// the successor may read that before it waits; one that triggers at its start
+// allows it constants only.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 

@@ -16,7 +16,13 @@
 // using q = Z p, (p_j, q_i) = 0 for i != j inside the window, and nd =
 // min(iteration, m) stored directions.  All dots are FP64; the last block to
 // finish sums the per-block partials in block order, so results do not
-// depend on which block finishes last.  The state words live in device
+// depend on which block finishes last.  The kernels are launched with
+// programmatic dependent launch and request what does not depend on their
+// predecessor before they wait for it; a run of 3 steps on the 64^3 cavity went
+// from 27.8 to 26.9 ms with it, on the 24 x 24 x 160 duct from 22.1 to 19.6 (1.5
+// of that from the restriction's ranges), on 16^3 one step from 2.72 to 2.34.
+// Checking the done flag before those requests cost more (2.5 us per kernel)
+// than the requests of iterations past the end do.  The state words live in device
 // memory, and every kernel returns at once when the done flag is set, so the
 // host can queue several iterations between status reads.
 #include <algorithm>
@@ -240,15 +246,11 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_fcg_spmv_dia(FcgArgs<double>
 }
 
 // DOTS = false: w = Z z only (the Jacobi part of the split iteration).
+// The first chunks of the matrix are requested before the wait for the
+// previous kernel (they do not depend on it).
 template <class VT, int MD, bool DOTS>
 __global__ void __launch_bounds__(kPcgThreads, 2) k_fcg_spmv_stencil(FcgArgs<VT> a) {
-  pdl_wait();
-  pdl_trigger();
-  if (*a.st.done) return;
   extern __shared__ __align__(16) unsigned char smem[];
-  const double* sc = a.st.sc;
-  const int m = (int)sc[kFcgM], it = (int)sc[kFcgIt];
-  const int nd = it < m ? it : m;
   const int n = a.n, fx = a.fd[0], fxy = a.fd[0] * a.fd[1];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nslices = (n + 31) >> 5;
@@ -264,18 +266,29 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_fcg_spmv_stencil(FcgArgs<VT>
   mbar_init_fence();
   __syncwarp();
   // the coefficients are read once per iteration: evict-first in L2, so the
-  // vectors and the coarse inverse stay
-  const unsigned long long once = l2_evict_first();
+  // vectors and the coarse inverse stay, but for the part that fits beside them
+  const unsigned long long once = l2_evict_first(), keep = l2_evict_last();
+  const int nkeep = (int)(total * a.keep_l2);
   auto issue = [&](int k) {  // chunk k of the warp's range into buffer k % kStBuf
     if (lane == 0 && k < total) {
       const int b = k % kStBuf;
       const VT* src = a.stencil + ((size_t)(s0 + k / 5) * 125 + (k % 5) * kStTaps) * 32;
       fence_proxy_async_smem();
       mbar_expect_tx(mbar + b, kChunkBytes);
-      bulk_g2s_hint(buf + (size_t)b * kStTaps * 32, src, kChunkBytes, mbar + b, once);
+      bulk_g2s_hint(buf + (size_t)b * kStTaps * 32, src, kChunkBytes, mbar + b, k < nkeep ? keep : once);
     }
   };
   for (int k = 0; k < kStBuf; k++) issue(k);
+  pdl_wait();
+  pdl_trigger();
+  if (*a.st.done) {
+    if (lane == 0)  // the copies in flight land before the block ends
+      for (int k = 0; k < kStBuf && k < total; k++) mbar_wait_bounded(mbar + k, 0u, a.st.timeout_ns);
+    return;
+  }
+  const double* sc = a.st.sc;
+  const int m = (int)sc[kFcgM], it = (int)sc[kFcgIt];
+  const int nd = it < m ? it : m;
   bool ok = true;
   int kfail = 0;
   const VT* __restrict__ z = a.z;
@@ -375,52 +388,77 @@ __global__ void __launch_bounds__(kCombineThreads) k_fcg_combine(FcgArgs<VT> a, 
   fcg_spmv_finish<MD>(a, v, nd, m, it);
 }
 
-template <class VT>
+// MD: directions at most.  Everything but w and the coefficients was complete
+// when the SpMV began, so the first elements' z, x, r, p and q are loaded before
+// the wait for it (slots of directions that do not exist yet hold values that
+// nothing uses).
+template <class VT, int MD>
 __global__ void __launch_bounds__(kFcgThreads) k_fcg_update(FcgArgs<VT> a) {
-  pdl_wait();
-  pdl_trigger();
-  if (*a.st.done) return;
+  pdl_trigger();  // the restriction reads only its tables before its wait
   const double* sc = a.st.sc;
-  const int m = (int)sc[kFcgM], it = (int)sc[kFcgIt];
-  const int nd = it < m ? it : m, slot = fcg_slot(it, m, (int)sc[kFcgAnchor]);
-  const VT alpha = (VT)sc[kFcgAlpha];
-  VT beta[kFcgMaxM];
-#pragma unroll
-  for (int j = 0; j < kFcgMaxM; j++) beta[j] = (VT)sc[kFcgBeta0 + j];
   const size_t n = (size_t)a.n;
-  double v[1] = {0};
   // UPD grid-stride elements per thread with all their loads issued before
   // any store (the element order, and so the order of the (r, r) sum, is the
   // grid-stride order)
   constexpr int UPD = 4;
   const int stride = gridDim.x * blockDim.x;
-  for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < a.n; i0 += UPD * stride) {
-    VT pi[UPD], qi[UPD], xo[UPD], ro[UPD];
+  int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  VT zo[UPD], xo[UPD], ro[UPD], po[UPD][MD], qo[UPD][MD];
+  auto load = [&](int nd) {
 #pragma unroll
     for (int u = 0; u < UPD; u++) {
       const int i = i0 + u * stride;
       if (i < a.n) {
-        pi[u] = a.z[i];
-        qi[u] = a.w[i];
+        zo[u] = a.z[i];
         xo[u] = a.x[i];
         ro[u] = a.r[i];
 #pragma unroll
-        for (int j = 0; j < kFcgMaxM; j++) {
+        for (int j = 0; j < MD; j++) {
           if (j < nd) {
-            pi[u] -= beta[j] * a.p[j * n + i];
-            qi[u] -= beta[j] * a.q[j * n + i];
+            po[u][j] = a.p[j * n + i];
+            qo[u][j] = a.q[j * n + i];
           }
         }
       }
+    }
+  };
+  constexpr bool early = MD <= 2;  // more directions: too many registers to hold
+  if (early) load(MD);
+  pdl_wait();
+  if (*a.st.done) return;
+  const int m = (int)sc[kFcgM], it = (int)sc[kFcgIt];
+  const int nd = it < m ? it : m, slot = fcg_slot(it, m, (int)sc[kFcgAnchor]);
+  bool loaded = early;
+  const VT alpha = (VT)sc[kFcgAlpha];
+  VT beta[MD];
+#pragma unroll
+  for (int j = 0; j < MD; j++) beta[j] = (VT)sc[kFcgBeta0 + j];
+  double v[1] = {0};
+  for (; i0 < a.n; i0 += UPD * stride) {
+    if (!loaded) load(nd);
+    loaded = false;
+    VT wo[UPD];
+#pragma unroll
+    for (int u = 0; u < UPD; u++) {
+      const int i = i0 + u * stride;
+      if (i < a.n) wo[u] = a.w[i];
     }
 #pragma unroll
     for (int u = 0; u < UPD; u++) {
       const int i = i0 + u * stride;
       if (i < a.n) {
-        a.p[slot * n + i] = pi[u];
-        a.q[slot * n + i] = qi[u];
-        a.x[i] = xo[u] + alpha * pi[u];
-        const VT ri = ro[u] - alpha * qi[u];
+        VT pi = zo[u], qi = wo[u];
+#pragma unroll
+        for (int j = 0; j < MD; j++) {
+          if (j < nd) {
+            pi -= beta[j] * po[u][j];
+            qi -= beta[j] * qo[u][j];
+          }
+        }
+        a.p[slot * n + i] = pi;
+        a.q[slot * n + i] = qi;
+        a.x[i] = xo[u] + alpha * pi;
+        const VT ri = ro[u] - alpha * qi;
         a.r[i] = ri;
         if (a.z1) a.z1[i] = a.dinv[i] * ri;
         v[0] += (double)ri * ri;
@@ -482,6 +520,16 @@ int nblocks(int n) {
 
 int fcg_blocks(int n) { return nblocks(n); }
 size_t stencil_elems(int n) { return (size_t)((n + 31) >> 5) * 125 * 32; }
+// About 70 MB of the 126 MB L2 can be held from one iteration to the next (the
+// FP64 solver's sweep, dia.cuh), less the coarse inverse, and not more than 0.6
+// of the matrix.  us per SpMV at 0 / 0.1 / 0.2 / 0.4 / 0.6: 24.6 / 23.6 / 24.0 /
+// 25.2 / 26.6 on the 65^3 grid (137 MB, inverse 48 MB), 16.0 / 16.0 / 14.7 /
+// 14.7 / 14.3 on 161 x 25 x 25 (50 MB, 8 MB), 16.1 / 16.1 / 14.9 / 14.6 / 14.7
+// on 49^3 (59 MB, 10 MB).
+float stencil_keep_fraction(int n, double inv_bytes) {
+  const double bytes = (double)stencil_elems(n) * sizeof(float);
+  return (float)std::max(0.0, std::min(0.6, (70e6 - inv_bytes) / bytes));
+}
 size_t zp_elems(int n) { return (size_t)((n + 31) >> 5) * 27 * 32; }
 int fcg_part_words(int n) { return kFcgParts * (nblocks(n) > kFcgMaxBlocks ? nblocks(n) : kFcgMaxBlocks); }
 
@@ -563,7 +611,8 @@ template <class VT>
 cudaError_t launch_fcg_update(const FcgArgs<VT>& a, cudaStream_t s) {
   int grid = nblocks(a.n);
   if (a.upd_grid > 0 && a.upd_grid < grid) grid = a.upd_grid;
-  return launch_k(a.pdl != 0, k_fcg_update<VT>, dim3(grid), dim3(kFcgThreads), 0, s, a);
+  auto k = a.st.m == 1 ? k_fcg_update<VT, 1> : a.st.m == 2 ? k_fcg_update<VT, 2> : k_fcg_update<VT, kFcgMaxM>;
+  return launch_k(a.pdl != 0, k, dim3(grid), dim3(kFcgThreads), 0, s, a);
 }
 
 template <class VT>

@@ -283,6 +283,7 @@ template <class VT> struct FcgArgs {
   int pdl;  // 1: the iteration kernels launch with programmatic dependent launch
   DiaArgs dia;   // ntap > 0: the matrix by offsets, used by the FP64 SpMV instead of the SELL arrays
   int dia_grid;  // blocks of that SpMV
+  float keep_l2;  // part of the structured matrix asked to stay in L2 (stencil_keep_fraction)
   int upd_grid;  // > 0: blocks of the update kernel (default: one thread per entry, at most kFcgMaxBlocks)
 };
 struct Int3 {
@@ -293,6 +294,9 @@ struct Int3 {
 // 32-row slices (stencil_elems(n) entries); *bad (host-zeroed) is set when a
 // coupling reaches further than two grid steps (the form does not apply).
 size_t stencil_elems(int n);
+// Part of the FP32 structured matrix of n rows that the SpMV asks to stay in L2
+// beside the coarse inverse of inv_bytes.
+float stencil_keep_fraction(int n, double inv_bytes);
 template <class VT>
 cudaError_t launch_stencil_build(int n, const int fd[3], const int* rp, const int* col, const double* val, VT* coef,
                                  int* bad, cudaStream_t s);
