@@ -17,6 +17,7 @@
 #include <cstdlib>
 #include <atomic>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <string>
 #include <utility>
@@ -44,8 +45,8 @@ struct cfd_unet {
 };
 
 namespace {
-constexpr int kFcgBatch = 4;  // flexible-CG iterations per captured graph
-// An instantiated graph of kFcgBatch flexible-CG iterations and the buffers
+constexpr int kFcgBatch = 4;  // flexible-CG iterations per captured graph (and a graph of one)
+// An instantiated graph of flexible-CG iterations and the buffers
 // and network state it was captured with.
 struct FcgGraph {
   struct Key {
@@ -208,12 +209,18 @@ struct cfd_ctx {
   // [window m = 1, m > 1]: the first inner solve of a mixed pressure solve
   // keeps the network's directions and the refinement solves do not, so
   // each window has its own graph instead of a re-capture per solve
-  FcgGraph fcg_graph[2][2][2];
+  // [kFcgBatch iterations (or the network's head), one iteration]
+  FcgGraph fcg_graph[2][2][2][2];
   void reset_fcg_graphs() {
     for (auto& gp : fcg_graph)
       for (auto& gq : gp)
-        for (auto& g : gq) g.reset();
+        for (auto& gr : gq)
+          for (auto& g : gr) g.reset();
   }
+  // ln of the mean residual reduction per iteration in the last solve from x0
+  // = 0 of each kind [FP32, FP64][first solve, refinement, network] (0: none
+  // yet): how many iterations to queue before the first look at a solve
+  double fcg_lnrate[2][3] = {};
   // CFD_FCG_PERSIST=1: the persistent two-level iteration (fcg_persist.cu)
   // for the FP32 inner solves on a structured grid instead of the per-kernel
   // iteration graphs; measured slower on the 64^3 cavity (about 85 against
@@ -1209,8 +1216,13 @@ int run_fcg2l(cfd_ctx* c, const FcgArgs<float>& a, const CoarseArgs<float>& ca) 
 // CFD_MIXED); VT = double: b, x are the caller's FP64 vectors.  The coarse
 // space must be built (ensure_coarse) before.  res = {iterations,
 // ||r||/||b||, status} with the status words of kernels.h (4 = stalled).
+// after (may be null): queues what follows the solve, before each look at its
+// state; its kernels have to do nothing while *fcg_done is 0.  *followed tells
+// whether the last of them ran.  The word fcg_sc[kFcgScalars] is read back
+// with the state (into h_small).
 template <class VT>
-int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, double* res, bool first_solve) {
+int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, double* res, bool first_solve,
+            const std::function<int()>& after = nullptr, bool* followed = nullptr) {
   cudaStream_t s = c->stream;
   const int n = c->P.NNp;
   // with fcg_net_iters > 0 the network serves the head of the first inner
@@ -1221,7 +1233,7 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
   UnetNet* netp = use_net ? &c->unet->net : nullptr;
   if (netp && netp->set_grid(c->udims, false)) return fail(c, CFD_E_NOMEM, "%s", netp->err.c_str());
   if (!c->fcg_sc.p) {
-    CU(c->fcg_sc.alloc(kFcgScalars));
+    CU(c->fcg_sc.alloc(kFcgScalars + 1));
     CU(c->fcg_part.alloc((size_t)fcg_part_words(n)));
     CU(c->fcg_cnt.alloc(1));
     CU(cudaMemsetAsync(c->fcg_cnt.p, 0, sizeof(unsigned), s));
@@ -1382,11 +1394,11 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
   // captured once per buffer / network configuration and replayed until the
   // done flag stops the kernels
   const int net_iters = !netp ? 0 : (c->opt.fcg_net_iters > 0 ? c->opt.fcg_net_iters : 1 << 30);
-  auto graph_for = [&](bool with_net, int iters, FcgGraph*& out) -> int {
+  auto graph_for = [&](bool with_net, int iters, bool single, FcgGraph*& out) -> int {
     out = nullptr;
     if (!c->fcg_use_graph || c->prof_on) return CFD_OK;
     if (with_net) CU(netp->prepare_tc(s));  // packs and plans outside the capture
-    FcgGraph& g = c->fcg_graph[sizeof(VT) == 4 ? 0 : 1][with_net ? 1 : 0][a.st.m > 1 ? 1 : 0];
+    FcgGraph& g = c->fcg_graph[sizeof(VT) == 4 ? 0 : 1][with_net ? 1 : 0][a.st.m > 1 ? 1 : 0][single ? 1 : 0];
     FcgGraph::Key key{a.b, a.x, a.r, with_net ? c->unet : nullptr, with_net ? netp->gen : 0,
                       with_net ? netp->plan_gen : 0, with_net ? netp->tc_enabled : false, pmap, dinv,
                       c->unet_dscale, n, c->coarse_gen, iters, a.st.m};
@@ -1418,17 +1430,29 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
   // where that applies
   bool persist = false;
   if constexpr (sizeof(VT) == 4) persist = !net_all && !split && fcg2l_fits(c, a, ca);
-  FcgGraph *G = nullptr, *GH = nullptr;
+  FcgGraph *G = nullptr, *G1 = nullptr, *GH = nullptr;
   {
-    int rc = persist ? CFD_OK : graph_for(net_all, kFcgBatch, G);
+    int rc = persist ? CFD_OK : graph_for(net_all, kFcgBatch, false, G);
+    if (!rc && !persist) rc = graph_for(net_all, 1, true, G1);
     if (rc) return rc;
     if (head > 0) {
-      rc = graph_for(true, std::min(head, kFcgBatch), GH);
+      rc = graph_for(true, std::min(head, kFcgBatch), false, GH);
       if (rc) return rc;
     }
   }
-  int issued = 0, batch = 2;
+  int issued = 0, batch = kFcgBatch;
   double rr_prev = -1;
+  bool ran_after = false;
+  auto look = [&]() -> int {  // the solve's state into h_small
+    if (after) {
+      int rc = after();
+      if (rc) return rc;
+    }
+    CU(cudaMemcpyAsync(c->h_small, c->fcg_sc.p, (kFcgScalars + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CU(cudaStreamSynchronize(s));
+    ran_after = after && c->h_small[kFcgStatus] >= 0;
+    return CFD_OK;
+  };
   if (head > 0) {
     // the network's iterations first, then the two-level part alone
     const int hb = std::min(head, kFcgBatch);
@@ -1448,20 +1472,24 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
   if constexpr (sizeof(VT) == 4) {
     if (persist) {
       int rc = run_fcg2l(c, a, ca);
+      if (!rc) rc = look();
       if (rc) return rc;
-      CU(cudaMemcpyAsync(c->h_small, c->fcg_sc.p, kFcgScalars * sizeof(double), cudaMemcpyDeviceToHost, s));
-      CU(cudaStreamSynchronize(s));
       if (c->prof_on) c->prof[CFD_K_FCG2L][2] += c->h_small[kFcgIt] - issued;
     }
   }
-  for (; !persist;) {
-    if (G) {
-      const int reps = (batch + kFcgBatch - 1) / kFcgBatch;
-      for (int k = 0; k < reps; k++) {
-        CU(cudaGraphLaunch(G->exec, s));
-        c->launches += G->launches;
+  // a solve from x0 = 0 is expected to take as many iterations as the last of
+  // its kind, scaled to its target
+  double& lnrate = c->fcg_lnrate[sizeof(VT) == 4 ? 0 : 1][use_net ? 2 : first_solve ? 0 : 1];
+  if (!warm && lnrate < 0) batch = (int)std::lround(std::log(rtol) / lnrate + 0.2) - issued;
+  while (!persist) {
+    batch = std::max(1, std::min({batch, 64, std::max(1, maxit - issued)}));
+    if (G && G1) {
+      for (int left = batch; left > 0;) {
+        FcgGraph* g = left >= kFcgBatch ? G : G1;
+        CU(cudaGraphLaunch(g->exec, s));
+        c->launches += g->launches;
+        left -= g->key.iters;
       }
-      batch = reps * kFcgBatch;
     } else {
       for (int k = 0; k < batch; k++) {
         int rc = iteration(true, net_all);
@@ -1469,24 +1497,28 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
       }
     }
     issued += batch;
-    CU(cudaMemcpyAsync(c->h_small, c->fcg_sc.p, kFcgScalars * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
+    int rc = look();
+    if (rc) return rc;
     const double* h = c->h_small;
     if (h[kFcgStatus] >= 0 || issued >= maxit) break;
     // size the next batch from the observed convergence rate
     const double rr = h[kFcgRR], target = rtol * rtol * h[kFcgBB];
+    const double from = rr_prev > 0 ? rr_prev : (warm ? -1 : h[kFcgBB]);
+    const int span = rr_prev > 0 ? batch : issued;
     int next = 4;
-    if (rr_prev > 0 && rr > 0 && rr < rr_prev) {
-      const double rate = std::log(rr / rr_prev) / batch;  // per iteration, < 0
+    if (from > 0 && rr > 0 && rr < from) {
+      const double rate = std::log(rr / from) / span;  // per iteration, < 0
       next = (int)std::ceil(std::log(target / rr) / rate);
     }
     rr_prev = rr;
-    batch = std::max(1, std::min(next, 16));
+    batch = std::min(next, 16);
   }
   const double* h = c->h_small;
   res[0] = h[kFcgIt];
   res[1] = h[kFcgBB] > 0 ? std::sqrt(h[kFcgRR] / h[kFcgBB]) : 0.0;
   res[2] = h[kFcgStatus] < 0 ? 1 : h[kFcgStatus];
+  if (followed) *followed = ran_after;
+  if (!warm && h[kFcgStatus] == 0 && res[0] > 0 && res[1] > 0 && res[1] < 1) lnrate = std::log(res[1]) / res[0];
   if (c->prof_on && !persist) {
     c->prof[CFD_K_FCG][2] += res[0];
     c->prof[CFD_K_SPMV_Z][2] += res[0];
@@ -1499,18 +1531,40 @@ bool twolevel(const cfd_ctx* c) { return c->opt.precond == CFD_PC_TWOLEVEL; }
 // solves that run flexible CG with a coarse space (and, when learned, the network)
 bool fcg_path(const cfd_ctx* c) { return learned(c) || twolevel(c); }
 
-// ||b - Z x||_2 in FP64 (also leaves r in ir_r and (float) r in f_b).
-int residual_norm(cfd_ctx* c, const double* b, const double* x, double* out) {
+// Queues r = b - Z x in FP64 (into ir_r, and (float) r into f_b) and *out =
+// ||r||_2^2 (device); when as launch_residual64.
+int queue_residual(cfd_ctx* c, const double* b, const double* x, double* out, const int* when = nullptr) {
   cudaStream_t s = c->stream;
   int nparts = c->res_blocks;
   if (x && c->dia_apply > 0) {
     nparts = c->dia_apply;
-    KL(CFD_K_RESID64, launch_residual_dia(c->dia(), b, x, c->ir_r.p, c->f_b.p, c->ir_part.p, nparts, s));
+    KL(CFD_K_RESID64, launch_residual_dia(c->dia(), b, x, c->ir_r.p, c->f_b.p, c->ir_part.p, nparts, when, s));
   } else {
     KL(CFD_K_RESID64, launch_residual64(c->P.NNp, c->zs_off.p, c->zs_col.p, c->zs_val.p, b, x, c->ir_r.p, c->f_b.p,
-                                        c->ir_part.p, c->res_blocks, s));
+                                        c->ir_part.p, c->res_blocks, when, s));
   }
-  KL(CFD_K_OTHER, launch_sum_partials(c->ir_part.p, nparts, c->ir_sum.p, s));
+  KL(CFD_K_OTHER, launch_sum_partials(c->ir_part.p, nparts, out, s));
+  return CFD_OK;
+}
+
+// ||b||_2 and ||b - Z x||_2 (x may be null: the same) with one wait.
+int residual_norms(cfd_ctx* c, const double* b, const double* x, double* bnorm, double* rnorm) {
+  cudaStream_t s = c->stream;
+  int rc = queue_residual(c, b, nullptr, c->ir_sum.p);
+  if (!rc && x) rc = queue_residual(c, b, x, c->ir_sum.p + 1);
+  if (rc) return rc;
+  CU(cudaMemcpyAsync(c->h_small, c->ir_sum.p, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  CU(cudaStreamSynchronize(s));
+  *bnorm = std::sqrt(c->h_small[0]);
+  *rnorm = x ? std::sqrt(c->h_small[1]) : *bnorm;
+  return CFD_OK;
+}
+
+// ||b - Z x||_2 in FP64 (also leaves r in ir_r and (float) r in f_b).
+int residual_norm(cfd_ctx* c, const double* b, const double* x, double* out) {
+  cudaStream_t s = c->stream;
+  int rc = queue_residual(c, b, x, c->ir_sum.p);
+  if (rc) return rc;
   CU(cudaMemcpyAsync(c->h_small, c->ir_sum.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
   *out = std::sqrt(c->h_small[0]);
@@ -1551,8 +1605,9 @@ int pressure_solve(cfd_ctx* c, const double* b, double* x, int warm, cfd_solve_s
     cudaStream_t s = c->stream;
     if (!warm) CU(cudaMemsetAsync(x, 0, c->P.NNp * sizeof(double), s));
     double bnorm = 0, rnorm = 0;
-    // ||b|| (x = 0: the residual is b itself, and f_b = b for the first inner solve)
-    int rc = residual_norm(c, b, nullptr, &bnorm);
+    // ||b|| (x = 0: the residual is b itself, and f_b = b for the first inner
+    // solve) and, warm, the residual of the given x
+    int rc = residual_norms(c, b, warm ? x : nullptr, &bnorm, &rnorm);
     if (rc) return rc;
     if (!std::isfinite(bnorm)) {
       z.status = 2;
@@ -1560,9 +1615,6 @@ int pressure_solve(cfd_ctx* c, const double* b, double* x, int warm, cfd_solve_s
       CU(cudaMemsetAsync(x, 0, c->P.NNp * sizeof(double), s));
       z.status = 0;
     } else {
-      rnorm = bnorm;
-      if (warm) rc = residual_norm(c, b, x, &rnorm);
-      if (rc) return rc;
       z.status = 1;
       int total = 0;
       for (int outer = 0; outer <= c->opt.max_outer; outer++) {
@@ -1570,13 +1622,23 @@ int pressure_solve(cfd_ctx* c, const double* b, double* x, int warm, cfd_solve_s
         if (rnorm <= rtol * bnorm) { z.status = 0; break; }
         if (outer == c->opt.max_outer || total >= c->opt.cg_maxit) break;
         double res[4] = {0, 0, 0, 0};
+        double next_rnorm = -1;  // < 0: not known yet
         // inner target: inner_rtol relative, but no tighter than needed
         double inner = std::max(c->opt.inner_rtol, 0.5 * rtol * bnorm / rnorm);
         if (fcg_path(c) && !z.fallback) {
           rc = ensure_coarse(c);
           if (rc) return rc;
-          rc = run_fcg<float>(c, c->f_b.p, c->f_x.p, 0, inner, c->opt.cg_maxit - total, res, outer == 0);
+          // the update of x and the next residual are queued behind the solve
+          // and read back with its state
+          bool followed = false;
+          auto after = [&]() -> int {
+            KL(CFD_K_OTHER, launch_axpy_f2d(c->P.NNp, c->f_x.p, x, c->fcg_done.p, s));
+            return queue_residual(c, b, x, c->fcg_sc.p + kFcgScalars, c->fcg_done.p);
+          };
+          rc = run_fcg<float>(c, c->f_b.p, c->f_x.p, 0, inner, c->opt.cg_maxit - total, res, outer == 0, after,
+                              &followed);
           if (rc) return rc;
+          if (followed) next_rnorm = std::sqrt(c->h_small[kFcgScalars]);
           const int fs = (int)res[2];
           if (fs == 4 || fs == 2 || (fs == 1 && res[1] > 0.5)) z.fallback = 1;  // Jacobi-PCG from here on
           if (fs == 2) res[2] = 0;  // the iterate is still finite: the outer residual decides
@@ -1586,8 +1648,12 @@ int pressure_solve(cfd_ctx* c, const double* b, double* x, int warm, cfd_solve_s
         }
         total += (int)res[0];
         if ((int)res[2] == 3) { z.status = 3; break; }
-        KL(CFD_K_OTHER, launch_axpy_f2d(c->P.NNp, c->f_x.p, x, s));
         z.outer = outer + 1;
+        if (next_rnorm >= 0 || std::isnan(next_rnorm)) {
+          rnorm = next_rnorm;
+          continue;
+        }
+        KL(CFD_K_OTHER, launch_axpy_f2d(c->P.NNp, c->f_x.p, x, nullptr, s));
         rc = residual_norm(c, b, x, &rnorm);
         if (rc) return rc;
       }

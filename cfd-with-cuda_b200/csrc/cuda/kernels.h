@@ -211,9 +211,10 @@ struct PcgDiaArgs {
 int pcg_dia_grid(int n, int device);
 // Blocks of the one-pass kernels (0: n too large for them), and the residual
 // r = b - Z x with rf = (float) r (may be null) and per-block partials of r^2.
+// when (may be null): the kernel does nothing while *when is 0.
 int dia_apply_grid(int n, int num_sms);
 cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
-                                int grid, cudaStream_t s);
+                                int grid, const int* when, cudaStream_t s);
 cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s);
 template <class VT>
 struct PcgArgs {
@@ -442,12 +443,12 @@ template <class VT>
 int pcg_max_grid(int n, int device);
 
 // r = b - Z x (FP64, SELL-32 Z) and the partial sum of r^2 per block; rf = (float) r.
-// x == null stands for x = 0 (r = b, Z is not read).
+// x == null stands for x = 0 (r = b, Z is not read).  when as above.
 cudaError_t launch_residual64(int n, const int* off, const int* col, const double* val, const double* b,
-                              const double* x, double* r, float* rf, double* part, int nblocks,
+                              const double* x, double* r, float* rf, double* part, int nblocks, const int* when,
                               cudaStream_t s);
 int residual_blocks(int n, int num_sms);
-cudaError_t launch_axpy_f2d(int n, const float* e, double* x, cudaStream_t s);
+cudaError_t launch_axpy_f2d(int n, const float* e, double* x, const int* when, cudaStream_t s);
 cudaError_t launch_sum_partials(const double* part, int n, double* out, cudaStream_t s);
 
 // CSR values -> SELL-32 values (padding entries set to 0).

@@ -223,7 +223,8 @@ __global__ void __launch_bounds__(kResThreads) k_residual64(int n, const int* __
                                                              const double* __restrict__ val,
                                                              const double* __restrict__ b,
                                                              const double* __restrict__ x, double* r, float* rf,
-                                                             double* part) {
+                                                             double* part, const int* when) {
+  if (when && *when == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double acc[1] = {0};
   if (i < n) {
@@ -243,7 +244,8 @@ __global__ void __launch_bounds__(kResThreads) k_residual64(int n, const int* __
   if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
 }
 
-__global__ void k_axpy_f2d(int n, const float* __restrict__ e, double* x) {
+__global__ void k_axpy_f2d(int n, const float* __restrict__ e, double* x, const int* when) {
+  if (when && *when == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] += (double)e[i];
 }
 
@@ -340,14 +342,15 @@ cudaError_t launch_pcg(const PcgArgs<VT>& a, int grid, cudaStream_t s) {
 int residual_blocks(int n, int) { return std::max(1, (n + kResThreads - 1) / kResThreads); }
 
 cudaError_t launch_residual64(int n, const int* off, const int* col, const double* val, const double* b,
-                              const double* x, double* r, float* rf, double* part, int nblocks, cudaStream_t s) {
-  k_residual64<<<nblocks, kResThreads, 0, s>>>(n, off, col, val, b, x, r, rf, part);
+                              const double* x, double* r, float* rf, double* part, int nblocks, const int* when,
+                              cudaStream_t s) {
+  k_residual64<<<nblocks, kResThreads, 0, s>>>(n, off, col, val, b, x, r, rf, part, when);
   return cudaGetLastError();
 }
 
-cudaError_t launch_axpy_f2d(int n, const float* e, double* x, cudaStream_t s) {
+cudaError_t launch_axpy_f2d(int n, const float* e, double* x, const int* when, cudaStream_t s) {
   int g = std::max(1, std::min((n + 255) / 256, 148 * 8));
-  k_axpy_f2d<<<g, 256, 0, s>>>(n, e, x);
+  k_axpy_f2d<<<g, 256, 0, s>>>(n, e, x, when);
   return cudaGetLastError();
 }
 

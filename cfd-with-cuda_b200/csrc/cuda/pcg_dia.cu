@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
 // SELL-32 form, 47 here).
 __global__ void __launch_bounds__(kDiaThreads, 1) k_residual_dia(DiaArgs d, const double* __restrict__ b,
                                                                  const double* __restrict__ x, double* r, float* rf,
-                                                                 double* part) {
+                                                                 double* part, const int* when) {
+  if (when && *when == 0) return;
   extern __shared__ double sv[];
   __shared__ int soff[kDiaMaxTaps + kDiaGroup];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -256,12 +257,13 @@ cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s) {
 int dia_apply_grid(int n, int num_sms) { return dia_blocks(n, num_sms); }
 
 cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
-                                int grid, cudaStream_t s) {
+                                int grid, const int* when, cudaStream_t s) {
   const int ns = (d.n + 31) / 32;
   if (grid < 1 || grid > ns || d.ntap < 1 || d.ntap > kDiaMaxTaps) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(k_residual_dia, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem);
   if (e != cudaSuccess) return e;
-  k_residual_dia<<<grid, kDiaThreads, dia_slot_bytes((ns + grid - 1) / grid), s>>>(d, b, x, r, rf, part);
+  k_residual_dia<<<grid, kDiaThreads, dia_slot_bytes((ns + grid - 1) / grid), s>>>(d, b, x, r, rf, part,
+                                                                                       when);
   return cudaGetLastError();
 }
 
