@@ -214,7 +214,8 @@ def step_bytes(info, steps, subiters, cg_iters, mixed, structured=False):
     sub-iteration the convection, step1 (K u, G p, update), G^T, step3 and
     about 12 element-wise passes over the FP64 state; per CG iteration
     cg_iteration_bytes; one K Acc pass per sub-iteration that did not end
-    its step (subiters - steps, exact when no step ran out)."""
+    its step (subiters - steps, exact when no step ran out), counted as a pass
+    of its own although a run shares step 1's."""
     per_sub = (algorithmic_bytes(info, "convect", 0, mixed) + algorithmic_bytes(info, "step1", 0, mixed)
                + algorithmic_bytes(info, "gt", 0, mixed) + algorithmic_bytes(info, "step3", 0, mixed)
                + 12 * 3 * info.NN * 8)

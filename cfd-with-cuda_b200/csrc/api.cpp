@@ -1682,7 +1682,34 @@ int reduce_norms(cfd_ctx* c) {
 
 bool mixed(const cfd_ctx* c) { return c->opt.precision == CFD_MIXED; }
 
-
+// step 1; with_kacc: K Acc_prev too, in the same pass over K (iter > 1).
+int step1(cfd_ctx* c, int iter, bool with_kacc) {
+  NEED(c->assembled && iter >= 1, "cfd_step1: bad state or iter");
+  cudaStream_t s = c->stream;
+  auto fill = [&](auto& a) {
+    a.NN = c->P.NN; a.iter = iter; a.dt = c->P.dt;
+    a.k_off = c->ks_off.p; a.k_col = c->ks_col.p; a.g_off = c->gs_off.p; a.g_col = c->gs_col.p;
+    a.un = c->un; a.r1conv = c->r1conv; a.kacc = c->kacc;
+    a.pn = c->pn; a.minv_free = c->minv_free.p; a.minv_orig = c->minv_orig.p;
+    a.unphalf = c->unphalf; a.d = c->dvec; a.r1out = c->r_debug ? c->r1dbg : nullptr;
+  };
+  if (mixed(c)) {
+    Step1Args<float> a{};
+    fill(a);
+    a.uprev = c->uphp32; a.accprev = with_kacc ? c->accp32 : nullptr; a.unphalf_g = c->uph32; a.d_g = c->d32;
+    a.r1conv32 = c->r1c32;
+    a.kval = c->ks_val32.p; a.g1 = c->gs1_32.p; a.g2 = c->gs2_32.p; a.g3 = c->gs3_32.p;
+    KL(CFD_K_STEP1, launch_step1<float>(a, c->num_sms, s));
+  } else {
+    Step1Args<double> a{};
+    fill(a);
+    a.uprev = c->unphalf_prev;
+    a.accprev = with_kacc ? c->acc_prev : nullptr;
+    a.kval = c->ks_val.p; a.g1 = c->gs1.p; a.g2 = c->gs2.p; a.g3 = c->gs3.p;
+    KL(CFD_K_STEP1, launch_step1<double>(a, c->num_sms, s));
+  }
+  return CFD_OK;
+}
 
 }  // namespace
 
@@ -1992,30 +2019,7 @@ int cfd_convect(cfd_ctx* c) {
 
 int cfd_step1(cfd_ctx* c, int iter) {
   if (!c) return CFD_E_BADARG;
-  NEED(c->assembled && iter >= 1, "cfd_step1: bad state or iter");
-  cudaStream_t s = c->stream;
-  auto fill = [&](auto& a) {
-    a.NN = c->P.NN; a.iter = iter; a.dt = c->P.dt;
-    a.k_off = c->ks_off.p; a.k_col = c->ks_col.p; a.g_off = c->gs_off.p; a.g_col = c->gs_col.p;
-    a.un = c->un; a.r1conv = c->r1conv; a.kacc = c->kacc;
-    a.pn = c->pn; a.minv_free = c->minv_free.p; a.minv_orig = c->minv_orig.p;
-    a.unphalf = c->unphalf; a.d = c->dvec; a.r1out = c->r_debug ? c->r1dbg : nullptr;
-  };
-  if (mixed(c)) {
-    Step1Args<float> a{};
-    fill(a);
-    a.uprev = c->uphp32; a.unphalf_g = c->uph32; a.d_g = c->d32;
-    a.r1conv32 = c->r1c32;
-    a.kval = c->ks_val32.p; a.g1 = c->gs1_32.p; a.g2 = c->gs2_32.p; a.g3 = c->gs3_32.p;
-    KL(CFD_K_STEP1, launch_step1<float>(a, c->num_sms, s));
-  } else {
-    Step1Args<double> a{};
-    fill(a);
-    a.uprev = c->unphalf_prev;
-    a.kval = c->ks_val.p; a.g1 = c->gs1.p; a.g2 = c->gs2.p; a.g3 = c->gs3.p;
-    KL(CFD_K_STEP1, launch_step1<double>(a, c->num_sms, s));
-  }
-  return CFD_OK;
+  return step1(c, iter, false);
 }
 
 int cfd_step2(cfd_ctx* c, int iter, cfd_solve_stats* st) {
@@ -2149,7 +2153,8 @@ int cfd_run(cfd_ctx* c, int nsteps, cfd_run_stats* st) {
     for (iter = 1; iter <= P.maxIter; iter++) {
       cfd_solve_stats ss{};
       if ((rc = cfd_convect(c))) return rc;
-      if ((rc = cfd_step1(c, iter))) return rc;
+      // K Acc_prev of the rotated acceleration rides on step 1's pass over K
+      if ((rc = step1(c, iter, iter > 1))) return rc;
       if ((rc = cfd_step2(c, iter, &ss))) return rc;
       if ((rc = cfd_step3(c, iter))) return rc;
       r.cg_iters += ss.iterations;
@@ -2159,7 +2164,8 @@ int cfd_run(cfd_ctx* c, int nsteps, cfd_run_stats* st) {
       if ((rc = cfd_check_iter(c, P.tolerance, &conv, nullptr))) return rc;
       if (conv) break;
       cfd_rotate(c);
-      if ((rc = cfd_k_times_acc(c))) return rc;
+      // no next step 1 in this step: leave K Acc_prev as the reference does
+      if (iter == P.maxIter && (rc = cfd_k_times_acc(c))) return rc;
     }
     r.last_iter = iter;
     int steady = 0;

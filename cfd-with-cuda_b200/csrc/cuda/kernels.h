@@ -114,7 +114,11 @@ struct Step1Args {
   const int *g_off, *g_col;  // SELL-32
   const VT *g1, *g2, *g3;
   const GVec<VT>* uprev;  // UnpHalf_prev, gathered by K
-  const double4 *un, *r1conv, *kacc;
+  // not null: K Acc_prev is computed here too, in the same pass over K, and
+  // stored into kacc (else kacc is read)
+  const GVec<VT>* accprev;
+  const double4 *un, *r1conv;
+  double4* kacc;
   const float4* r1conv32;  // may be null: the FP32 convection term, read instead of r1conv
   const double *pn, *minv_free, *minv_orig;
   double4 *unphalf, *d, *r1out;  // r1out may be null

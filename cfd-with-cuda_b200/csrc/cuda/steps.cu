@@ -20,6 +20,8 @@
 // read with streaming (evict-first) loads so the gathered vectors stay in
 // L2.  Matrix values are VT (double or float, accumulated in VT); vectors
 // stay FP64.
+#include <type_traits>
+
 #include "kernels.h"
 
 namespace cfd {
@@ -52,6 +54,9 @@ inline int rows_grid(long long rows) {
 //   k_spmv_k3  16 / 14 / 9.2 / 7.0  36/30/17/13      39/33/29/40      59 / 108 / 118 / 170
 //   k_step3    8.7/ 6.1/ 4.8/ 4.3   17/9.8/7.0/10    20/14/18/25      40 / 52 / 67 / 107
 //   k_gt       30 / 24 / 13 / 8.3   60/46/25/14      72/55/30/17      75 / 58 / 37 / 37   114/130/122/131
+// (taken before the loads were ordered as at for_entries, which moved both sides
+// of each line alike: at the chosen split, FP64 n = 8 step 1 10 -> 7.2, n = 32
+// k_gt 28 -> 26, FP32 n = 24 k_spmv_k3 29 -> 24)
 // and k_gt in FP64 at n = 64 193 / 188 / 191 / 187, in FP32 on the duct of 24
 // x 24 x 160 (3145 slices) 78 / 63 / 63 / 53.
 struct SplitRule {
@@ -70,30 +75,84 @@ inline int row_split(long long rows, const SplitRule& rule) {
 constexpr int block_threads(int split) { return split == 1 ? kRowThreads : 32 * split; }
 inline int split_grid(long long rows, int sp) { return sp == 1 ? rows_grid(rows) : (int)((rows + 31) / 32); }
 
+// What is read in order for one entry: the value(s) and the column.
+template <class T>
+struct KEntry {
+  int c;
+  T v;
+};
+template <class T>
+struct GEntry {
+  int c;
+  T x, y, z;
+};
 // One entry of a row and the vector values it multiplies.
 template <class T>
 struct alignas(4 * sizeof(T)) Entry {
   T a, b, c, d;
 };
+// The same for two vectors.
+template <class T>
+struct Entry2 {
+  T a, b, c, d, x, y, z;
+};
 // Shared memory of a split slice: FP32 entries on their way to the first
 // warp, or NV FP64 partial sums of every warp.
 template <class VT, class E, int NV, int SPLIT>
-struct SplitBuf {
+struct alignas(32) SplitBuf {  // an Entry2 buffer is read as one of Entry too
   static constexpr bool ordered = sizeof(VT) == 4;
   union {
     E e[ordered ? 4 * SPLIT : 1][32];
     VT v[ordered ? 1 : SPLIT][NV][32];
   };
 };
-// Entries of a slice's rows, w of them: load(j) fetches entry j of the
-// thread's row, use(e) consumes it.  FP32 with SPLIT > 1: each of the block's
-// warps loads four of the next 4 SPLIT entries (the loads of the next group
-// are in flight while the first warp consumes the current one).
-template <int SPLIT, class B, class L, class U>
-__device__ __forceinline__ void for_entries(B& buf, int w, L load, U use) {
-  if constexpr (SPLIT == 1) {
+// Entries of a slice's rows, w of them: stream(j) reads entry j of the thread's
+// row, gather its vector values, use consumes both, in order.  FP32 with SPLIT
+// > 1: each of the block's warps loads four of the next 4 SPLIT entries (the
+// loads of the next group are in flight while the first warp consumes the
+// current one).
+//
+// SPLIT = 1, one thread per row: every entry is a chain of column -> gather ->
+// FMA, and what bounds a launch is how many chains its warps keep in flight
+// against how much of the gathered vector the L1 keeps between them.  D = 0
+// leaves the order to the compiler (unrolled by four); D > 0 gathers D entries
+// together while the next D are read.  More D means more registers, fewer warps
+// and a wider front of columns, so the best is small and differs by kernel (us
+// on the 64^3 cavity, duct of 24 x 24 x 160 in brackets; K / G loop of step 1):
+//   FP32  step 1 D = 0/0 369..456 (135..167)   0/2 373 (135)    2/2 458  4/4 389  8/8 454
+//         with K Acc_prev  0/0 704 (261)  2/2 523 (191)  3/2 494 (181)  3/3 474 (174)  4/4 491  8/8 636
+//         step 3  0 160  1 187  2 163  4 174  8 196     K v  0 228  1 303  2 229  3 293  8 340
+//         G^T  0 113  1 131  2 116  3 122  4 149
+//   FP64  step 1 0/0 637  2/0 550  2/2 576  3/3 627  4/4 700  8/8 847
+//         with K Acc_prev  0/0 880  0/2 841  2/2 890  4/4 961
+//         step 3  0 217  1 211  2 213  4 219  8 373     K v  0 414  1 462  2 404  4 418  8 498
+// The column is read before the value where it is the head of the chain (split
+// slices, K v FP32 on 24^3 elements 29 -> 24, G^T FP64 at 64^3 191 -> 175, FP32 on
+// the duct 56 -> 52); in step 1's FP32 K loop the value goes first (3/3 with K
+// Acc_prev 488 -> 474).
+template <int SPLIT, int D, class B, class S, class G, class U>
+__device__ __forceinline__ void for_entries(B& buf, int w, S stream, G gather, U use) {
+  auto load = [&](int j) { return gather(stream(j)); };
+  if constexpr (SPLIT == 1 && D == 0) {
 #pragma unroll 4
     for (int j = 0; j < w; j++) use(load(j));
+  } else if constexpr (SPLIT == 1) {
+    decltype(stream(0)) st[D];
+#pragma unroll
+    for (int i = 0; i < D; i++)
+      if (i < w) st[i] = stream(i);
+    for (int j0 = 0; j0 < w; j0 += D) {
+      decltype(load(0)) e[D];
+#pragma unroll
+      for (int i = 0; i < D; i++)
+        if (j0 + i < w) e[i] = gather(st[i]);
+#pragma unroll
+      for (int i = 0; i < D; i++)
+        if (j0 + D + i < w) st[i] = stream(j0 + D + i);
+#pragma unroll
+      for (int i = 0; i < D; i++)
+        if (j0 + i < w) use(e[i]);
+    }
   } else if constexpr (!B::ordered) {
 #pragma unroll 4
     for (int j = threadIdx.x >> 5; j < w; j += SPLIT) use(load(j));
@@ -143,42 +202,76 @@ __device__ __forceinline__ void split_sum(B& buf, VT (&v)[NV]) {
 // UnpHalf = Un + dt R1 MdInv (:3781-3783) -- the Dirichlet zeroing is the
 // zero in minv_free.  Also writes d = UnpHalf/dt^2 - [iter>1] MdOrigInv KAcc,
 // the input of step2 (blascoCodinaHuerta.cpp:3821-3832).
-template <class VT, int SPLIT>
+//
+// ACC (iter > 1 inside cfd_run): the K Acc_prev of calculate_KtimesAcc_prev in
+// the same pass over K, one read of its values and columns instead of two (us
+// of step 1 and K Acc_prev: 64^3 FP64 1044 -> 841, FP32 597 -> 474, duct FP32
+// 219 -> 174, 32^3 FP64 142 -> 131, 8^3 FP64 13.2 -> 9.5; 24^3 FP32 72 -> 46,
+// 16^3 FP32 27 -> 22).
+template <class VT, int SPLIT, bool ACC>
 __global__ void __launch_bounds__(block_threads(SPLIT)) k_step1(Step1Args<VT> a) {
-  __shared__ SplitBuf<VT, Entry<VT>, 6, SPLIT> buf;
+  __shared__ SplitBuf<VT, std::conditional_t<ACC, Entry2<VT>, Entry<VT>>, ACC ? 9 : 6, SPLIT> buf;
+  constexpr bool fp32 = sizeof(VT) == 4;
   const int l = threadIdx.x & 31;
   const int row = SPLIT == 1 ? blockIdx.x * blockDim.x + threadIdx.x : 32 * blockIdx.x + l;
   if (SPLIT == 1 && row >= a.NN) return;
   const int s = row >> 5;
   const double inv_dt2 = 1.0000000000000000 / (a.dt * a.dt);
-  VT kx = 0, ky = 0, kz = 0, gx = 0, gy = 0, gz = 0;
+  VT kx = 0, ky = 0, kz = 0, gx = 0, gy = 0, gz = 0, ax = 0, ay = 0, az = 0;
   {
-    const int b = __ldg(a.k_off + s), w = (__ldg(a.k_off + s + 1) - b) >> 5;
-    const int* col = a.k_col + b + l;
-    const VT* val = a.kval + b + l;
-    for_entries<SPLIT>(
-        buf, w,
-        [&](int j) {
-          const VT v = __ldcs(val + 32 * j);
-          const auto x = ldgv(a.uprev + __ldcs(col + 32 * j));
-          return Entry<VT>{v, (VT)x.x, (VT)x.y, (VT)x.z};
-        },
-        [&](const Entry<VT>& e) {
-          kx += e.a * e.b;
-          ky += e.a * e.c;
-          kz += e.a * e.d;
-        });
+    const int b = __ldg(a.k_off + s), w = (__ldg(a.k_off + s + 1) - b) >> 5, bl = b + l;
+    // order of the two loads as in the table at for_entries
+    auto stream = [&](int j) {
+      KEntry<VT> k;
+      if constexpr (fp32 && SPLIT == 1) {
+        k.v = __ldcs(a.kval + bl + 32 * j);
+        k.c = __ldcs(a.k_col + bl + 32 * j);
+      } else {
+        k.c = __ldcs(a.k_col + bl + 32 * j);
+        k.v = __ldcs(a.kval + bl + 32 * j);
+      }
+      return k;
+    };
+    if constexpr (ACC) {
+      for_entries<SPLIT, fp32 ? 3 : 0>(
+          buf, w, stream,
+          [&](const KEntry<VT>& k) {
+            const auto x = ldgv(a.uprev + k.c);
+            const auto y = ldgv(a.accprev + k.c);
+            return Entry2<VT>{k.v, (VT)x.x, (VT)x.y, (VT)x.z, (VT)y.x, (VT)y.y, (VT)y.z};
+          },
+          [&](const Entry2<VT>& e) {
+            kx += e.a * e.b;
+            ky += e.a * e.c;
+            kz += e.a * e.d;
+            ax += e.a * e.x;
+            ay += e.a * e.y;
+            az += e.a * e.z;
+          });
+    } else {
+      for_entries<SPLIT, fp32 ? 0 : 2>(
+          buf, w, stream,
+          [&](const KEntry<VT>& k) {
+            const auto x = ldgv(a.uprev + k.c);
+            return Entry<VT>{k.v, (VT)x.x, (VT)x.y, (VT)x.z};
+          },
+          [&](const Entry<VT>& e) {
+            kx += e.a * e.b;
+            ky += e.a * e.c;
+            kz += e.a * e.d;
+          });
+    }
   }
   {
-    const int b = __ldg(a.g_off + s), w = (__ldg(a.g_off + s + 1) - b) >> 5;
-    const int* col = a.g_col + b + l;
-    for_entries<SPLIT>(
-        buf, w,
+    const int b = __ldg(a.g_off + s), w = (__ldg(a.g_off + s + 1) - b) >> 5, bl = b + l;
+    auto& gbuf = reinterpret_cast<SplitBuf<VT, Entry<VT>, 6, SPLIT>&>(buf);
+    for_entries<SPLIT, fp32 ? (ACC ? 3 : 2) : ACC ? 2 : 0>(
+        gbuf, w,
         [&](int j) {
-          const VT p = (VT)__ldg(a.pn + __ldcs(col + 32 * j));
-          return Entry<VT>{__ldcs(a.g1 + b + l + 32 * j), __ldcs(a.g2 + b + l + 32 * j),
-                           __ldcs(a.g3 + b + l + 32 * j), p};
+          const int e = bl + 32 * j;
+          return GEntry<VT>{__ldcs(a.g_col + e), __ldcs(a.g1 + e), __ldcs(a.g2 + e), __ldcs(a.g3 + e)};
         },
+        [&](const GEntry<VT>& g) { return Entry<VT>{g.x, g.y, g.z, (VT)__ldg(a.pn + g.c)}; },
         [&](const Entry<VT>& e) {
           gx += e.a * e.d;
           gy += e.b * e.d;
@@ -186,10 +279,16 @@ __global__ void __launch_bounds__(block_threads(SPLIT)) k_step1(Step1Args<VT> a)
         });
   }
   if constexpr (SPLIT > 1) {
-    VT v[6] = {kx, ky, kz, gx, gy, gz};
-    split_sum<SPLIT>(buf, v);
+    if constexpr (ACC) {
+      VT v[9] = {kx, ky, kz, gx, gy, gz, ax, ay, az};
+      split_sum<SPLIT>(buf, v);
+      kx = v[0], ky = v[1], kz = v[2], gx = v[3], gy = v[4], gz = v[5], ax = v[6], ay = v[7], az = v[8];
+    } else {
+      VT v[6] = {kx, ky, kz, gx, gy, gz};
+      split_sum<SPLIT>(buf, v);
+      kx = v[0], ky = v[1], kz = v[2], gx = v[3], gy = v[4], gz = v[5];
+    }
     if (threadIdx.x >= 32 || row >= a.NN) return;
-    kx = v[0], ky = v[1], kz = v[2], gx = v[3], gy = v[4], gz = v[5];
   }
   double4 rc;
   if (a.r1conv32) {
@@ -218,7 +317,13 @@ __global__ void __launch_bounds__(block_threads(SPLIT)) k_step1(Step1Args<VT> a)
   d.w = 0.0;
   if (a.iter != 1) {
     const double mo = a.minv_orig[row];
-    const double4 ka = a.kacc[row];
+    double4 ka;
+    if constexpr (ACC) {
+      ka = make_double4((double)ax, (double)ay, (double)az, 0.0);
+      a.kacc[row] = ka;
+    } else {
+      ka = a.kacc[row];
+    }
     d.x = d.x - mo * ka.x;
     d.y = d.y - mo * ka.y;
     d.z = d.z - mo * ka.z;
@@ -239,12 +344,15 @@ __global__ void __launch_bounds__(block_threads(SPLIT)) k_gt(GtArgs<VT> a) {
   const int s = row >> 5;
   const int b = __ldg(a.gt_off + s) + l, w = (__ldg(a.gt_off + s + 1) - __ldg(a.gt_off + s)) >> 5;
   VT acc[1] = {0};
-  for_entries<SPLIT>(
+  for_entries<SPLIT, 0>(
       buf, w,
       [&](int j) {
         const int e = b + 32 * j;
-        const auto d = ldgv(a.d + __ldcs(a.gt_col + e));
-        return __ldcs(a.gt1 + e) * (VT)d.x + __ldcs(a.gt2 + e) * (VT)d.y + __ldcs(a.gt3 + e) * (VT)d.z;
+        return GEntry<VT>{__ldcs(a.gt_col + e), __ldcs(a.gt1 + e), __ldcs(a.gt2 + e), __ldcs(a.gt3 + e)};
+      },
+      [&](const GEntry<VT>& g) {
+        const auto d = ldgv(a.d + g.c);
+        return g.x * (VT)d.x + g.y * (VT)d.y + g.z * (VT)d.z;
       },
       [&](VT t) { acc[0] += t; });
   split_sum<SPLIT>(buf, acc);
@@ -267,13 +375,13 @@ __global__ void __launch_bounds__(block_threads(SPLIT)) k_step3(Step3Args<VT> a)
   auto products = [&]() {
     const int s = row >> 5;
     const int b = __ldg(a.g_off + s) + l, w = (__ldg(a.g_off + s + 1) - __ldg(a.g_off + s)) >> 5;
-    for_entries<SPLIT>(
+    for_entries<SPLIT, sizeof(VT) == 8 ? 1 : 0>(
         buf, w,
         [&](int j) {
           const int e = b + 32 * j;
-          const VT p = (VT)__ldg(a.pdot + __ldcs(a.g_col + e));
-          return Entry<VT>{__ldcs(a.g1 + e), __ldcs(a.g2 + e), __ldcs(a.g3 + e), p};
+          return GEntry<VT>{__ldcs(a.g_col + e), __ldcs(a.g1 + e), __ldcs(a.g2 + e), __ldcs(a.g3 + e)};
         },
+        [&](const GEntry<VT>& g) { return Entry<VT>{g.x, g.y, g.z, (VT)__ldg(a.pdot + g.c)}; },
         [&](const Entry<VT>& e) {
           gx += e.a * e.d;
           gy += e.b * e.d;
@@ -339,13 +447,15 @@ __global__ void __launch_bounds__(block_threads(SPLIT)) k_spmv_k3(SpmvK3Args<VT>
   const int s = row >> 5;
   const int b = __ldg(a.off + s) + l, w = (__ldg(a.off + s + 1) - __ldg(a.off + s)) >> 5;
   VT sx = 0, sy = 0, sz = 0;
-  for_entries<SPLIT>(
+  for_entries<SPLIT, sizeof(VT) == 8 ? 2 : 0>(
       buf, w,
       [&](int j) {
         const int e = b + 32 * j;
-        const VT v = __ldcs(a.val + e);
-        const auto x = ldgv(a.x + __ldcs(a.col + e));
-        return Entry<VT>{v, (VT)x.x, (VT)x.y, (VT)x.z};
+        return KEntry<VT>{__ldcs(a.col + e), __ldcs(a.val + e)};
+      },
+      [&](const KEntry<VT>& k) {
+        const auto x = ldgv(a.x + k.c);
+        return Entry<VT>{k.v, (VT)x.x, (VT)x.y, (VT)x.z};
       },
       [&](const Entry<VT>& e) {
         sx += e.a * e.b;
@@ -464,33 +574,28 @@ inline int ew_grid(long long n) {
 
 }  // namespace
 
-// Launches kernel<VT, SPLIT> with the SPLIT of the row count.
-#define SPLIT_LAUNCH(kernel, rows, rule)                                                  \
-  do {                                                                                    \
-    const int sp_ = row_split<VT>(rows, rule), g_ = split_grid(rows, sp_);                \
-    switch (sp_) {                                                                        \
-      case 1: kernel<VT, 1><<<g_, kRowThreads, 0, s>>>(a); break;                         \
-      case 2: kernel<VT, 2><<<g_, block_threads(2), 0, s>>>(a); break;                         \
-      case 4: kernel<VT, 4><<<g_, block_threads(4), 0, s>>>(a); break;                         \
-      default: kernel<VT, 8><<<g_, block_threads(8), 0, s>>>(a); break;                        \
-    }                                                                                     \
-    return cudaGetLastError();                                                            \
+// Launches kernel<VT, SPLIT, ...> with the SPLIT of the row count.
+#define SPLIT_LAUNCH(kernel, rows, rule, ...)                                                              \
+  do {                                                                                                     \
+    const int sp_ = row_split<VT>(rows, rule), g_ = split_grid(rows, sp_);                                 \
+    switch (sp_) {                                                                                         \
+      case 1: kernel<VT, 1 __VA_OPT__(, ) __VA_ARGS__><<<g_, kRowThreads, 0, s>>>(a); break;               \
+      case 2: kernel<VT, 2 __VA_OPT__(, ) __VA_ARGS__><<<g_, block_threads(2), 0, s>>>(a); break;          \
+      case 4: kernel<VT, 4 __VA_OPT__(, ) __VA_ARGS__><<<g_, block_threads(4), 0, s>>>(a); break;          \
+      default: kernel<VT, 8 __VA_OPT__(, ) __VA_ARGS__><<<g_, block_threads(8), 0, s>>>(a); break;         \
+    }                                                                                                      \
+    return cudaGetLastError();                                                                             \
   } while (0)
 
 template <class VT>
 cudaError_t launch_step1(const Step1Args<VT>& a, int, cudaStream_t s) {
-  SPLIT_LAUNCH(k_step1, a.NN, kStep1Rule);
+  if (a.accprev) SPLIT_LAUNCH(k_step1, a.NN, kStep1Rule, true);
+  SPLIT_LAUNCH(k_step1, a.NN, kStep1Rule, false);
 }
 template <class VT>
 cudaError_t launch_gt(const GtArgs<VT>& a, int, cudaStream_t s) {
   SPLIT_LAUNCH(k_gt, a.NNp, kGtRule);
 }
-template <class VT>
-int step3_blocks(int NN) {
-  return split_grid(NN, row_split<VT>(NN, kStep3Rule));
-}
-template int step3_blocks<double>(int);
-template int step3_blocks<float>(int);
 template <class VT>
 cudaError_t launch_step3(const Step3Args<VT>& a, cudaStream_t s) {
   SPLIT_LAUNCH(k_step3, a.NN, kStep3Rule);
@@ -499,6 +604,12 @@ template <class VT>
 cudaError_t launch_spmv_k3(const SpmvK3Args<VT>& a, int, cudaStream_t s) {
   SPLIT_LAUNCH(k_spmv_k3, a.NN, kSpmvK3Rule);
 }
+template <class VT>
+int step3_blocks(int NN) {
+  return split_grid(NN, row_split<VT>(NN, kStep3Rule));
+}
+template int step3_blocks<double>(int);
+template int step3_blocks<float>(int);
 int pupdate_blocks(int NNp, int num_sms) { return ew_grid(NNp) < num_sms * 4 ? ew_grid(NNp) : num_sms * 4; }
 cudaError_t launch_pressure_update(int NNp, double dt, const double* pn, const double* pdot, const double* pprev,
                                    double* pnp1, double* part, int nblocks, cudaStream_t s) {
