@@ -91,9 +91,10 @@ __global__ void __launch_bounds__(k16X * k16Y * k16Z) k_conv_16to1(ConvDesc d) {
   constexpr int HX = k16X + 2, HY = k16Y + 2, HZ = k16Z + 2;
   __shared__ uint4 tile[HX * HY * HZ][2];
   __shared__ float4 sw[27 * 4];
-  if (d.skip && *d.skip) return;
   for (int i = threadIdx.x; i < 27 * 16; i += blockDim.x) ((float*)sw)[i] = bf(d.w[i]);
   const float b0 = d.bias[0];
+  pdl_wait();
+  if (d.skip && *d.skip) return;
   const int nx = d.out_dims[0], ny = d.out_dims[1], nz = d.out_dims[2];
   const int tbx = (nx + k16X - 1) / k16X, tby = (ny + k16Y - 1) / k16Y;
   const int bx = blockIdx.x % tbx, by = (blockIdx.x / tbx) % tby, bz = blockIdx.x / (tbx * tby);
@@ -104,8 +105,7 @@ __global__ void __launch_bounds__(k16X * k16Y * k16Z) k_conv_16to1(ConvDesc d) {
     const int gx = x0 - 1 + hx, gy = y0 - 1 + hy, gz = z0 - 1 + hz;
     uint4 u = make_uint4(0, 0, 0, 0);
     if (gx >= 0 && gy >= 0 && gz >= 0 && gx < nx && gy < ny && gz < nz)
-      u = __ldg(reinterpret_cast<const uint4*>(d.inA + ((size_t)gx + (size_t)nx * (gy + (size_t)ny * gz)) * 16) +
-                half);
+      u = reinterpret_cast<const uint4*>(d.inA + ((size_t)gx + (size_t)nx * (gy + (size_t)ny * gz)) * 16)[half];
     tile[vox][half] = u;
   }
   __syncthreads();
@@ -143,9 +143,11 @@ __global__ void __launch_bounds__(k16X * k16Y * k16Z) k_conv_c1to16(ConvDesc d) 
   __shared__ float tile[HX * HY * HZ];
   __shared__ float4 sw[27 * 4];
   __shared__ float sb[16];
-  if (d.skip && *d.skip) return;
   for (int i = threadIdx.x; i < 27 * 16; i += blockDim.x) ((float*)sw)[i] = bf(d.w[i]);
   if (threadIdx.x < 16) sb[threadIdx.x] = d.bias[threadIdx.x];
+  pdl_trigger();
+  pdl_wait();
+  if (d.skip && *d.skip) return;
   const int nx = d.out_dims[0], ny = d.out_dims[1], nz = d.out_dims[2];
   const int tbx = (nx + k16X - 1) / k16X, tby = (ny + k16Y - 1) / k16Y;
   const int bx = blockIdx.x % tbx, by = (blockIdx.x / tbx) % tby, bz = blockIdx.x / (tbx * tby);
@@ -193,11 +195,13 @@ __global__ void __launch_bounds__(k16X * k16Y * k16Z) k_conv_c1to16(ConvDesc d) 
 // Prolongation plus skip for CH channels: one thread per fine voxel, 16-byte
 // vector loads and stores, 32-bit index arithmetic.  The corners are summed
 // in the order (z, y, x) of the coarse cell, as the trilinear weights of the
-// fine index pick them.
+// fine index pick them.  May start before the layer in front has finished, so
+// its inputs are not read-only for the kernel's whole life (no __restrict__).
 template <int CH>
-__global__ void __launch_bounds__(256) k_up_fwd_v(Dims3 g, const __nv_bfloat16* __restrict__ in,
-                                                  const __nv_bfloat16* __restrict__ skip, __nv_bfloat16* out,
-                                                  const int* skipflag) {
+__global__ void __launch_bounds__(256) k_up_fwd_v(Dims3 g, const __nv_bfloat16* in, const __nv_bfloat16* skip,
+                                                  __nv_bfloat16* out, const int* skipflag) {
+  pdl_trigger();
+  pdl_wait();
   if (skipflag && *skipflag) return;
   const int fx = g.f[0], fy = g.f[1], fz = g.f[2], cx = g.c[0], cy = g.c[1];
   const int nf = fx * fy * fz;
@@ -247,6 +251,7 @@ __global__ void __launch_bounds__(256) k_up_fwd_v(Dims3 g, const __nv_bfloat16* 
 
 __global__ void k_up_fwd(Dims3 g, int ch, const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* skip,
                          __nv_bfloat16* out, const int* skipflag) {
+  pdl_wait();
   if (skipflag && *skipflag) return;
   const long long nf = (long long)g.f[0] * g.f[1] * g.f[2];
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nf * ch;
@@ -297,6 +302,7 @@ __global__ void k_up_bwd(Dims3 g, int ch4, const float4* __restrict__ dfine, flo
 template <class T>
 __global__ void k_input(int nv, const T* __restrict__ r, const int* __restrict__ pmap, const double* rr,
                         double scale, __nv_bfloat16* x, const int* skipflag) {
+  pdl_trigger();
   if (skipflag && *skipflag) return;
   double c = scale;
   if (rr) c = rr[0] > 0.0 ? sqrt((double)nv / rr[0]) : 0.0;
@@ -374,21 +380,19 @@ cudaError_t with_smem(F kernel, size_t bytes) {
 
 }  // namespace
 
-cudaError_t conv3_forward(const ConvDesc& d, cudaStream_t s) {
+cudaError_t conv3_forward(const ConvDesc& d, bool pdl, cudaStream_t s) {
   const int cin = d.ca + d.cb;
   const long long nv = (long long)d.out_dims[0] * d.out_dims[1] * d.out_dims[2];
   const int gx = grid1(nv, 128);
   if (cin == 1 && d.cout == 16 && d.stride == 1 && d.out && !d.out_f32 && nv < (1LL << 31)) {
     const long long tiles = (long long)((d.out_dims[0] + k16X - 1) / k16X) * ((d.out_dims[1] + k16Y - 1) / k16Y) *
                             ((d.out_dims[2] + k16Z - 1) / k16Z);
-    k_conv_c1to16<<<(unsigned)tiles, k16X * k16Y * k16Z, 0, s>>>(d);
-    return cudaGetLastError();
+    return launch_k(pdl, k_conv_c1to16, dim3((unsigned)tiles), dim3(k16X * k16Y * k16Z), 0, s, d);
   }
   if (d.ca == 16 && d.cb == 0 && d.cout == 1 && d.stride == 1 && d.out_f32 && !d.out && nv < (1LL << 31)) {
     const long long tiles = (long long)((d.out_dims[0] + k16X - 1) / k16X) * ((d.out_dims[1] + k16Y - 1) / k16Y) *
                             ((d.out_dims[2] + k16Z - 1) / k16Z);
-    k_conv_16to1<<<(unsigned)tiles, k16X * k16Y * k16Z, 0, s>>>(d);
-    return cudaGetLastError();
+    return launch_k(pdl, k_conv_16to1, dim3((unsigned)tiles), dim3(k16X * k16Y * k16Z), 0, s, d);
   }
   if (cin <= 48) {
     const size_t sm = (size_t)27 * cin * 16 * sizeof(float);
@@ -405,7 +409,8 @@ cudaError_t conv3_forward(const ConvDesc& d, cudaStream_t s) {
 }
 
 cudaError_t upsample_forward(const int* cdims, const int* fdims, int ch, const __nv_bfloat16* in,
-                             const __nv_bfloat16* skip, __nv_bfloat16* out, const int* skipflag, cudaStream_t s) {
+                             const __nv_bfloat16* skip, __nv_bfloat16* out, const int* skipflag, bool pdl,
+                             cudaStream_t s) {
   Dims3 g;
   for (int i = 0; i < 3; i++) {
     g.c[i] = cdims[i];
@@ -413,11 +418,8 @@ cudaError_t upsample_forward(const int* cdims, const int* fdims, int ch, const _
   }
   const long long nf = (long long)fdims[0] * fdims[1] * fdims[2];
   if (skip && nf < (1LL << 31) && (ch == 16 || ch == 32)) {
-    if (ch == 16)
-      k_up_fwd_v<16><<<grid1(nf), 256, 0, s>>>(g, in, skip, out, skipflag);
-    else
-      k_up_fwd_v<32><<<grid1(nf), 256, 0, s>>>(g, in, skip, out, skipflag);
-    return cudaGetLastError();
+    return launch_k(pdl, ch == 16 ? k_up_fwd_v<16> : k_up_fwd_v<32>, dim3(grid1(nf)), dim3(256), 0, s, g, in, skip,
+                    out, skipflag);
   }
   const long long n = nf * ch;
   k_up_fwd<<<grid1(n), 256, 0, s>>>(g, ch, in, skip, out, skipflag);

@@ -33,7 +33,9 @@ struct ConvDesc {
   const int* skip;            // optional device flag: the kernel does nothing while *skip != 0
 };
 
-cudaError_t conv3_forward(const ConvDesc& d, cudaStream_t s);
+// pdl as in conv3_forward_tc (the forms that use it are the first layer's and
+// the single-output layer's).
+cudaError_t conv3_forward(const ConvDesc& d, bool pdl, cudaStream_t s);
 
 // Data gradient: dx = add + conv^T(dOut, W) in FP32 (add may be null), and
 // weight gradients dW[k][ci][co] += sum_v in[s v + off_k][ci] dOut[v][co],
@@ -52,7 +54,8 @@ cudaError_t conv3_wgrad(const ConvDesc& d, const float* dout, const __nv_bfloat1
 // out = P(in) + skip: vertex-centred trilinear prolongation from coarse dims c
 // to fine dims f = 2c - 1 (ch channels), plus an optional fine skip tensor.
 cudaError_t upsample_forward(const int* cdims, const int* fdims, int ch, const __nv_bfloat16* in,
-                             const __nv_bfloat16* skip, __nv_bfloat16* out, const int* skipflag, cudaStream_t s);
+                             const __nv_bfloat16* skip, __nv_bfloat16* out, const int* skipflag, bool pdl,
+                             cudaStream_t s);
 // transpose of upsample_forward: coarse gradient = R(fine gradient), ch a multiple of 4
 cudaError_t upsample_backward(const int* cdims, const int* fdims, int ch, const float* dfine, float* dcoarse,
                               cudaStream_t s);
@@ -101,6 +104,7 @@ struct ConvTcParams {
   float* out_f32;
   int act;
   const int* skip;
+  int pdl;   // the next layer may be launched early (pdl_trigger)
   int* err;  // set when a bounded wait gives up
   // persistent form: shared-memory stages of the halo brick (1 or 2), TMEM
   // columns allocated per CTA and accumulators in the ring; fold = 1: the
@@ -131,7 +135,10 @@ cudaError_t conv_tc_pack(const __nv_bfloat16* w, int cin, int cout, int stride, 
 // taps folded into N (stride 1 only; the weights packed with fold = 1).
 int conv_tc_plan(const ConvDesc& d, const __nv_bfloat16* wpack, int num_sms, ConvTcPlan& plan, int pipe = 0);
 // Launches a planned convolution; out_f32 (FP32-output layers) and skip
-// replace the plan's pointers for this launch.
-cudaError_t conv3_forward_tc(const ConvTcPlan& plan, float* out_f32, const int* skip, int* err, cudaStream_t s);
+// replace the plan's pointers for this launch.  pdl: launched before the layer
+// in front has finished; the packed weights and the bias are then read early, so
+// whatever wrote them has to be complete when that layer starts.
+cudaError_t conv3_forward_tc(const ConvTcPlan& plan, float* out_f32, const int* skip, int* err, bool pdl,
+                             cudaStream_t s);
 
 }  // namespace cfd

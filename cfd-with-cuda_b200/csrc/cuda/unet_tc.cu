@@ -120,14 +120,14 @@ template <int CIN, int STRIDE>
 __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ ConvTcParams p) {
   constexpr int NCH = CIN / 8, KSTEPS = CIN / 16, NPH = STRIDE == 2 ? 8 : 1;
   constexpr int NWARP = kTcThreads / 32;
-  if (p.skip && *p.skip) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* A = smem;
   unsigned char* W = smem + (size_t)NPH * NCH * p.plane_bytes;
   const unsigned wbytes = 27u * CIN * p.N * 2u;
-  // barrier 0: weights; barrier 1 + w: MMAs issued by warp w
+  // barrier 0: weights; barrier 1 + w: MMAs issued by warp w; then the halo
   unsigned long long* bars = (unsigned long long*)(W + wbytes);  // wbytes is a multiple of 16
-  unsigned* tmem_slot = (unsigned*)(bars + 1 + NWARP);
+  unsigned long long* hbar = bars + 1 + NWARP;
+  unsigned* tmem_slot = (unsigned*)(bars + 2 + NWARP);
   float* sbias = (float*)(tmem_slot + 2);  // N floats
 
   const int b = blockIdx.x, slice = blockIdx.y;
@@ -136,24 +136,23 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ 
   const int HX = p.halo[0], HY = p.halo[1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  // While the layer in front of this one still runs (programmatic dependent
+  // launch): the barriers, the weights, which no kernel of the pass writes, the
+  // bias, the accumulator columns and the zero rows.  A layer is 4 to 20 us
+  // of mostly latency, one phase after the other, so the launch and the copy of
+  // up to 110 KB of weights per block count: us per application (13 layers) without
+  // and with the early start, 65^3 208 and 197, duct 25 x 25 x 161 157 and 146,
+  // 33 x 17 x 9 124 and 94, 5^3 115 and 82.
   if (threadIdx.x == 0) {
-    for (int i = 0; i <= NWARP; i++) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 2 + NWARP; i++) mbar_init(&bars[i], 1);
     mbar_init_fence();
+    mbar_expect_tx(&bars[0], wbytes);
+    bulk_g2s(W, p.wpack + (size_t)slice * 27 * CIN * p.N, wbytes, &bars[0]);
   }
   if (warp == 0) tmem_alloc(tmem_slot, kTmemCols);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const unsigned tmem = *tmem_slot;
   for (int i = threadIdx.x; i < p.N; i += blockDim.x) {
     const int co = slice * p.N + i;
     sbias[i] = co < p.cout ? p.bias[co] : 0.f;
-  }
-  if (threadIdx.x == 0) {
-    const unsigned abytes = (unsigned)NPH * NCH * 16u * (unsigned)(HX * HY * p.halo[2]);
-    mbar_expect_tx(&bars[0], wbytes + abytes);
-    bulk_g2s(W, p.wpack + (size_t)slice * 27 * CIN * p.N, wbytes, &bars[0]);
-    load_halo<NCH, STRIDE>(p, A, x0, y0, z0, &bars[0]);
   }
   {
     // rows past the halo box that tap shifts of the last tiles can read: zeros
@@ -164,7 +163,26 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ 
     }
   }
   fence_proxy_async_smem();
-  bool ok = __syncthreads_and(mbar_wait_bounded(&bars[0], 0, kTcWaitNs));
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem = *tmem_slot;
+  // The accumulator columns are allocated: the next layer's blocks may come in.
+  if (p.pdl) pdl_trigger();
+  pdl_wait();
+  const bool skip = p.skip && *p.skip;
+  if (!skip && threadIdx.x == 0) {
+    mbar_expect_tx(hbar, (unsigned)NPH * NCH * 16u * (unsigned)(HX * HY * p.halo[2]));
+    load_halo<NCH, STRIDE>(p, A, x0, y0, z0, hbar);
+  }
+  bool ok = mbar_wait_bounded(&bars[0], 0, kTcWaitNs);
+  if (!skip) ok = ok && mbar_wait_bounded(hbar, 0, kTcWaitNs);
+  ok = __syncthreads_and(ok);
+  if (skip) {
+    if (!ok && threadIdx.x == 0 && p.err) atomicExch(p.err, 1);
+    if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+    return;
+  }
   bool loads_done = ok, mma_done = true;
 
   const unsigned idesc = umma_idesc(p.N);
@@ -288,7 +306,10 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(const __grid_constant__ 
     // accumulator columns are released
     if (threadIdx.x == 0) {
       if (p.err) atomicExch(p.err, 1);
-      if (!loads_done) mbar_wait_bounded(&bars[0], 0, kTcWaitNs);
+      if (!loads_done) {
+        mbar_wait_bounded(&bars[0], 0, kTcWaitNs);
+        mbar_wait_bounded(hbar, 0, kTcWaitNs);
+      }
     }
     if (!mma_done && lane == 0) mbar_wait_bounded(&bars[1 + warp], phase ^ 1, kTcWaitNs);
   }
@@ -367,6 +388,7 @@ __global__ void __launch_bounds__(kPipeThreads) k_conv_pipe(const __grid_constan
   constexpr int NCH = CIN / 8, KSTEPS = CIN / 16, NPH = STRIDE == 2 ? 8 : 1;
   constexpr int NG = FOLD ? 9 : 27;       // MMA groups per K step
   constexpr int TSTEP = FOLD ? 126 : 128;  // output rows per tile
+  pdl_wait();
   if (p.skip && *p.skip) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int nst = p.astages, nacc = p.nacc;
@@ -920,11 +942,13 @@ int conv_tc_plan(const ConvDesc& d, const __nv_bfloat16* wpack, int num_sms, Con
   return 0;
 }
 
-cudaError_t conv3_forward_tc(const ConvTcPlan& plan, float* out_f32, const int* skip, int* err, cudaStream_t s) {
+cudaError_t conv3_forward_tc(const ConvTcPlan& plan, float* out_f32, const int* skip, int* err, bool pdl,
+                             cudaStream_t s) {
   ConvTcParams p = plan.p;
   if (p.out_f32 && out_f32) p.out_f32 = out_f32;
   p.skip = skip;
   p.err = err;
+  p.pdl = pdl && !p.out_f32;  // the last layer lets nothing in early
   void (*k)(ConvTcParams) = nullptr;
   if (plan.pipe) {
     switch (p.cin * 8 + p.stride * 2 + p.fold) {
@@ -959,8 +983,7 @@ cudaError_t conv3_forward_tc(const ConvTcPlan& plan, float* out_f32, const int* 
   // always the largest a block may have.
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   if (e != cudaSuccess) return e;
-  k<<<dim3(plan.grid_x, p.nslices), kTcThreads, plan.smem, s>>>(p);
-  return cudaGetLastError();
+  return launch_k(pdl, k, dim3(plan.grid_x, p.nslices), dim3(kTcThreads), plan.smem, s, p);
 }
 
 }  // namespace cfd

@@ -91,6 +91,7 @@ int UnetNet::init(unsigned long long seed) {
     return -1;
   }
   if (const char* e = std::getenv("CFD_UNET_TC")) tc_enabled = std::atoi(e) != 0;
+  if (const char* e = std::getenv("CFD_PDL")) pdl = std::atoi(e) != 0;
   if (const char* e = std::getenv("CFD_CONV_PIPE")) conv_pipe = std::atoi(e);
   if (!own_stream && cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking) != cudaSuccess) return -1;
   const size_t b = (size_t)nparam * sizeof(float);
@@ -249,13 +250,14 @@ cudaError_t UnetNet::forward(cudaStream_t s, float* out_f32, const int* skip) {
     cudaError_t e;
     if (op >= 0) {
       if (tc_enabled && plan_ok[op]) {
-        e = conv3_forward_tc(plans[op], out_f32, skip, tc_err, s);
+        e = conv3_forward_tc(plans[op], out_f32, skip, tc_err, pdl, s);
       } else
-        e = conv3_forward(conv_desc(*this, op, out_f32, skip), s);
+        e = conv3_forward(conv_desc(*this, op, out_f32, skip), pdl, s);
     } else {
       const UnetUpSpec& u = kUnetUp[-1 - op];
       const int lc = kUnetTensor[u.in].level, lf = kUnetTensor[u.out].level;
-      e = upsample_forward(dims[lc], dims[lf], kUnetTensor[u.out].ch, act[u.in], act[u.skip], act[u.out], skip, s);
+      e = upsample_forward(dims[lc], dims[lf], kUnetTensor[u.out].ch, act[u.in], act[u.skip], act[u.out], skip, pdl,
+                           s);
     }
     launches++;
     if (e != cudaSuccess) return e;

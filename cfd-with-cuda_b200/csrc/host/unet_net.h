@@ -82,6 +82,11 @@ struct UnetNet {
   float* h_pinned = nullptr;
   int gen = 0;  // bumped whenever an activation buffer moves
 
+  // The layers of a forward pass start before the layer in front has finished
+  // (programmatic dependent launch; CFD_PDL=0 turns it off).  The input kernel,
+  // before the first layer, is launched as usual, so whatever precedes the pass
+  // (packing of the weights, an Adam step) is complete by then.
+  bool pdl = true;
   // tensor-core path: packed weights and launch plans of the stride-1 layers
   bool tc_enabled = true;
   // tensor-core kernel of each layer (CFD_CONV_PIPE): 0 one CTA per brick;
