@@ -28,8 +28,8 @@ namespace {
 constexpr int kRestrictThreads = 512;
 constexpr int kRestrictLines = 1024;  // y-z support lines per coarse pair at most
 template <class VT>
-__global__ void __launch_bounds__(kRestrictThreads) k_restrict(CoarseArgs<VT> a, const VT* __restrict__ r,
-                                                               float* __restrict__ c, const int* done) {
+__global__ void __launch_bounds__(kRestrictThreads) k_restrict(CoarseArgs<VT> a, const VT* r, float* c,
+                                                               const int* done) {
   pdl_trigger();  // the coarse solve reads only constants before its wait
   extern __shared__ double sline[];  // G x W partial sums
   __shared__ double swt[kRestrictLines];
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kRestrictThreads) k_restrict(CoarseArgs<VT> a,
 // sum_i h[i] c[i] over 8 FP16 entries packed in q and 8 FP32 values at c
 __device__ __forceinline__ float dot8(const uint4& q, const float* c) {
   const __half2* h = reinterpret_cast<const __half2*>(&q);
-  const float4 c0 = __ldg(reinterpret_cast<const float4*>(c)), c1 = __ldg(reinterpret_cast<const float4*>(c) + 1);
+  const float4 c0 = reinterpret_cast<const float4*>(c)[0], c1 = reinterpret_cast<const float4*>(c)[1];
   float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]), f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
   return (f0.x * c0.x + f0.y * c0.y) + (f1.x * c0.z + f1.y * c0.w) + (f2.x * c1.x + f2.y * c1.y) +
          (f3.x * c1.z + f3.y * c1.w);
@@ -98,8 +98,7 @@ __device__ __forceinline__ float dot8(const uint4& q, const float* c) {
 constexpr int kMvThreads = 128, kMvLoads = 6;  // 6 x 128 x 8 entries >= kCoarseMaxNodes of the solver
 template <class VT>
 __global__ void __launch_bounds__(kMvThreads) k_coarse_mv(int nc, int ld, const __half* __restrict__ inv, float rscale,
-                                                          const float* __restrict__ c, VT* __restrict__ e,
-                                                          const int* done) {
+                                                          const float* c, VT* e, const int* done) {
   const int row = blockIdx.x;
   const int nv8 = nc >> 3, tail = nc & 7;  // whole 8-entry groups inside the row, then a tail
   const uint4* ir = reinterpret_cast<const uint4*>(inv + (size_t)row * ld);
@@ -137,9 +136,9 @@ __global__ void __launch_bounds__(kMvThreads) k_coarse_mv(int nc, int ld, const 
 // the rest of a thread's first voxel is loaded before the wait for it.
 template <class VT>
 __global__ void __launch_bounds__(256) k_precond(CoarseArgs<VT> a, int nv, const VT* __restrict__ r,
-                                                 const VT* __restrict__ dinv, const VT* __restrict__ e,
+                                                 const VT* __restrict__ dinv, const VT* e,
                                                  const float* __restrict__ y, const double* rr, double dscale,
-                                                 VT* __restrict__ z, const int* done) {
+                                                 VT* z, const int* done) {
   pdl_trigger();  // the SpMV reads only the matrix before its wait
   const int cx = a.cd[0], cxy = a.cd[0] * a.cd[1];
   const int bx = a.cd[0] > 1, by = a.cd[1] > 1, bz = a.cd[2] > 1;

@@ -132,7 +132,9 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, int* err, unsigned l
 // block of this one has reached it.  A kernel that triggers after its own wait
 // promises its successor that everything before this kernel is complete, so
 // the successor may read that before it waits; one that triggers at its start
-// allows it constants only.
+// allows it constants only.  What the kernel before writes is read with plain
+// loads: __ldg and __restrict__ promise data that nobody writes while the
+// reading kernel lives, and its life begins before that kernel ends.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 

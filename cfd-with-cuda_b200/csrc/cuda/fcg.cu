@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_fcg_spmv_stencil(FcgArgs<VT>
   const int nd = it < m ? it : m;
   bool ok = true;
   int kfail = 0;
-  const VT* __restrict__ z = a.z;
+  const VT* z = a.z;
   const int reach = 2 + 2 * fx + 2 * fxy;  // largest |j - i| of a tap
   double v[fcg_parts<MD>()];
 #pragma unroll
@@ -314,9 +314,9 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_fcg_spmv_stencil(FcgArgs<VT>
       if (ok) {
         const VT* q = buf + (size_t)b * kStTaps * 32 + lane;
         if (inside)
-          stencil_plane_shfl<false, true>(q, z, i + fxy * dz, fx, n, lane, acc);
+          stencil_plane_shfl<false>(q, z, i + fxy * dz, fx, n, lane, acc);
         else
-          stencil_plane_shfl<true, true>(q, z, i + fxy * dz, fx, n, lane, acc);
+          stencil_plane_shfl<true>(q, z, i + fxy * dz, fx, n, lane, acc);
       }
       __syncwarp();
       if (ok) issue(k + kStBuf);
@@ -347,7 +347,7 @@ template <class VT, int MD>
 __global__ void __launch_bounds__(kCombineThreads) k_fcg_combine(FcgArgs<VT> a, CoarseArgs<VT> ca,
                                                                  const float* __restrict__ wst,
                                                                  const int* __restrict__ wlo,
-                                                                 const VT* __restrict__ e) {
+                                                                 const VT* e) {
   pdl_wait();
   pdl_trigger();
   if (*a.st.done) return;

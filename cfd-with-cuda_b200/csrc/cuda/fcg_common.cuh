@@ -20,12 +20,12 @@ constexpr int kFcgParts = fcg_parts<kFcgMaxM>();
 
 template <class VT>
 __device__ __forceinline__ VT sell_row(const int* __restrict__ off, const int* __restrict__ col,
-                                       const VT* __restrict__ val, const VT* __restrict__ x, int i) {
+                                       const VT* __restrict__ val, const VT* x, int i) {
   const int s = i >> 5, l = i & 31;
   const int bb = __ldg(off + s) + l, w = (__ldg(off + s + 1) - __ldg(off + s)) >> 5;
   VT q = 0;
 #pragma unroll 4
-  for (int j = 0; j < w; j++) q += __ldcs(val + bb + 32 * j) * __ldg(x + __ldcs(col + bb + 32 * j));
+  for (int j = 0; j < w; j++) q += __ldcs(val + bb + 32 * j) * x[__ldcs(col + bb + 32 * j)];
   return q;
 }
 
@@ -68,41 +68,15 @@ constexpr size_t stencil_smem_bytes() {
 }
 
 // One dz plane of a row (25 taps, coefficients q[t * 32] in shared memory)
-// into the five per-dy accumulators.
-template <bool CLAMP, class VT>
-__device__ __forceinline__ void stencil_plane(const VT* q, const VT* __restrict__ z, int base, int fx, int n,
-                                              VT (&acc)[5]) {
-#pragma unroll
-  for (int dy = -2; dy <= 2; dy++) {
-    const int rb = base + fx * dy;
-#pragma unroll
-    for (int dx = -2; dx <= 2; dx++) {
-      VT zv;
-      if constexpr (CLAMP) {
-        int j = rb + dx;
-        j = j < 0 ? 0 : (j >= n ? n - 1 : j);
-        zv = __ldg(z + j);
-      } else {
-        zv = __ldg(z + rb + dx);
-      }
-      acc[dy + 2] += q[((dy + 2) * 5 + dx + 2) * 32] * zv;
-    }
-  }
-}
-
-// The same plane with the gathers shared across the warp: the 32 rows of a
+// into the five per-dy accumulators, with the gathers shared across the warp: the 32 rows of a
 // slice are consecutive grid nodes, so lane l + dx holds z[rb(l) + dx] of
 // lane l.  Lane l loads z[rb(l) - 2] and lanes 0..3 the four values past the
 // warp's window; the five dx taps then come from shuffles.  Two loads per
-// dy row instead of five, identical products and sums.  NC: read-only
-// (non-coherent) loads, for a z that no thread of the launch writes.
-template <bool NC, class VT>
-__device__ __forceinline__ VT ld_z(const VT* z, int j) {
-  if constexpr (NC) return __ldg(z + j);
-  return z[j];
-}
-template <bool CLAMP, bool NC, class VT>
-__device__ __forceinline__ void stencil_plane_shfl(const VT* q, const VT* __restrict__ z, int base, int fx, int n,
+// dy row instead of five.  z is written by the kernel before, which may still
+// run when this one starts, so it is read with plain loads (no __ldg, no
+// __restrict__: those promise data that nobody writes while the kernel lives).
+template <bool CLAMP, class VT>
+__device__ __forceinline__ void stencil_plane_shfl(const VT* q, const VT* z, int base, int fx, int n,
                                                    int lane, VT (&acc)[5]) {
 #pragma unroll
   for (int dy = -2; dy <= 2; dy++) {
@@ -112,8 +86,8 @@ __device__ __forceinline__ void stencil_plane_shfl(const VT* q, const VT* __rest
       j0 = j0 < 0 ? 0 : (j0 >= n ? n - 1 : j0);
       j1 = j1 < 0 ? 0 : (j1 >= n ? n - 1 : j1);
     }
-    const VT w0 = ld_z<NC>(z, j0);
-    const VT w1 = lane < 4 ? ld_z<NC>(z, j1) : (VT)0;
+    const VT w0 = z[j0];
+    const VT w1 = lane < 4 ? z[j1] : (VT)0;
 #pragma unroll
     for (int dx = -2; dx <= 2; dx++) {
       VT zv;

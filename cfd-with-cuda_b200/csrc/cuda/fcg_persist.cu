@@ -369,9 +369,9 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_fcg2l(FcgArgs<float> a, Coar
           }
           const float* q = buf + (size_t)b * kStTaps * 32 + lane;
           if (inside)
-            stencil_plane_shfl<false, false>(q, z, i + fxy * dz, fx, n, lane, acc);
+            stencil_plane_shfl<false>(q, z, i + fxy * dz, fx, n, lane, acc);
           else
-            stencil_plane_shfl<true, false>(q, z, i + fxy * dz, fx, n, lane, acc);
+            stencil_plane_shfl<true>(q, z, i + fxy * dz, fx, n, lane, acc);
           __syncwarp();
           pend_lo = K + 1;
           issue(k + kStBuf);
