@@ -386,7 +386,7 @@ int device_patterns(cfd_ctx* c, bool& built) {
   cudaStream_t s = c->stream;
   const int NN = P.NN, NNp = P.NNp, NE = P.NE;
   const long long nent = 27LL * NE;
-  DevBuf<int> cnt, inc_rp, inc_el, pos, len, flag, adj_rp, adj_col;
+  DevBuf<int> cnt, inc_rp, inc_el, pos, len, big, flag, adj_rp, adj_col;
   CU(cnt.alloc(NN));
   CU(cudaMemsetAsync(cnt.p, 0, (size_t)NN * sizeof(int), s));
   CU(launch_incidence_count(nent, c->ltog.p, cnt.p, s));
@@ -402,11 +402,13 @@ int device_patterns(cfd_ctx* c, bool& built) {
   CU(flag.alloc(1));
   CU(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
   CU(len.alloc(std::max(NN, NE)));
+  CU(big.alloc((size_t)std::max(NN, NE) + 1));
   PatArgs a{};
   a.ltog = c->ltog.p;
   a.inc_rp = inc_rp.p;
   a.inc_el = inc_el.p;
   a.len = len.p;
+  a.big = big.p;
   a.overflow = flag.p;
   // one pattern: pass 0 (lengths), host row pointers, pass 1 (columns)
   auto one = [&](int mode, int nrows, DevBuf<int>& drp, DevBuf<int>& dcol, std::vector<int>& rp, int& maxlen,

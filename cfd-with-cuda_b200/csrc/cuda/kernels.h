@@ -412,6 +412,7 @@ struct PatArgs {
   const int* rp;                      // row pointers of the pattern written in pass 1
   int* col;                           // its columns (pass 1)
   int* len;                           // row lengths (pass 0)
+  int* big;                           // 1 + rows words: number and list of the rows too large for a warp
   int* overflow;                      // set when a row has more candidates than a block holds
 };
 // mode 0: K rows (nodes of the elements around a node), 1: G rows (their
