@@ -76,6 +76,11 @@ struct UnetNet {
   long long gcap[kUnetTensors] = {};
   float* lossv = nullptr;
   float* wg_work = nullptr;  // partial sums of one layer's weight gradient
+  // The backward pass runs the weight gradients on a stream of their own beside
+  // the chain of data gradients: ev_dout marks a layer's output gradient as
+  // ready, ev_wg the last weight gradient as done.
+  cudaStream_t wg_stream = nullptr;
+  cudaEvent_t ev_dout = nullptr, ev_wg = nullptr;
   long long wg_cap = 0;
   float* host_io = nullptr;  // device copies of host-side inputs and targets
   long long host_io_cap = 0;
