@@ -16,6 +16,8 @@
 //   take the columns q of G row v and add (G_d[v][q]*Minv[v]) * G_d[v][p] to
 //   a shared accumulator of row p.  Lanes of one v never collide, so the
 //   accumulation order is fixed (deterministic, ascending v as in the oracle).
+//   Bound by the chain of gathers and searches per v; reading the next v's row
+//   meanwhile: 30^3 elements 1.37 -> 1.12 ms.
 #include <cstdio>
 
 #include "kernels.h"
@@ -55,9 +57,30 @@ __device__ __forceinline__ T jacobian_inv(const T (*X)[3], const Basis* __restri
 
 constexpr int kAsmThreads = 128;
 
+// Slots of three columns in one sorted CSR row, or -1; the three searches run in
+// step, so that a round of loads costs one latency.
+__device__ __forceinline__ void search3(const int* __restrict__ col, int b, int e, const int* key, int (&slot)[3]) {
+  int lo[3] = {b, b, b};
+  for (int n = e - b; n > 1;) {
+    const int h = n >> 1;
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+      if (__ldg(col + lo[q] + h) <= key[q]) lo[q] += h;
+    n -= h;
+  }
+#pragma unroll
+  for (int q = 0; q < 3; q++) slot[q] = b < e && __ldg(col + lo[q]) == key[q] ? lo[q] : -1;
+}
+
+// Threads 0 .. 80 own a 3 x 3 tile of Ke each, threads 96 .. 122 a row of the
+// Ge_d (8 corners) and of Me: 2.1 shared-memory reads per entry and Gauss point
+// of Ke instead of 7, 9 searches in 3 chains instead of 6 x 1, and the row sums
+// of Me by sum_j Sv_j (27 steps; the double sum over j and Gauss points was a
+// serial 729 of one warp).  30^3 elements, 27 Gauss points: 1.80 -> 0.83 ms.
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
   __shared__ double sSv[kMaxNGP][27];
   __shared__ double sSp[kMaxNGP][8];
+  __shared__ double sum[kMaxNGP];  // sum_j Sv_j
   __shared__ double X[8][3];
   __shared__ int lt[27];
   __shared__ double iJ[kMaxNGP][3][3];
@@ -67,6 +90,12 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
   const Basis* B = a.basis;
   for (int i = t; i < ngp * 27; i += blockDim.x) sSv[i / 27][i % 27] = B->Sv[i / 27][i % 27];
   for (int i = t; i < ngp * 8; i += blockDim.x) sSp[i / 8][i % 8] = B->Sp[i / 8][i % 8];
+  __syncthreads();
+  if (t < ngp) {
+    double s = 0;
+    for (int j = 0; j < 27; j++) s += sSv[t][j];
+    sum[t] = s;
+  }
   for (int pos = a.e_begin + blockIdx.x; pos < a.e_end; pos += gridDim.x) {
     const int e = a.elist ? a.elist[pos] : pos;
     __syncthreads();
@@ -88,58 +117,69 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
       for (int i = 0; i < 3; i++) gd[k][j][i] = iJ[k][i][0] * r0 + iJ[k][i][1] * r1 + iJ[k][i][2] * r2;
     }
     __syncthreads();
-    // Ke and row sums of Me
-    for (int idx = t; idx < 729 + 27; idx += blockDim.x) {
-      if (idx < 729) {
-        int i = idx / 27, j = idx % 27;
-        double s = 0;
-        for (int k = 0; k < ngp; k++)
-          s += a.viscosity * (gd[k][i][0] * gd[k][j][0] + gd[k][i][1] * gd[k][j][1] + gd[k][i][2] * gd[k][j][2]) *
-               wd[k];
-        int row = lt[i], col = lt[j];
-        int slot = bsearch_slot(a.k_col, a.k_rp[row], a.k_rp[row + 1], col);
-        if (slot >= 0) {
-          if (a.plain)
-            a.kval[slot] += s;
-          else
-            atomicAdd(a.kval + slot, s);
-        }
-      } else {
-        int i = idx - 729;
-        double s = 0;
-        for (int j = 0; j < 27; j++) {
-          double mij = 0;
-          for (int k = 0; k < ngp; k++) mij += sSv[k][i] * sSv[k][j] * wd[k];
-          s += mij;
-        }
-        if (a.plain)
-          a.msum[lt[i]] += s;
-        else
-          atomicAdd(a.msum + lt[i], s);
-      }
-    }
-    // Ge_d[i][m] = -(1/rho) sum_k Sp[k][m] dSv_i/dx_d detJ w
-    for (int idx = t; idx < 216; idx += blockDim.x) {
-      int i = idx / 8, m = idx % 8;
-      double s0 = 0, s1 = 0, s2 = 0;
+    auto add = [&](double* to, double s) {
+      if (a.plain)
+        *to += s;
+      else
+        atomicAdd(to, s);
+    };
+    if (t < 81) {
+      const int i0 = 3 * (t / 9), j0 = 3 * (t % 9);
+      double s[3][3] = {};
       for (int k = 0; k < ngp; k++) {
-        double f = a.inv_density * sSp[k][m];
-        s0 -= f * gd[k][i][0] * wd[k];
-        s1 -= f * gd[k][i][1] * wd[k];
-        s2 -= f * gd[k][i][2] * wd[k];
+        double u[3][3], v[3][3];
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+#pragma unroll
+          for (int d = 0; d < 3; d++) {
+            u[m][d] = gd[k][i0 + m][d];
+            v[m][d] = gd[k][j0 + m][d];
+          }
+        const double w = wd[k];
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+#pragma unroll
+          for (int n = 0; n < 3; n++)
+            s[m][n] += a.viscosity * (u[m][0] * v[n][0] + u[m][1] * v[n][1] + u[m][2] * v[n][2]) * w;
       }
-      int row = lt[i], col = lt[m];
-      int slot = bsearch_slot(a.g_col, a.g_rp[row], a.g_rp[row + 1], col);
-      if (slot >= 0) {
-        if (a.plain) {
-          a.g1[slot] += s0;
-          a.g2[slot] += s1;
-          a.g3[slot] += s2;
-        } else {
-          atomicAdd(a.g1 + slot, s0);
-          atomicAdd(a.g2 + slot, s1);
-          atomicAdd(a.g3 + slot, s2);
+#pragma unroll
+      for (int m = 0; m < 3; m++) {
+        const int row = lt[i0 + m];
+        int slot[3];
+        search3(a.k_col, a.k_rp[row], a.k_rp[row + 1], lt + j0, slot);
+#pragma unroll
+        for (int n = 0; n < 3; n++)
+          if (slot[n] >= 0) add(a.kval + slot[n], s[m][n]);
+      }
+    } else if (t >= 96 && t < 96 + 27) {
+      // Ge_d[i][m] = -(1/rho) sum_k Sp[k][m] dSv_i/dx_d detJ w
+      const int i = t - 96, row = lt[i];
+      double s[8][3] = {}, ms = 0;
+      for (int k = 0; k < ngp; k++) {
+        const double w = wd[k], g0 = gd[k][i][0], g1 = gd[k][i][1], g2 = gd[k][i][2];
+        ms += sSv[k][i] * sum[k] * w;
+#pragma unroll
+        for (int m = 0; m < 8; m++) {
+          const double f = a.inv_density * sSp[k][m];
+          s[m][0] -= f * g0 * w;
+          s[m][1] -= f * g1 * w;
+          s[m][2] -= f * g2 * w;
         }
+      }
+      add(a.msum + row, ms);
+      const int b = a.g_rp[row], end = a.g_rp[row + 1];
+#pragma unroll
+      for (int m0 = 0; m0 < 9; m0 += 3) {
+        const int key[3] = {lt[m0], lt[m0 + 1], m0 + 2 < 8 ? lt[m0 + 2] : lt[m0]};
+        int slot[3];
+        search3(a.g_col, b, end, key, slot);
+#pragma unroll
+        for (int n = 0; n < 3; n++)
+          if (m0 + n < 8 && slot[n] >= 0) {
+            add(a.g1 + slot[n], s[m0 + n][0]);
+            add(a.g2 + slot[n], s[m0 + n][1]);
+            add(a.g3 + slot[n], s[m0 + n][2]);
+          }
       }
     }
   }
@@ -193,19 +233,61 @@ __global__ void __launch_bounds__(32 * kZWarps) k_build_z(ZArgs a) {
       acc[2 * stride + i] = 0.0;
     }
     __syncwarp();
-    for (int t = a.gt_rp[p]; t < a.gt_rp[p + 1]; t++) {
-      const int v = a.gt_col[t];
-      const double m = a.minv_orig[v];
-      const double p1 = a.gt1[t], p2 = a.gt2[t], p3 = a.gt3[t];
-      for (int j = a.g_rp[v] + lane; j < a.g_rp[v + 1]; j += 32) {
-        int pos = bsearch_smem(cols, len, a.g_col[j]);
-        if (pos >= 0) {
-          acc[pos] += (a.g1[j] * m) * p1;
-          acc[stride + pos] += (a.g2[j] * m) * p2;
-          acc[2 * stride + pos] += (a.g3[j] * m) * p3;
-        }
+    const int t1 = a.gt_rp[p + 1];
+    for (int tc = a.gt_rp[p]; tc < t1; tc += 32) {
+      // lane l holds entry tc + l of G^T; the G row of the next one is read
+      // while the current one is added
+      const int nt = min(32, t1 - tc);
+      int jb = 0, je = 0;
+      double lm = 0, l1 = 0, l2 = 0, l3 = 0;
+      if (lane < nt) {
+        const int v = a.gt_col[tc + lane];
+        lm = a.minv_orig[v];
+        l1 = a.gt1[tc + lane];
+        l2 = a.gt2[tc + lane];
+        l3 = a.gt3[tc + lane];
+        jb = a.g_rp[v];
+        je = a.g_rp[v + 1];
       }
-      __syncwarp();
+      int j = 0, e = 0, c = -1;
+      double x1 = 0, x2 = 0, x3 = 0;
+      auto fetch = [&](int q) {
+        j = __shfl_sync(0xffffffffu, jb, q) + lane;
+        e = __shfl_sync(0xffffffffu, je, q);
+        c = -1;
+        if (j < e) {
+          c = a.g_col[j];
+          x1 = a.g1[j];
+          x2 = a.g2[j];
+          x3 = a.g3[j];
+        }
+      };
+      fetch(0);
+      for (int q = 0; q < nt; q++) {
+        const double m = __shfl_sync(0xffffffffu, lm, q), p1 = __shfl_sync(0xffffffffu, l1, q);
+        const double p2 = __shfl_sync(0xffffffffu, l2, q), p3 = __shfl_sync(0xffffffffu, l3, q);
+        int jj = j, cc = c;
+        const int ee = e;
+        double y1 = x1, y2 = x2, y3 = x3;
+        if (q + 1 < nt) fetch(q + 1);
+        while (cc >= 0) {
+          const int pos = bsearch_smem(cols, len, cc);
+          if (pos >= 0) {
+            acc[pos] += (y1 * m) * p1;
+            acc[stride + pos] += (y2 * m) * p2;
+            acc[2 * stride + pos] += (y3 * m) * p3;
+          }
+          jj += 32;  // rows longer than a warp
+          cc = -1;
+          if (jj < ee) {
+            cc = a.g_col[jj];
+            y1 = a.g1[jj];
+            y2 = a.g2[jj];
+            y3 = a.g3[jj];
+          }
+        }
+        __syncwarp();
+      }
     }
     for (int i = lane; i < len; i += 32) {
       double z = (acc[i] + acc[stride + i]) + acc[2 * stride + i];

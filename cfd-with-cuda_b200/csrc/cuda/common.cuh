@@ -226,18 +226,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* m, unsigne
   return true;
 }
 
-// Position of key in the sorted range col[b, e); -1 when absent.
-__device__ __forceinline__ int bsearch_slot(const int* __restrict__ col, int b, int e, int key) {
-  int lo = b, hi = e - 1;
-  while (lo <= hi) {
-    int mid = (lo + hi) >> 1;
-    int c = __ldg(col + mid);
-    if (c == key) return mid;
-    if (c < key) lo = mid + 1; else hi = mid - 1;
-  }
-  return -1;
-}
-
 // Kernel launch, with the programmatic-stream-serialisation attribute when
 // pdl is set (the kernel must then call pdl_wait() before it reads what the
 // previous kernel wrote).
