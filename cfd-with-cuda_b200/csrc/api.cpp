@@ -161,7 +161,7 @@ struct cfd_ctx {
   // the persistent PCG (0: too many rows for it) and of the one-pass kernels
   DevBuf<int> zd_off;
   DevBuf<double> zd_coef;
-  int zd_ntap = 0, zd_reach = 0, dia_grid = 0, dia_apply = 0;
+  int zd_ntap = 0, zd_reach = 0, dia_grid = 0, dia_cluster = 0, dia_apply = 0;
   DiaArgs dia() const { return DiaArgs{(int)P.NNp, zd_ntap, zd_reach, zd_off.p, zd_coef.p}; }
   DevBuf<int> nb64, nb32;  // per PCG block: [lo..., hi...] neighbour block ranges
   DevBuf<int> cg_err;
@@ -734,7 +734,7 @@ int upload_problem(cfd_ctx* c) {
 // iteration bounds and not its bytes, at any fill).
 int find_diagonals(cfd_ctx* c) {
   const int n = (int)c->P.NNp;
-  c->zd_ntap = c->dia_grid = c->dia_apply = 0;
+  c->zd_ntap = c->dia_grid = c->dia_cluster = c->dia_apply = 0;
   c->zd_off.reset();
   c->zd_coef.reset();
   const int apply = dia_apply_grid(n, c->num_sms);
@@ -758,6 +758,7 @@ int find_diagonals(cfd_ctx* c) {
   c->zd_ntap = ntap;
   c->zd_reach = std::max(-off.front(), off.back());
   c->dia_grid = pcg_dia_grid(n, c->device);
+  c->dia_cluster = c->dia_grid > 0 ? pcg_cluster_blocks(n, c->zd_ntap) : 0;
   c->dia_apply = apply;
   return CFD_OK;
 }
@@ -766,8 +767,10 @@ int find_diagonals(cfd_ctx* c) {
 
 int run_pcg64(cfd_ctx* c, const double* b, double* x, int warm, double rtol, int maxit, double* res) {
   cudaStream_t s = c->stream;
-  CU(cudaMemsetAsync(c->cg_sync.p, 0, c->cg_sync.bytes(), s));
-  CU(cudaMemsetAsync(c->cg_err.p, 0, sizeof(int), s));
+  if (c->dia_cluster == 0) {  // the one-cluster form has neither counters nor an error word
+    CU(cudaMemsetAsync(c->cg_sync.p, 0, c->cg_sync.bytes(), s));
+    CU(cudaMemsetAsync(c->cg_err.p, 0, sizeof(int), s));
+  }
   if (c->dia_grid > 0) {
     PcgDiaArgs a{};
     a.d = c->dia();
@@ -775,7 +778,7 @@ int run_pcg64(cfd_ctx* c, const double* b, double* x, int warm, double rtol, int
     a.part = c->cg_part.p; a.sync = c->cg_sync.p; a.err = c->cg_err.p;
     a.rtol = rtol; a.maxit = maxit; a.warm = warm; a.result = c->cg_res.p;
     a.timeout_ns = 2000000000ULL;
-    KL(CFD_K_PCG64, launch_pcg_dia(a, c->dia_grid, s));
+    KL(CFD_K_PCG64, launch_pcg_dia(a, c->dia_grid, c->dia_cluster, s));
   } else {
     PcgArgs<double> a{};
     a.n = c->P.NNp;

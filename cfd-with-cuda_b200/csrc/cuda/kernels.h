@@ -213,13 +213,17 @@ struct PcgDiaArgs {
   unsigned long long timeout_ns;
 };
 int pcg_dia_grid(int n, int device);
+// Blocks of the one-cluster form of the solve (0: the matrix does not fit the
+// shared memory of a cluster, or the device has no room for one).
+int pcg_cluster_blocks(int n, int ntap);
 // Blocks of the one-pass kernels (0: n too large for them), and the residual
 // r = b - Z x with rf = (float) r (may be null) and per-block partials of r^2.
 // when (may be null): the kernel does nothing while *when is 0.
 int dia_apply_grid(int n, int num_sms);
 cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
                                 int grid, const int* when, cudaStream_t s);
-cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s);
+// cluster > 0: the one-cluster form on that many blocks, else grid blocks.
+cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, int cluster, cudaStream_t s);
 template <class VT>
 struct PcgArgs {
   int n;

@@ -179,6 +179,242 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   }
 }
 
+// ---- small grids: the same iteration in one cluster of up to 16 blocks ----
+// Block k of C owns slices as above, one row per thread with its ten vector
+// entries in registers; the whole matrix stays in the cluster, in registers where
+// a warp has one group of taps (ONE), else in shared memory.  Each block keeps the
+// m it gathers (double buffered) in shared memory: a block writes its rows of m
+// straight into the copies of the blocks that gather them, and its partial sums
+// into every block, and one hardware cluster barrier per iteration covers both.
+// No flag, no poll, no trip to L2.  A seventeenth warp adds the partials (in the
+// same order in every block, so all take the same decisions) and forms alpha and
+// beta beside the product.  Bound by latency: the product's chain, the row sums,
+// the block's sums and the barrier.  us per iteration, launch included, on cavities of
+// n^3 elements (the matrix of 12^3 no longer fits the shared memory of 16 blocks;
+// with part of it streamed from L2 13^3 took 5.8 against 5.3, 16^3 8.1 against 7.1):
+//   n              2    4    6    8    10   11
+//   k_pcg_dia      4.6  5.0  4.7  4.9  5.7  5.1
+//   k_pcg_cluster  2.4  2.3  2.4  2.5  2.9  3.1
+// Vectors in shared memory and the scalars in every thread instead: 3.4 to 4.5.
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+constexpr int kClMax = 16;                       // blocks of a cluster at most
+constexpr int kClThreads = kDiaThreads + 32;     // the product's warps and the scalars' one
+
+// Groups of taps of a warp at most.
+int cluster_groups(int slices, int ntap) {
+  return (slices * ((ntap + kDiaGroup - 1) / kDiaGroup) + kDiaWarps - 1) / kDiaWarps;
+}
+// Shared memory of a block: slots of its slices, two copies of m, the
+// coefficients where a warp has more than one group.
+size_t cluster_smem(int n, int slices, int ntap) {
+  const int groups = cluster_groups(slices, ntap);
+  return dia_slot_bytes(slices) + 2 * (size_t)n * sizeof(double) +
+         (groups > 1 ? (size_t)groups * kDiaWarps * kDiaGroup * 32 * sizeof(double) : 0);
+}
+
+template <bool ONE>
+__global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(PcgDiaArgs a, int groups) {
+  extern __shared__ double sv[];
+  __shared__ __align__(16) int soff[kDiaMaxTaps + kDiaGroup];
+  __shared__ double spart[2][kClMax][4], swarp[kDiaWarps][4], sred[4];
+  __shared__ int sstat;
+  const int n = a.d.n, nslices = (n + 31) >> 5, C = gridDim.x, rank = blockIdx.x;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int s0 = (int)((long long)nslices * rank / C), ns = (int)((long long)nslices * (rank + 1) / C) - s0;
+  const int ng = (a.d.ntap + kDiaGroup - 1) / kDiaGroup, T = ns * ng;
+  const int g0 = T * min(warp, kDiaWarps) / kDiaWarps, g1 = T * min(warp + 1, kDiaWarps) / kDiaWarps;
+  // the copies of m lie at the same place in every block
+  double* const mb[2] = {sv, sv + n};
+  double(*const slot)[32] = reinterpret_cast<double(*)[32]>(sv + 2 * n);
+  double* const res = sv + 2 * n + (ns + kDiaWarps) * 32 + (size_t)warp * groups * kDiaGroup * 32 + lane;
+  const int r0 = 32 * s0, nr = min(32 * ns, n - r0), reach = a.d.reach;
+  const bool mine = t < nr;
+  const int row = r0 + t;
+  auto block_of = [&](int i) { return (int)(((long long)C * ((i >> 5) + 1) - 1) / nslices); };
+  const int lo = block_of(max(r0 - reach, 0)), hi = block_of(min(r0 + nr - 1 + reach, n - 1));
+  // warps that share the thread's row
+  const int w0 = warp < ns ? (kDiaWarps * (warp * ng + 1) - 1) / T : 0;
+  const int w1 = warp < ns ? (kDiaWarps * (warp + 1) * ng - 1) / T : -1;
+
+  for (int k = t; k < kDiaMaxTaps + kDiaGroup; k += kClThreads) soff[k] = k < a.d.ntap ? a.d.off[k] : 0;
+  for (int k = t; k < n; k += kClThreads) {
+    mb[0][k] = a.warm ? a.x[k] : 0.0;
+    mb[1][k] = 0.0;
+  }
+  // with fewer groups than warps some slots are never written
+  for (int k = t; k < (ns + kDiaWarps) * 32; k += kClThreads) slot[0][k] = 0.0;
+  double c[kDiaGroup];
+  for (int g = g0; g < g1; g++) {
+    const int sl = g / ng, t0 = (g - sl * ng) * kDiaGroup;
+    const double* p = a.d.coef + ((size_t)(s0 + sl) * a.d.ntap + t0) * 32 + lane;
+#pragma unroll
+    for (int k = 0; k < kDiaGroup; k++) {
+      c[k] = t0 + k < a.d.ntap ? __ldg(p + 32 * k) : 0.0;
+      if (!ONE) res[((g - g0) * kDiaGroup + k) * 32] = c[k];
+    }
+  }
+  __syncthreads();
+
+  auto product = [&](const double* v) {
+    if (g0 >= g1) return;
+    int sl = g0 / ng;
+    double acc[4] = {0, 0, 0, 0};
+    for (int g = g0; g < g1; g++) {
+      const int t0 = (g - sl * ng) * kDiaGroup, i0 = (s0 + sl) * 32, i = i0 + lane;
+      const double* rs = res + (g - g0) * kDiaGroup * 32;
+      const bool inside = i0 >= reach && i0 + 31 + reach < n;
+      double x[kDiaGroup];
+#pragma unroll
+      for (int k = 0; k < kDiaGroup; k += 4) {
+        const int4 o = *reinterpret_cast<const int4*>(soff + t0 + k);
+        const int j[4] = {i + o.x, i + o.y, i + o.z, i + o.w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) x[k + e] = v[inside ? j[e] : min(max(j[e], 0), n - 1)];
+      }
+#pragma unroll
+      for (int k = 0; k < kDiaGroup; k++) acc[k & 3] += (ONE ? c[k] : rs[k * 32]) * x[k];
+      if (g + 1 == g1 || g + 1 == (sl + 1) * ng) {
+        slot[sl + warp][lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        acc[0] = acc[1] = acc[2] = acc[3] = 0;
+        sl++;
+      }
+    }
+  };
+  auto row_sum = [&]() {
+    double y[4] = {0, 0, 0, 0};
+    for (int w = w0; w <= w1; w += 4)
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        if (w + e <= w1) y[e] += slot[warp + w + e][lane];
+    return (y[0] + y[1]) + (y[2] + y[3]);
+  };
+  auto send = [&](double* copy, double v) {  // the thread's m into the copies that gather it
+    for (int k = lo; k <= hi; k++) st_cluster(cluster_addr(copy + row, k), v);
+  };
+  // Sum over k < count of the four values at v[k]: lane l holds that of value l & 3.
+  auto sum4 = [&](const double (*v)[4], int count) {
+    const int k = lane >> 2;
+    double y = (k < count ? v[k][lane & 3] : 0.0) + (k + 8 < count ? v[k + 8][lane & 3] : 0.0);
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    return y;
+  };
+  auto post = [&](double (&v)[4], int buf) {  // the block's partial sums into every block
+    if (warp < ns) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) swarp[warp][k] = v[k];
+      }
+    }
+    __syncthreads();
+    if (warp == kDiaWarps) {
+      const double y = sum4(swarp, ns);
+      for (int k = lane >> 2; k < C; k += 8) st_cluster(cluster_addr(&spart[buf][rank][lane & 3], k), y);
+    }
+  };
+
+  if (a.warm) product(mb[0]);
+  cluster_barrier();  // every block runs and has set up its copies
+  double r = 0, u = 0, w = 0, z = 0, q = 0, s = 0, p = 0, x = 0, m = 0, dinv = 0;
+  double v[4] = {0, 0, 0, 0};
+  if (mine) {
+    const double bi = a.b[row];
+    dinv = a.dinv[row];
+    r = a.warm ? bi - row_sum() : bi;
+    u = r * dinv;
+    x = a.warm ? mb[0][row] : 0.0;
+    send(mb[1], u);
+    v[3] = bi * bi;
+  }
+  cluster_barrier();
+  product(mb[1]);
+  __syncthreads();
+  if (mine) {
+    w = row_sum();
+    m = w * dinv;
+    send(mb[0], m);
+    v[0] = r * u;
+    v[1] = w * u;
+    v[2] = r * r;
+  }
+  post(v, 0);
+  cluster_barrier();
+
+  double bnorm = 0, tol = 0, igam = 0, ialpha = 0;  // the scalars' warp
+  int its = 0;
+  for (int i = 0;; i++) {
+    if (warp == kDiaWarps) {
+      const double y = sum4(spart[i & 1], C);
+      const double gam = __shfl_sync(0xffffffffu, y, 0), del = __shfl_sync(0xffffffffu, y, 1);
+      const double rn = sqrt(__shfl_sync(0xffffffffu, y, 2));
+      if (i == 0) {
+        bnorm = sqrt(__shfl_sync(0xffffffffu, y, 3));
+        tol = a.rtol * bnorm;
+      }
+      int st = -1;
+      if (!isfinite(bnorm) || !isfinite(rn))
+        st = 2;
+      else if (bnorm == 0.0 || rn <= tol)
+        st = 0;
+      else if (i >= a.maxit)
+        st = 1;
+      const double beta = gam * igam, alpha = gam / (del - beta * gam * ialpha);  // i = 0: igam = 0
+      if (lane == 0) {
+        sred[0] = alpha;
+        sred[1] = beta;
+        sred[2] = bnorm == 0.0 ? 0.0 : rn;
+        sred[3] = bnorm;
+        sstat = st;
+      }
+      igam = 1.0 / gam;
+      ialpha = 1.0 / alpha;
+    } else {
+      product(mb[i & 1]);
+    }
+    __syncthreads();
+    if (sstat >= 0) break;
+    double d[4] = {0, 0, 0, 0};
+    if (mine) {
+      const double alpha = sred[0], beta = sred[1];
+      z = row_sum() + beta * z;
+      q = m + beta * q;
+      s = w + beta * s;
+      p = u + beta * p;
+      x += alpha * p;
+      r -= alpha * s;
+      u -= alpha * q;
+      w -= alpha * z;
+      m = w * dinv;
+      send(mb[(i + 1) & 1], m);
+      d[0] = r * u;
+      d[1] = w * u;
+      d[2] = r * r;
+    }
+    its++;
+    post(d, (i + 1) & 1);
+    cluster_barrier();
+  }
+  if (mine) a.x[row] = sstat == 0 && sred[3] == 0.0 ? 0.0 : x;
+  if (rank == 0 && t == 0) {
+    a.result[0] = its;
+    a.result[1] = sred[3] > 0 ? sred[2] / sred[3] : 0.0;
+    a.result[2] = sstat;
+    a.result[3] = sred[3];
+  }
+}
+
 // r = b - Z x in FP64, rf = (float) r, per-block partial of r^2: one pass over
 // the coefficients, bound by their stream (us on the 64^3 cavity: 68 on the
 // SELL-32 form, 47 here).
@@ -243,8 +479,59 @@ int pcg_dia_grid(int n, int device) {
   return dia_smem((ns + grid - 1) / grid) <= (size_t)kDiaMaxSmem ? grid : 0;
 }
 
-cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, cudaStream_t s) {
+namespace {
+using ClusterKernel = void (*)(PcgDiaArgs, int);
+// Launch of a cluster of C blocks; false when they cannot hold the matrix.
+bool cluster_config(int n, int ntap, int C, ClusterKernel& k, int& groups, cudaLaunchConfig_t& cfg,
+                    cudaLaunchAttribute& attr) {
+  const int ns = (n + 31) / 32, slices = (ns + C - 1) / C;
+  groups = cluster_groups(slices, ntap);
+  k = groups == 1 ? k_pcg_cluster<true> : k_pcg_cluster<false>;
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = cluster_smem(n, slices, ntap);
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = C;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  // a row per thread of the product's warps, and the shared memory of a block
+  return C <= ns && slices <= kDiaWarps && cfg.dynamicSmemBytes <= (size_t)kDiaMaxSmem &&
+         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem) == cudaSuccess &&
+         cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+}
+}  // namespace
+
+int pcg_cluster_blocks(int n, int ntap) {
+  if (n < 1 || ntap < 1 || ntap > kDiaMaxTaps) return 0;
+  const int ns = (n + 31) / 32;
+  int C = kClMax;
+  while (C > ns) C /= 2;
+  ClusterKernel k;
+  int groups = 0, active = 0;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  // not every device (or partition of one) has room for a cluster of 16
+  const bool ok = cluster_config(n, ntap, C, k, groups, cfg, attr) &&
+                  cudaOccupancyMaxActiveClusters(&active, k, &cfg) == cudaSuccess && active >= 1;
+  if (!ok) cudaGetLastError();
+  return ok ? C : 0;
+}
+
+cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, int cluster, cudaStream_t s) {
   const int ns = (a.d.n + 31) / 32;
+  if (cluster > 0) {
+    ClusterKernel k;
+    int groups = 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    if (cluster > kClMax || a.d.ntap < 1 || a.d.ntap > kDiaMaxTaps ||
+        !cluster_config(a.d.n, a.d.ntap, cluster, k, groups, cfg, attr))
+      return cudaErrorInvalidValue;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, k, a, groups);
+  }
   if (grid < 1 || grid > ns || a.d.ntap < 1 || a.d.ntap > kDiaMaxTaps) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(k_pcg_dia, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem);
   if (e != cudaSuccess) return e;
