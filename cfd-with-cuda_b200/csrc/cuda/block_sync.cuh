@@ -41,6 +41,8 @@ struct BlockSync {
   __device__ __forceinline__ bool give_up(unsigned long long t0) const {
     return ld_volatile_i32(err) != 0 || global_ns() - t0 > timeout_ns;
   }
+  // THREADS > 0: called by the block's first THREADS threads only.
+  template <int THREADS = 0>
   __device__ bool wait_nb(unsigned k) {
     __shared__ int ok;
     if (threadIdx.x < 32) {
@@ -67,43 +69,53 @@ struct BlockSync {
         ok = good;
       }
     }
-    __syncthreads();
+    if constexpr (THREADS > 0)
+      asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+    else
+      __syncthreads();
     return ok != 0;
   }
-  // Waits until `target` arrivals, then every block sums the partials in the
-  // same fixed order (FP64): all blocks see identical values.
+  // Waits until `target` arrivals, then sums the partials in one fixed order
+  // (FP64): every block sees identical values, in every lane.  Called by one warp.
+  template <int NV>
+  __device__ bool warp_red(unsigned target, const double* buf, double (&sum)[NV]) {
+    const int G = gridDim.x, lane = threadIdx.x & 31;
+    int good = 1;
+    const unsigned long long t0 = global_ns();
+    for (int spin = 1; ld_acquire_u32(cnt) < target; spin++) {
+      if (spin % kPollCheck == 0 && give_up(t0)) {
+        good = 0;
+        break;
+      }
+    }
+    good = __all_sync(0xffffffffu, good);
+#pragma unroll
+    for (int k = 0; k < NV; k++) sum[k] = 0;
+    if (!good) {
+      if (lane == 0) atomicExch(err, 1);
+      return false;
+    }
+#pragma unroll 5
+    for (int i = lane; i < G; i += 32)
+#pragma unroll
+      for (int k = 0; k < NV; k++) sum[k] += __ldcg(buf + (size_t)k * G + i);
+#pragma unroll
+    for (int k = 0; k < NV; k++) sum[k] = warp_sum(sum[k]);
+    return true;
+  }
+  // The same for the whole block, by its first warp.
   template <int NV>
   __device__ bool wait_red(unsigned target, const double* buf, double (&v)[NV]) {
     __shared__ double res[NV];
     __shared__ int ok;
-    const int G = gridDim.x;
     if (threadIdx.x < 32) {
-      int good = 1;
-      const unsigned long long t0 = global_ns();
-      for (int spin = 1; ld_acquire_u32(cnt) < target; spin++) {
-        if (spin % kPollCheck == 0 && give_up(t0)) {
-          good = 0;
-          break;
-        }
+      double sum[NV];
+      const bool good = warp_red<NV>(target, buf, sum);
+      if (threadIdx.x == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) res[k] = sum[k];
+        ok = good;
       }
-      good = __all_sync(0xffffffffu, good);
-      if (good) {
-        double sum[NV];
-#pragma unroll
-        for (int k = 0; k < NV; k++) sum[k] = 0;
-#pragma unroll 5
-        for (int i = threadIdx.x; i < G; i += 32)
-#pragma unroll
-          for (int k = 0; k < NV; k++) sum[k] += __ldcg(buf + (size_t)k * G + i);
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-          sum[k] = warp_sum(sum[k]);
-          if (threadIdx.x == 0) res[k] = sum[k];
-        }
-      } else if (threadIdx.x == 0) {
-        atomicExch(err, 1);
-      }
-      if (threadIdx.x == 0) ok = good;
     }
     __syncthreads();
 #pragma unroll

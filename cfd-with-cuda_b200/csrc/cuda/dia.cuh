@@ -29,19 +29,19 @@ __device__ __forceinline__ double ld_coef(const double* p, unsigned long long po
 }
 
 // The block's share of the matrix: slices [s0, s0 + ns), ng groups per slice.
-// Warp w owns groups [g0, g1) of the ns ng; its part of slice s goes to
+// Warp w of nw owns groups [g0, g1) of the ns ng; its part of slice s goes to
 // slot[s + w] (distinct for every warp and slice that meet).
 struct DiaRows {
   DiaArgs d;
   const int* off;  // shared memory
   double (*slot)[32];
-  int s0, ns, ng, g0, g1;
+  int nw, s0, ns, ng, g0, g1;
   // the first groups of every warp, keep_bytes over the whole matrix, stay
   // in L2 from one iteration of a solve to the next; the rest passes through
   int gk;
   unsigned long long keep, once;
 
-  __device__ __forceinline__ int owner(int g) const { return (kDiaWarps * (g + 1) - 1) / (ns * ng); }
+  __device__ __forceinline__ int owner(int g) const { return (nw * (g + 1) - 1) / (ns * ng); }
   // The coefficients of group g of the block.
   __device__ __forceinline__ void load(int g, int lane, double (&c)[kDiaGroup]) const {
     const int sl = g / ng, t0 = (g - sl * ng) * kDiaGroup;
@@ -100,9 +100,10 @@ struct DiaRows {
 constexpr double kPcgKeepBytes = 70e6;
 
 // Sets up the block's share and its offsets table (kDiaMaxTaps + kDiaGroup ints
-// of shared memory); slot: dia_slot_bytes(its slices).  The caller
+// of shared memory); slot: dia_slot_bytes(its slices); nw <= kDiaWarps.  The caller
 // synchronises the block before the first product.
-__device__ __forceinline__ DiaRows dia_rows(const DiaArgs& d, int* soff, double* slot, double keep_bytes) {
+__device__ __forceinline__ DiaRows dia_rows(const DiaArgs& d, int* soff, double* slot, double keep_bytes,
+                                            int nw = kDiaWarps) {
   const int nslices = (d.n + 31) >> 5, G = gridDim.x, warp = threadIdx.x >> 5;
   // padding taps: coefficient 0 at offset 0
   for (int k = threadIdx.x; k < kDiaMaxTaps + kDiaGroup; k += kDiaThreads) soff[k] = k < d.ntap ? d.off[k] : 0;
@@ -113,8 +114,9 @@ __device__ __forceinline__ DiaRows dia_rows(const DiaArgs& d, int* soff, double*
   M.ns = (int)((long long)nslices * (blockIdx.x + 1) / G) - M.s0;
   M.ng = (d.ntap + kDiaGroup - 1) / kDiaGroup;
   const int T = M.ns * M.ng;
-  M.g0 = T * warp / kDiaWarps;
-  M.g1 = T * (warp + 1) / kDiaWarps;
+  M.nw = nw;  // the warps from nw on own nothing
+  M.g0 = T * min(warp, nw) / nw;
+  M.g1 = T * min(warp + 1, nw) / nw;
   M.slot = reinterpret_cast<double(*)[32]>(slot);
   M.keep = l2_evict_last();
   M.once = l2_evict_first();

@@ -9,25 +9,30 @@
 // - One block of 16 warps per SM owns a contiguous range of 32-row slices, and
 //   all ten vectors of its rows stay in shared memory; only m, which other
 //   blocks gather, is published to global memory.
-// - The products are split evenly over the block's warps in groups of 16 taps,
-//   whatever the number of slices: a warp owns a contiguous run of groups, and
-//   a slice that several warps share has a partial sum from each, added in
-//   warp order.  So a grid of one slice per block (729 rows) still has 8 warps
-//   at work on it.  The coefficients of the next group are loaded while the
-//   current one multiplies, and those of the first while the block waits for
-//   its neighbours.
-// - The dot products of an iteration are posted before its SpMV and
-//   collected after it; blocks wait only for the blocks whose rows they
-//   gather.  Every wait is bounded.
+// - The products are split evenly over the block's warps in groups of 16
+//   taps, whatever the number of slices: a warp owns a contiguous run of groups,
+//   and a slice that several warps share has a partial sum from each, added in
+//   warp order.  The coefficients of the next group are loaded while the current
+//   one multiplies, and those of the first while the block waits for its
+//   neighbours.
+// - The dot products of an iteration are posted before its SpMV.  One warp
+//   collects them and forms alpha and beta: beside the SpMV, which it then takes
+//   no part in, up to 12 slices per block (BESIDE), after it above that, where a
+//   sixteenth of the loads in flight is worth more (the first form below / after /
+//   beside: 40^3, 14.5 slices, 14.5 / - / 15.2, 48^3 20.3 / 19.6 / 19.1 to 19.6, 64^3
+//   41.0 / 40.0 / 44.1 on one device).  The other warps wait only for
+//   the blocks whose rows they gather.  Every wait is bounded.
 //
 // What bounds it: the coefficient stream on large grids; the latency of the
-// two waits, the gathers and the block sums on small ones.  Measured per
-// iteration on cavities of n^3 elements, against k_pcg on the SELL-32 form (us):
-//   n          4     8     16    24    32    48    64
-//   k_pcg      15.8  17.0  19.9  20.4  21.2  42    77.5
-//   k_pcg_dia  4.7   5.1   6.5   8.4   10.6  19.6  43.7
+// wait for the neighbours, the gathers and the block sums on small ones.  Measured
+// per iteration on cavities of n^3 elements, against k_pcg on the SELL-32 form (us):
+//   n                     12    14    16    20    24    28    32    40    48    64
+//   k_pcg                             19.9        20.4        21.2        42    77.5
+//   sums after the SpMV,
+//   scalars by all        5.7   6.4   6.6   7.1   8.4   9.7   10.4  15.0  19.9  44.0
+//   k_pcg_dia             5.9   5.8   6.1   6.0   7.8   8.1   9.4         19.6  43
 // of which L2 residence of part of the coefficients (dia.cuh) gave 13.0 -> 10.6
-// at n = 32 and 46 -> 43.7 at 64: 0.98 of the copy rate on the 275 MB.  Half
+// at n = 32 and 46 -> 43.7 at 64: the copy rate on the 275 MB.  Half
 // the coefficients (Z is symmetric) would halve that, but the mirror reads of
 // other blocks' rows come from L2 at about the same rate.  Keeping the
 // coefficients of small grids in the L1 changed nothing there and cost the
@@ -44,20 +49,28 @@ namespace {
 
 constexpr int kDiaVecs = 10;   // r u w z q s p x m dinv
 constexpr int kDiaMaxSmem = 224 * 1024;
+constexpr int kBesideSlices = 12;  // slices of a block up to which one of its warps only reduces
 
 size_t dia_smem(int slices) {
   return (size_t)slices * 32 * kDiaVecs * sizeof(double) + dia_slot_bytes(slices);
 }
 
+// BESIDE: the last warp only reduces, beside the SpMV; else the first one does, after it.
+template <bool BESIDE>
 __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
+  constexpr int PROD = BESIDE ? kDiaWarps - 1 : kDiaWarps;  // warps of the products and the rows
   extern __shared__ double sv[];
   __shared__ int soff[kDiaMaxTaps + kDiaGroup];
+  __shared__ double sred[4];  // alpha, beta, ||r||, ||b||
+  __shared__ int sstat, sdead;
   const int n = a.d.n, nslices = (n + 31) >> 5, G = gridDim.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool sums = warp == (BESIDE ? PROD : 0);  // the warp of the reductions
+  const bool rows = warp < PROD;
   const int R = 32 * ((int)((long long)nslices * (blockIdx.x + 1) / G) - (int)((long long)nslices * blockIdx.x / G));
   double *r = sv, *u = r + R, *w = u + R, *z = w + R, *q = z + R, *s = q + R, *p = s + R, *x = p + R, *m = x + R,
          *dinv = m + R;
-  const DiaRows M = dia_rows(a.d, soff, dinv + R, kPcgKeepBytes);
+  const DiaRows M = dia_rows(a.d, soff, dinv + R, kPcgKeepBytes, PROD);
   const int r0 = 32 * M.s0, nr = min(R, n - r0), reach = a.d.reach;
 
   auto block_of = [&](int row) { return (int)(((long long)G * ((row >> 5) + 1) - 1) / nslices); };
@@ -78,8 +91,9 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
     M.multiply(warp, lane, a.x, c);
     __syncthreads();
   }
+  if (threadIdx.x == 0) sdead = 0;
   double bb = 0;
-  for (int i = threadIdx.x; i < nr; i += kDiaThreads) {
+  for (int i = threadIdx.x; i < nr && rows; i += 32 * PROD) {
     const double bi = a.b[r0 + i], di = a.dinv[r0 + i];
     const double ri = a.warm ? bi - M.row(i >> 5, i & 31) : bi;
     r[i] = ri;
@@ -96,7 +110,7 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   if (alive) M.multiply(warp, lane, mb[1], c);
   __syncthreads();
   double v[4] = {0, 0, 0, bb};
-  for (int i = threadIdx.x; i < nr; i += kDiaThreads) {
+  for (int i = threadIdx.x; i < nr && rows; i += 32 * PROD) {
     const double wi = alive ? M.row(i >> 5, i & 31) : 0.0, mi = wi * dinv[i];
     w[i] = wi;
     m[i] = mi;
@@ -108,41 +122,55 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   block_partials<4>(v, a.part);
   bs.publish_arrive(2);
 
-  double bnorm = 0, tol = 0, rn = 0, gam_old = 1, alpha_old = 1;
-  int its = 0, status = 1;
+  double bnorm = 0, tol = 0, gam_old = 1, alpha_old = 1;  // the reductions' warp
+  int its = 0, status;
   for (int i = 0;; i++) {
-    // n_i = Z m_i  (neighbours' m_i published at phase i + 2)
-    if (alive) alive = bs.wait_nb((unsigned)i + 2);
-    if (alive) M.multiply(warp, lane, mb[i & 1], c);
-    // reduction of iteration i (posted before the SpMV); its barriers also
-    // order the slots' writes before the reads below
-    double red[4];
-    if (!alive || !bs.wait_red<4>((unsigned)(i + 1) * (unsigned)G, a.part + (size_t)(i & 1) * 4 * G, red)) {
-      status = 3;
-      break;
+    if (rows) {
+      // n_i = Z m_i  (neighbours' m_i published at phase i + 2)
+      if (alive) alive = bs.wait_nb<BESIDE ? 32 * PROD : 0>((unsigned)i + 2);
+      if (alive)
+        M.multiply(warp, lane, mb[i & 1], c);
+      else if (threadIdx.x == 0)
+        sdead = 1;
     }
-    if (i == 0) {
-      bnorm = sqrt(red[3]);
-      tol = a.rtol * bnorm;
+    if (sums) {
+      // reduction of iteration i, posted before the SpMV
+      double red[4];
+      const bool ok = bs.warp_red<4>((unsigned)(i + 1) * (unsigned)G, a.part + (size_t)(i & 1) * 4 * G, red);
+      if (i == 0) {
+        bnorm = sqrt(red[3]);
+        tol = a.rtol * bnorm;
+      }
+      const double rn = sqrt(red[2]);
+      int st = -1;
+      if (!ok)
+        st = 3;
+      else if (!isfinite(bnorm) || !isfinite(rn))
+        st = 2;
+      else if (bnorm == 0.0 || rn <= tol)
+        st = 0;
+      else if (i >= a.maxit)
+        st = 1;
+      const double gam = red[0], del = red[1];
+      const double beta = i > 0 ? gam / gam_old : 0.0;
+      const double alpha = i > 0 ? gam / (del - beta * gam / alpha_old) : gam / del;
+      gam_old = gam;
+      alpha_old = alpha;
+      if (lane == 0) {
+        sred[0] = alpha;
+        sred[1] = beta;
+        sred[2] = bnorm == 0.0 ? 0.0 : rn;
+        sred[3] = bnorm;
+        sstat = st;
+      }
     }
-    rn = sqrt(red[2]);
-    if (!isfinite(bnorm) || !isfinite(rn)) { status = 2; break; }
-    if (bnorm == 0.0) {
-      for (int k = threadIdx.x; k < nr; k += kDiaThreads) x[k] = 0.0;
-      rn = 0;
-      status = 0;
-      break;
-    }
-    if (rn <= tol) { status = 0; break; }
-    if (its >= a.maxit) { status = 1; break; }
-    const double gam = red[0], del = red[1];
-    const double beta = i > 0 ? gam / gam_old : 0.0;
-    const double alpha = i > 0 ? gam / (del - beta * gam / alpha_old) : gam / del;
-    gam_old = gam;
-    alpha_old = alpha;
+    __syncthreads();
+    status = sdead ? 3 : sstat;
+    if (status >= 0) break;
+    const double alpha = sred[0], beta = sred[1];
     double* mnext = mb[(i + 1) & 1];
     double d[4] = {0, 0, 0, 0};
-    for (int k = threadIdx.x; k < nr; k += kDiaThreads) {
+    for (int k = threadIdx.x; k < nr && rows; k += 32 * PROD) {
       const double zi = M.row(k >> 5, k & 31) + beta * z[k];
       const double qi = m[k] + beta * q[k];
       const double si = w[k] + beta * s[k];
@@ -169,13 +197,13 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
     block_partials<4>(d, a.part + (size_t)((i + 1) & 1) * 4 * G);
     bs.publish_arrive((unsigned)i + 3);
   }
-  __syncthreads();
-  for (int k = threadIdx.x; k < nr; k += kDiaThreads) a.x[r0 + k] = x[k];
+  const bool zero = status == 0 && sred[3] == 0.0;
+  for (int k = threadIdx.x; k < nr && rows; k += 32 * PROD) a.x[r0 + k] = zero ? 0.0 : x[k];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     a.result[0] = its;
-    a.result[1] = bnorm > 0 ? rn / bnorm : 0.0;
+    a.result[1] = sred[3] > 0 ? sred[2] / sred[3] : 0.0;
     a.result[2] = status;
-    a.result[3] = bnorm;
+    a.result[3] = sred[3];
   }
 }
 
@@ -207,8 +235,8 @@ __device__ __forceinline__ void st_cluster(unsigned addr, double v) {
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-constexpr int kClMax = 16;                       // blocks of a cluster at most
-constexpr int kClThreads = kDiaThreads + 32;     // the product's warps and the scalars' one
+constexpr int kClMax = 16;                      // blocks of a cluster at most
+constexpr int kClThreads = kDiaThreads + 32;    // the product's warps and the scalars' one
 
 // Groups of taps of a warp at most.
 int cluster_groups(int slices, int ntap) {
@@ -471,11 +499,13 @@ __global__ void k_dia_fill(DiaArgs d, const int* __restrict__ rp, const int* __r
 int pcg_dia_grid(int n, int device) {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1) return 0;
-  // one slice per block up to 96 slices, then three until every SM has a block:
-  // fewer blocks wait on fewer neighbours and arrivals (16^3, 154 slices: 8.0 us
-  // per iteration on 148 blocks, 6.7 on 51; 20^3, 290 slices: 9.2 on 148, 7.8 on
-  // 96; 12^3, 69 slices: 5.4 on 69, 6.0 on 23)
-  const int ns = (n + 31) / 32, grid = ns <= 96 ? std::min(sms, ns) : std::min(sms, (ns + 2) / 3);
+  // three slices per block until every SM has one: fewer blocks wait on fewer
+  // neighbours and arrivals.  us per iteration with 1 / 2 / 3 / 4 slices: 12^3 (69
+  // slices) 7.5 / 6.2 / 5.9 / 6.8, 13^3 5.3 / 5.4 / 5.6 / 6.1, 14^3 6.9 / 6.1 / 5.8 /
+  // 6.9, 16^3 8.0 / 6.2 / 6.6 / 7.6, 20^3 6.4 / 6.3 / 5.5 / 6.6, 22^3 7.6 / 7.5 / 6.4 /
+  // 8.4.  Smaller grids, where no cluster is to be had: one slice per block (729 rows
+  // on 23 blocks).
+  const int ns = (n + 31) / 32, grid = std::min(sms, ns <= 64 ? ns : (ns + 2) / 3);
   return dia_smem((ns + grid - 1) / grid) <= (size_t)kDiaMaxSmem ? grid : 0;
 }
 
@@ -533,12 +563,13 @@ cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, int cluster, cudaStrea
     return cudaLaunchKernelEx(&cfg, k, a, groups);
   }
   if (grid < 1 || grid > ns || a.d.ntap < 1 || a.d.ntap > kDiaMaxTaps) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_pcg_dia, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem);
+  const int slices = (ns + grid - 1) / grid;
+  const void* k = slices <= kBesideSlices ? (const void*)k_pcg_dia<true> : (const void*)k_pcg_dia<false>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem);
   if (e != cudaSuccess) return e;
   PcgDiaArgs args = a;
   void* params[] = {&args};
-  return cudaLaunchCooperativeKernel((const void*)k_pcg_dia, dim3(grid), dim3(kDiaThreads), params,
-                                     dia_smem((ns + grid - 1) / grid), s);
+  return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kDiaThreads), params, dia_smem(slices), s);
 }
 
 int dia_apply_grid(int n, int num_sms) { return dia_blocks(n, num_sms); }
