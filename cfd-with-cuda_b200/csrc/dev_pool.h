@@ -1,8 +1,8 @@
 // Device memory of one solver context, taken from the driver in a few large
 // blocks.  A context makes about ninety allocations while it loads a deck, and
 // every cudaMalloc and cudaFree synchronises the device and costs 0.1 to 0.4 ms
-// (up to tens of ms on a host whose GPUs are shared); a block costs about as
-// much as one of them.  New deck to first step on a graded 30^3 mesh (27
+// (tens of ms while other processes of the host allocate too); a block costs about
+// as much as one of them.  New deck to first step on a graded 30^3 mesh (27
 // Gauss points): 63 ms with an allocation per buffer, 36 ms from the pool.
 //
 // The pool belongs to its context (single-threaded use) and gives everything

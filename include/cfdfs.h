@@ -253,8 +253,7 @@ int cfd_unet_gradient(cfd_unet* net, const int dims[3], const float* x, const fl
                       float* loss, float* grad);
 /* Forward convolutions on the tensor cores (tcgen05, the default where the
  * layer shape allows: stride 1, 16/32/64 input channels) or all on the
- * CUDA-core kernels (on = 0).  The backward pass always uses the CUDA-core
- * kernels. */
+ * CUDA-core kernels (on = 0).  The backward pass is the same either way. */
 int cfd_unet_set_tensor_cores(cfd_unet* net, int on);
 /* CFD_E_TIMEOUT if a bounded wait inside a tensor-core convolution gave up
  * since the network was created (the output of that launch is invalid). */
