@@ -18,7 +18,7 @@
 //   corner coordinates are gathered with consecutive threads on consecutive
 //   elements at the same local node, which for a structured numbering are
 //   neighbouring nodes (few cache lines per warp request);
-// - TPE threads share an element, each owning GPT Gauss points: a nodal
+// - TPE threads share an element (four; more where there are few elements), each owning GPT Gauss points: a nodal
 //   value read from shared memory serves GPT Gauss points, and a warp reads
 //   the basis values of only TPE Gauss points per node at a time;
 // - the scatter again runs consecutive threads over consecutive elements.
@@ -260,7 +260,16 @@ cudaError_t launch_convect(const ConvArgs<T>& a, int num_sms, cudaStream_t s) {
   if (ne <= 0) return cudaSuccess;
   if (a.ngp > kMaxNGP || a.ngp < 1) return cudaErrorInvalidValue;
   // 4 threads per element, 32 elements per block: 2 Gauss points per thread
-  // at NGP 8, 7 at NGP 27
+  // at NGP 8, 7 at NGP 27.  Up to a few blocks per SM of a finer split (a small mesh, or
+  // one colour of it), whose latency is one Gauss point and a quarter (an eighth) of
+  // the block's gathers, that one: us per launch, events included, 4 / 16 threads per
+  // element in FP64, then in FP32, on n^3 elements: n = 8 18.2 / 12.3, 15.9 / 10.7;
+  // n = 12 18.5 / 14.6, 16.0 / 11.8; n = 16 18.6 / 19.1, 16.4 / 13.2; n = 20 23.0 / 28.8,
+  // 16.9 / 16.4; at NGP 27, 4 / 32 threads: n = 8 27.6 / 12.7, 21.0 / 11.9; n = 12 28.4
+  // / 16.7, 20.8 / 13.2; n = 16 28.7 / 29.2, 22.2 / 18.0.
+  if (ne <= (sizeof(T) == 8 ? 16 : 32) * num_sms)
+    return a.ngp <= 8 ? launch_convect_cfg<T, 16, 1>(a, ne, num_sms, s)
+                      : launch_convect_cfg<T, 32, 1>(a, ne, num_sms, s);
   if (a.ngp <= 8) return launch_convect_cfg<T, 4, 2>(a, ne, num_sms, s);
   return launch_convect_cfg<T, 4, 7>(a, ne, num_sms, s);
 }
