@@ -18,9 +18,10 @@
 //   corner coordinates are gathered with consecutive threads on consecutive
 //   elements at the same local node, which for a structured numbering are
 //   neighbouring nodes (few cache lines per warp request);
-// - TPE threads share an element (four; more where there are few elements), each owning GPT Gauss points: a nodal
-//   value read from shared memory serves GPT Gauss points, and a warp reads
-//   the basis values of only TPE Gauss points per node at a time;
+// - TPE threads share an element (four; in FP64 more where there are few elements),
+//   each owning GPT Gauss points: a nodal value read from shared memory serves GPT
+//   Gauss points, and a warp reads the basis values of only TPE Gauss points per
+//   node at a time;
 // - the scatter again runs consecutive threads over consecutive elements.
 // Results are scattered with FP64 atomics (no element colouring; in mixed
 // precision as one FP32 16-byte vector reduction per element node into an
@@ -260,16 +261,21 @@ cudaError_t launch_convect(const ConvArgs<T>& a, int num_sms, cudaStream_t s) {
   if (ne <= 0) return cudaSuccess;
   if (a.ngp > kMaxNGP || a.ngp < 1) return cudaErrorInvalidValue;
   // 4 threads per element, 32 elements per block: 2 Gauss points per thread
-  // at NGP 8, 7 at NGP 27.  Up to a few blocks per SM of a finer split (a small mesh, or
-  // one colour of it), whose latency is one Gauss point and a quarter (an eighth) of
-  // the block's gathers, that one: us per launch, events included, 4 / 16 threads per
-  // element in FP64, then in FP32, on n^3 elements: n = 8 18.2 / 12.3, 15.9 / 10.7;
-  // n = 12 18.5 / 14.6, 16.0 / 11.8; n = 16 18.6 / 19.1, 16.4 / 13.2; n = 20 23.0 / 28.8,
-  // 16.9 / 16.4; at NGP 27, 4 / 32 threads: n = 8 27.6 / 12.7, 21.0 / 11.9; n = 12 28.4
-  // / 16.7, 20.8 / 13.2; n = 16 28.7 / 29.2, 22.2 / 18.0.
-  if (ne <= (sizeof(T) == 8 ? 16 : 32) * num_sms)
-    return a.ngp <= 8 ? launch_convect_cfg<T, 16, 1>(a, ne, num_sms, s)
-                      : launch_convect_cfg<T, 32, 1>(a, ne, num_sms, s);
+  // at NGP 8, 7 at NGP 27.  FP64, up to a few blocks per SM of a finer split (a small
+  // mesh, or one colour of it), whose latency is one Gauss point and a quarter (an
+  // eighth) of the block's gathers, that one: us per launch, events included, 4 / 16
+  // threads per element on n^3 elements: n = 8 18.2 / 12.3, n = 12 18.5 / 14.6, n = 16
+  // 18.6 / 19.1, n = 20 23.0 / 28.8; at NGP 27, 4 / 32 threads: n = 8 27.6 / 12.7, n = 12
+  // 28.4 / 16.7, n = 16 28.7 / 29.2.  FP32 keeps the one form: the blocks add to a node
+  // in the order in which they arrive, and on a small mesh that order, and with it the
+  // rounding of the FP32 sum, goes with the elements of a block.  With the finer split
+  // (n = 8 15.9 / 10.7 us) the pressure of a mixed run on 12^3 elements moved by 4e-7,
+  // where the runs of one form repeat to the last bit.
+  if constexpr (sizeof(T) == 8) {
+    if (ne <= 16 * num_sms)
+      return a.ngp <= 8 ? launch_convect_cfg<T, 16, 1>(a, ne, num_sms, s)
+                        : launch_convect_cfg<T, 32, 1>(a, ne, num_sms, s);
+  }
   if (a.ngp <= 8) return launch_convect_cfg<T, 4, 2>(a, ne, num_sms, s);
   return launch_convect_cfg<T, 4, 7>(a, ne, num_sms, s);
 }
