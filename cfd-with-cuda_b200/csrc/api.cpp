@@ -708,7 +708,7 @@ int upload_problem(cfd_ctx* c) {
 
   CU(c->cg_err.alloc(1));
   c->res_blocks = residual_blocks((int)NNp, c->num_sms);
-  CU(c->ir_part.alloc(std::max(c->res_blocks, c->dia_apply)));
+  CU(c->ir_part.alloc(c->res_blocks));
   CU(c->ir_sum.alloc(2));
   c->nub = mixed(c) ? step3_blocks<float>((int)NN) : step3_blocks<double>((int)NN);
   c->npb = pupdate_blocks((int)NNp, c->num_sms);
@@ -1540,15 +1540,14 @@ bool fcg_path(const cfd_ctx* c) { return learned(c) || twolevel(c); }
 // ||r||_2^2 (device); when as launch_residual64.
 int queue_residual(cfd_ctx* c, const double* b, const double* x, double* out, const int* when = nullptr) {
   cudaStream_t s = c->stream;
-  int nparts = c->res_blocks;
-  if (x && c->dia_apply > 0) {
-    nparts = c->dia_apply;
-    KL(CFD_K_RESID64, launch_residual_dia(c->dia(), b, x, c->ir_r.p, c->f_b.p, c->ir_part.p, nparts, when, s));
+  if (x && c->zd_ntap > 0) {
+    KL(CFD_K_RESID64,
+       launch_residual_dia(c->dia(), b, x, c->ir_r.p, c->f_b.p, c->ir_part.p, c->res_blocks, when, s));
   } else {
     KL(CFD_K_RESID64, launch_residual64(c->P.NNp, c->zs_off.p, c->zs_col.p, c->zs_val.p, b, x, c->ir_r.p, c->f_b.p,
                                         c->ir_part.p, c->res_blocks, when, s));
   }
-  KL(CFD_K_OTHER, launch_sum_partials(c->ir_part.p, nparts, out, s));
+  KL(CFD_K_OTHER, launch_sum_partials(c->ir_part.p, c->res_blocks, out, s));
   return CFD_OK;
 }
 

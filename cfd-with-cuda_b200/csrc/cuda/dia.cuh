@@ -1,6 +1,6 @@
 // Products with a matrix stored by offsets (DiaArgs, kernels.h), for kernels
 // whose blocks each own a contiguous range of 32-row slices (pcg_dia.cu, the
-// FP64 SpMV of flexible CG, the FP64 residual).  The work of a block is split
+// FP64 SpMV of flexible CG).  The work of a block is split
 // evenly over its 16 warps in groups of 16 taps, and the coefficients of the
 // next group are loaded while the current one multiplies.
 #pragma once

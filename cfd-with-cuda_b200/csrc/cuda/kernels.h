@@ -216,12 +216,8 @@ int pcg_dia_grid(int n, int device);
 // Blocks of the one-cluster form of the solve (0: the matrix does not fit the
 // shared memory of a cluster, or the device has no room for one).
 int pcg_cluster_blocks(int n, int ntap);
-// Blocks of the one-pass kernels (0: n too large for them), and the residual
-// r = b - Z x with rf = (float) r (may be null) and per-block partials of r^2.
-// when (may be null): the kernel does nothing while *when is 0.
+// Blocks of the one-pass SpMV (0: n too large for it).
 int dia_apply_grid(int n, int num_sms);
-cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
-                                int grid, const int* when, cudaStream_t s);
 // cluster > 0: the one-cluster form on that many blocks, else grid blocks.
 cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, int cluster, cudaStream_t s);
 template <class VT>
@@ -452,10 +448,14 @@ template <class VT>
 int pcg_max_grid(int n, int device);
 
 // r = b - Z x (FP64, SELL-32 Z) and the partial sum of r^2 per block; rf = (float) r.
-// x == null stands for x = 0 (r = b, Z is not read).  when as above.
+// x == null stands for x = 0 (r = b, Z is not read).  when (may be null): the
+// kernel does nothing while *when is 0.
 cudaError_t launch_residual64(int n, const int* off, const int* col, const double* val, const double* b,
                               const double* x, double* r, float* rf, double* part, int nblocks, const int* when,
                               cudaStream_t s);
+// The same on the matrix by offsets, equal to the last bit.
+cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
+                                int nblocks, const int* when, cudaStream_t s);
 int residual_blocks(int n, int num_sms);
 cudaError_t launch_axpy_f2d(int n, const float* e, double* x, const int* when, cudaStream_t s);
 cudaError_t launch_sum_partials(const double* part, int n, double* out, cudaStream_t s);

@@ -244,6 +244,58 @@ __global__ void __launch_bounds__(kResThreads) k_residual64(int n, const int* __
   if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
 }
 
+constexpr int kResGroup = 16;
+
+// The same on the matrix by offsets: 8 bytes per entry instead of 12, no chain from
+// column to gather (us per launch in mixed runs, norms of b included, SELL-32 / here:
+// 8^3 16 / 10, 24^3 32 / 13, 64^3 55 / 36, duct of 24 x 24 x 160 35 / 18; groups of 8 or
+// 25 taps instead of 16: 64^3 41 / 36, 24^3 16 / 12).  A thread adds its row's products in
+// the order of the entries, in one sum, as k_residual64 does, and the blocks own the same
+// rows; a tap without an entry adds 0 x, so every number is equal to the last bit.  That
+// matters: r is rounded to FP32 for the next inner solve, and an entry that rounds
+// the other way moved the pressure of mixed runs by up to 1.5e-8 (rows split over a block's
+// warps: 8^3 8, 24^3 10, 64^3 38 us).
+__global__ void __launch_bounds__(kResThreads) k_residual_dia(DiaArgs d, const double* __restrict__ b,
+                                                               const double* __restrict__ x, double* r, float* rf,
+                                                               double* part, const int* when) {
+  if (when && *when == 0) return;
+  __shared__ int soff[kDiaMaxTaps + kResGroup];
+  for (int k = threadIdx.x; k < kDiaMaxTaps + kResGroup; k += kResThreads) soff[k] = k < d.ntap ? d.off[k] : 0;
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double acc[1] = {0};
+  if (i < d.n) {
+    const double* cf = d.coef + (size_t)(i >> 5) * d.ntap * 32 + (i & 31);
+    const int i0 = i & ~31;
+    const bool inside = i0 >= d.reach && i0 + 31 + d.reach < d.n;
+    double q = 0, c[kResGroup], y[kResGroup];
+    // the coefficients of the next taps are read while the current ones multiply
+    auto load = [&](int k0) {
+#pragma unroll
+      for (int k = 0; k < kResGroup; k++) c[k] = k0 + k < d.ntap ? __ldcs(cf + 32 * (k0 + k)) : 0.0;
+    };
+    load(0);
+    for (int k0 = 0; k0 < d.ntap; k0 += kResGroup) {
+      double v[kResGroup];
+#pragma unroll
+      for (int k = 0; k < kResGroup; k++) {
+        const int j = i + soff[k0 + k];
+        y[k] = __ldg(x + (inside ? j : min(max(j, 0), d.n - 1)));
+        v[k] = c[k];
+      }
+      load(k0 + kResGroup);
+#pragma unroll
+      for (int k = 0; k < kResGroup; k++) q += v[k] * y[k];
+    }
+    const double ri = b[i] - q;
+    r[i] = ri;
+    if (rf) rf[i] = (float)ri;
+    acc[0] = ri * ri;
+  }
+  block_sum<1>(acc);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
+}
+
 __global__ void k_axpy_f2d(int n, const float* __restrict__ e, double* x, const int* when) {
   if (when && *when == 0) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] += (double)e[i];
@@ -345,6 +397,13 @@ cudaError_t launch_residual64(int n, const int* off, const int* col, const doubl
                               const double* x, double* r, float* rf, double* part, int nblocks, const int* when,
                               cudaStream_t s) {
   k_residual64<<<nblocks, kResThreads, 0, s>>>(n, off, col, val, b, x, r, rf, part, when);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
+                                int nblocks, const int* when, cudaStream_t s) {
+  if (d.ntap < 1 || d.ntap > kDiaMaxTaps) return cudaErrorInvalidValue;
+  k_residual_dia<<<nblocks, kResThreads, 0, s>>>(d, b, x, r, rf, part, when);
   return cudaGetLastError();
 }
 

@@ -443,34 +443,6 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(PcgDiaArgs a, int
   }
 }
 
-// r = b - Z x in FP64, rf = (float) r, per-block partial of r^2: one pass over
-// the coefficients, bound by their stream (us on the 64^3 cavity: 68 on the
-// SELL-32 form, 47 here).
-__global__ void __launch_bounds__(kDiaThreads, 1) k_residual_dia(DiaArgs d, const double* __restrict__ b,
-                                                                 const double* __restrict__ x, double* r, float* rf,
-                                                                 double* part, const int* when) {
-  if (when && *when == 0) return;
-  extern __shared__ double sv[];
-  __shared__ int soff[kDiaMaxTaps + kDiaGroup];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const DiaRows M = dia_rows(d, soff, sv, 0.0);
-  double c[kDiaGroup];
-  if (M.g0 < M.g1) M.load(M.g0, lane, c);
-  __syncthreads();
-  M.multiply(warp, lane, x, c);
-  __syncthreads();
-  const int r0 = 32 * M.s0, nr = min(32 * M.ns, d.n - r0);
-  double v[1] = {0};
-  for (int i = threadIdx.x; i < nr; i += kDiaThreads) {
-    const double ri = b[r0 + i] - M.row(i >> 5, i & 31);
-    r[r0 + i] = ri;
-    if (rf) rf[r0 + i] = (float)ri;
-    v[0] += ri * ri;
-  }
-  block_sum<1>(v);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
-}
-
 __global__ void k_dia_mark(int n, const int* __restrict__ rp, const int* __restrict__ col, unsigned char* mark) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     for (int k = rp[i]; k < rp[i + 1]; k++) {
@@ -573,17 +545,6 @@ cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, int cluster, cudaStrea
 }
 
 int dia_apply_grid(int n, int num_sms) { return dia_blocks(n, num_sms); }
-
-cudaError_t launch_residual_dia(const DiaArgs& d, const double* b, const double* x, double* r, float* rf, double* part,
-                                int grid, const int* when, cudaStream_t s) {
-  const int ns = (d.n + 31) / 32;
-  if (grid < 1 || grid > ns || d.ntap < 1 || d.ntap > kDiaMaxTaps) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(k_residual_dia, cudaFuncAttributeMaxDynamicSharedMemorySize, kDiaMaxSmem);
-  if (e != cudaSuccess) return e;
-  k_residual_dia<<<grid, kDiaThreads, dia_slot_bytes((ns + grid - 1) / grid), s>>>(d, b, x, r, rf, part,
-                                                                                       when);
-  return cudaGetLastError();
-}
 
 cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, cudaStream_t s) {
   k_dia_mark<<<std::max(1, std::min((n + 255) / 256, 148 * 8)), 256, 0, s>>>(n, rp, col, mark);
