@@ -74,13 +74,16 @@ __device__ __forceinline__ void search3(const int* __restrict__ col, int b, int 
 
 // Threads 0 .. 80 own a 3 x 3 tile of Ke each, threads 96 .. 122 a row of the
 // Ge_d (8 corners) and of Me: 2.1 shared-memory reads per entry and Gauss point
-// of Ke instead of 7, 9 searches in 3 chains instead of 6 x 1, and the row sums
-// of Me by sum_j Sv_j (27 steps; the double sum over j and Gauss points was a
-// serial 729 of one warp).  30^3 elements, 27 Gauss points: 1.80 -> 0.83 ms.
+// of Ke instead of 7, 9 searches in 3 chains instead of 6 x 1.  The tiles of Me go
+// with those of Ke, and a row's 27 entries are then added in order (a serial 729 of one
+// warp before).  The order is kept because a lumped mass that differs in its last
+// bit changes the rounding of a mixed run's FP32 velocities: with the row sum as
+// sum_k Sv_i (sum_j Sv_j) wd its pressure moved by up to 3.5e-8.  30^3 elements, 27 Gauss
+// points: 1.80 -> 0.80 ms, 8 points 0.70 -> 0.52 (0.83 and 0.46 with that sum).
 __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
   __shared__ double sSv[kMaxNGP][27];
   __shared__ double sSp[kMaxNGP][8];
-  __shared__ double sum[kMaxNGP];  // sum_j Sv_j
+  __shared__ double sM[27][27];  // Me
   __shared__ double X[8][3];
   __shared__ int lt[27];
   __shared__ double iJ[kMaxNGP][3][3];
@@ -90,12 +93,6 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
   const Basis* B = a.basis;
   for (int i = t; i < ngp * 27; i += blockDim.x) sSv[i / 27][i % 27] = B->Sv[i / 27][i % 27];
   for (int i = t; i < ngp * 8; i += blockDim.x) sSp[i / 8][i % 8] = B->Sp[i / 8][i % 8];
-  __syncthreads();
-  if (t < ngp) {
-    double s = 0;
-    for (int j = 0; j < 27; j++) s += sSv[t][j];
-    sum[t] = s;
-  }
   for (int pos = a.e_begin + blockIdx.x; pos < a.e_end; pos += gridDim.x) {
     const int e = a.elist ? a.elist[pos] : pos;
     __syncthreads();
@@ -125,7 +122,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
     };
     if (t < 81) {
       const int i0 = 3 * (t / 9), j0 = 3 * (t % 9);
-      double s[3][3] = {};
+      double s[3][3] = {}, me[3][3] = {};
       for (int k = 0; k < ngp; k++) {
         double u[3][3], v[3][3];
 #pragma unroll
@@ -139,9 +136,15 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
 #pragma unroll
         for (int m = 0; m < 3; m++)
 #pragma unroll
-          for (int n = 0; n < 3; n++)
+          for (int n = 0; n < 3; n++) {
             s[m][n] += a.viscosity * (u[m][0] * v[n][0] + u[m][1] * v[n][1] + u[m][2] * v[n][2]) * w;
+            me[m][n] += sSv[k][i0 + m] * sSv[k][j0 + n] * w;
+          }
       }
+#pragma unroll
+      for (int m = 0; m < 3; m++)
+#pragma unroll
+        for (int n = 0; n < 3; n++) sM[i0 + m][j0 + n] = me[m][n];
 #pragma unroll
       for (int m = 0; m < 3; m++) {
         const int row = lt[i0 + m];
@@ -154,10 +157,9 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
     } else if (t >= 96 && t < 96 + 27) {
       // Ge_d[i][m] = -(1/rho) sum_k Sp[k][m] dSv_i/dx_d detJ w
       const int i = t - 96, row = lt[i];
-      double s[8][3] = {}, ms = 0;
+      double s[8][3] = {};
       for (int k = 0; k < ngp; k++) {
         const double w = wd[k], g0 = gd[k][i][0], g1 = gd[k][i][1], g2 = gd[k][i][2];
-        ms += sSv[k][i] * sum[k] * w;
 #pragma unroll
         for (int m = 0; m < 8; m++) {
           const double f = a.inv_density * sSp[k][m];
@@ -166,7 +168,6 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
           s[m][2] -= f * g2 * w;
         }
       }
-      add(a.msum + row, ms);
       const int b = a.g_rp[row], end = a.g_rp[row + 1];
 #pragma unroll
       for (int m0 = 0; m0 < 9; m0 += 3) {
@@ -181,6 +182,12 @@ __global__ void __launch_bounds__(kAsmThreads) k_assemble(AsmArgs a) {
             add(a.g3 + slot[n], s[m0 + n][2]);
           }
       }
+    }
+    __syncthreads();
+    if (t >= 96 && t < 96 + 27) {
+      double ms = 0;
+      for (int j = 0; j < 27; j++) ms += sM[t - 96][j];
+      add(a.msum + lt[t - 96], ms);
     }
   }
 }

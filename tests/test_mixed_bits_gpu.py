@@ -24,6 +24,8 @@ OPTIONS = {
 CASES = [
     # the FP64 residual between inner solves
     "duct_4_40_174.2_two_3", "cav_16_1_27_jac",
+    # the lumped mass
+    "duct_4_60_174.2_jac_3", "cav_12_1.5_8_jac",
 ]
 
 
