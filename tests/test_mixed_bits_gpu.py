@@ -26,6 +26,8 @@ CASES = [
     "duct_4_40_174.2_two_3", "cav_16_1_27_jac",
     # the lumped mass
     "duct_4_60_174.2_jac_3", "cav_12_1.5_8_jac",
+    # the coarse right-hand side of a line cut into ranges
+    "duct_6_70_250_two_3",
 ]
 
 
