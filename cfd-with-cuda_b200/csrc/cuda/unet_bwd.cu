@@ -3,13 +3,27 @@
 //
 // Weights and stored activations are BF16, so only the gradient g of a
 // layer's output needs more than the tensor core's input type.  It is split
-// exactly into three BF16 parts by truncation (8 + 8 + 8 = 24 mantissa bits),
-// and every product with it becomes three mma.sync.m16n8k16 that start from
-// zero and are chained lo, mid, hi; their sum over 16 terms is then added to
-// an FP32 accumulator in registers.  So no product is rounded, and the long
-// sums run in round-to-nearest FP32 adds, one per 16 terms, whatever the
-// tensor core does inside a step.  (A tensor-memory accumulator would carry
-// the whole sum through the tensor core's own additions.)
+// into three BF16 parts by truncation (8 + 8 + 8 = 24 mantissa bits: exact for
+// |g| >= 2^-110, below that off by less than 2^-133, BF16's smallest number),
+// and every product with it becomes three mma.sync of 16 terms, one per part,
+// each from zero.  The tensor core truncates what an addition inside a step shifts
+// out, always towards zero, which adds up over the layers where rounding does not;
+// so the parts are not chained through its accumulator but added in
+// round-to-nearest FP32, lo, mid, hi and then the running sum, and the data
+// gradient, whose errors every layer in front inherits, takes the hi part in two
+// steps of eight terms.  (A tensor-memory accumulator would carry the whole sum
+// through the tensor core's own additions.)  Error of a layer's weight gradient
+// against 64 bits from the same stored activations, first / middle / last layer, in
+// 1e-7:
+//                                        65^3               161 x 25 x 25
+//   FP32 on CUDA cores, atomics          1.5 / 1.2 / 1.6    1.1 / 1.8 / 1.1
+//   three parts chained                  1.1 / 2.1 / 0.26   1.8 / 2.2 / 0.27
+//   parts added apart                    0.62 / 1.3 / 0.26  1.1 / 1.4 / 0.27
+//   the same, hi in steps of eight       0.38 / 0.98 / 0.26 0.56 / 0.98 / 0.27
+//   (weight gradient in steps of eight too: 0.38 / 0.89 / 0.26, 0.56 / 0.83 / 0.27)
+// and the calls, in ms, gradient of 65^3 and batch of 4 on 161 x 25 x 25: chained 1.40
+// and 2.68, apart 1.44 and 2.74, hi in steps of eight 1.51 and 2.88, both kernels 1.55
+// and 2.95.
 //
 // Both kernels use the row numbering of the forward convolution: a block
 // stages a brick of voxels with a one-voxel halo in shared memory, rows
@@ -24,10 +38,9 @@
 // latency of staging, at one or two blocks per SM (the layers are small:
 // 0.5 to 3.8 GFLOP).  Measured on one sample of a 65^3 grid, against FP32
 // CUDA-core kernels with one voxel (data) or one tap (weights) per thread
-// row: data gradients 3.06 -> 0.40 ms, weight and bias gradients 6.9 -> 0.39
-// ms, the whole gradient call 13.0 -> 1.6 ms; a batch of 4 on 161 x 25 x 25
-// 21.6 -> 3.3 ms.  Error of the gradient against 64 bits (same stored
-// activations): 1.5e-7 -> 5.3e-8 relative at 65^3, 1.1e-7 -> 5.7e-8 on
+// row: the whole gradient call 13.0 -> 1.51 ms; a batch of 4 on 161 x 25 x 25
+// 21.6 -> 2.88 ms.  Error of the whole gradient against 64 bits (same stored
+// activations): 1.5e-7 -> 3.4e-8 relative at 65^3, 1.1e-7 -> 3.2e-8 on
 // 161 x 25 x 25.
 #include <cuda_bf16.h>
 
@@ -56,8 +69,9 @@ struct BwdParams {
 
 __device__ __forceinline__ unsigned pack2(unsigned a, unsigned b) { return (a >> 16) | (b & 0xffff0000u); }
 
-// g = hi + mid + lo exactly for every finite g (three truncations to BF16);
-// an infinity or NaN stays in hi.  Returned in the upper halves.
+// g = hi + mid + lo (three truncations to BF16): exact for |g| >= 2^-110, off by
+// less than 2^-133 below; an infinity or NaN stays in hi.  Returned in the upper
+// halves.
 __device__ __forceinline__ void split3(float g, unsigned& hi, unsigned& mid, unsigned& lo) {
   const unsigned u = __float_as_uint(g);
   if ((u & 0x7f800000u) == 0x7f800000u) {
@@ -118,6 +132,15 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], 
       "{%0, %1, %2, %3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// c += A B (16 x 8 x 8): the first (a0, a1, b0) or second (a2, a3, b1) half of the
+// terms of the fragments above
+__device__ __forceinline__ void mma1688(float (&c)[4], unsigned a0, unsigned a1, unsigned b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(b0));
 }
 
 __device__ __forceinline__ void brick_origin(const BwdParams& p, int b, int& x0, int& y0, int& z0) {
@@ -237,11 +260,16 @@ __global__ void __launch_bounds__(32 * kWgWarps, CI * CO < 512 ? 2 : 1) k_wgrad(
               ldsm4_t(aA + (unsigned)((row0 + s + toff[a]) * PI + 32 * m), af);
 #pragma unroll
               for (int n = 0; n < 2; n++) {
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
+                float v[4];
 #pragma unroll
-                for (int part = 2; part >= 0; part--) mma16816(c, af, bf[part][2 * n], bf[part][2 * n + 1]);
+                for (int part = 2; part >= 0; part--) {
+                  float c[4] = {0.f, 0.f, 0.f, 0.f};
+                  mma16816(c, af, bf[part][2 * n], bf[part][2 * n + 1]);
 #pragma unroll
-                for (int e = 0; e < 4; e++) acc[a][m][2 * n2 + n][e] += c[e];
+                  for (int e = 0; e < 4; e++) v[e] = part == 2 ? c[e] : v[e] + c[e];
+                }
+#pragma unroll
+                for (int e = 0; e < 4; e++) acc[a][m][2 * n2 + n][e] += v[e];
               }
             }
           }
@@ -394,19 +422,31 @@ __global__ void __launch_bounds__(kDgThreads, 2) k_dgrad(const __grid_constant__
         for (int kc = 0; kc < CO / 16; kc++) {
           unsigned bw[4];
           ldsm4(rb + 32 * kc, bw);
-          float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+          float v[2][4];
 #pragma unroll
           for (int part = 2; part >= 0; part--) {
             unsigned af[4];
             ldsm4(ra + 2 * part * CO + 32 * kc, af);
-            mma16816(c0, af, bw[0], bw[1]);
-            mma16816(c1, af, bw[2], bw[3]);
+#pragma unroll
+            for (int n = 0; n < 2; n++) {
+              float c[4] = {0.f, 0.f, 0.f, 0.f};
+              if (part == 0) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                mma1688(c, af[0], af[1], bw[2 * n]);
+                mma1688(d, af[2], af[3], bw[2 * n + 1]);
+#pragma unroll
+                for (int e = 0; e < 4; e++) c[e] += d[e];
+              } else {
+                mma16816(c, af, bw[2 * n], bw[2 * n + 1]);
+              }
+#pragma unroll
+              for (int e = 0; e < 4; e++) v[n][e] = part == 2 ? c[e] : v[n][e] + c[e];
+            }
           }
 #pragma unroll
-          for (int e = 0; e < 4; e++) {
-            acc[0][e] += c0[e];
-            acc[1][e] += c1[e];
-          }
+          for (int n = 0; n < 2; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[n][e] += v[n][e];
         }
       };
       if constexpr (STRIDE == 2) {
