@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(kW1Threads) k_wgrad_1(const __grid_constant__ 
   constexpr int HX = kOX + 2, HY = kOY + 2, HZ = kOZ + 2, SG = FIRST ? 1 : -1;
   __shared__ float s[HX * HY * HZ];
   __shared__ float4 qv[kOX * kOY * kOZ * 4];
-  __shared__ float red[kW1Threads * 12];
+  __shared__ __align__(16) float red[kW1Threads * 12];  // read and written as float4 too
   const int t = threadIdx.x, cq = t & 3, yz = (t >> 2) % 9, grp = t / 36;
   const int dy = SG * (yz % 3 - 1), dz = SG * (yz / 3 - 1);
   const int nx = p.vd[0], ny = p.vd[1], nz = p.vd[2];
