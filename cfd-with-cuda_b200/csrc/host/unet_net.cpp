@@ -248,7 +248,12 @@ cudaError_t UnetNet::prepare_tc(cudaStream_t s) {
 
 cudaError_t UnetNet::forward(cudaStream_t s, float* out_f32, const int* skip) {
   if (!out_f32) out_f32 = out;
+  // layers read their packed weights before they wait for the layer in front, so
+  // where the pass packs them itself, between the input kernel and the first
+  // layer, that layer starts after the packing has finished
+  bool early = pdl;
   if (tc_enabled) {
+    if (packs_dirty) early = false;
     cudaError_t e = prepare_tc(s);
     if (e != cudaSuccess) return e;
   }
@@ -256,17 +261,18 @@ cudaError_t UnetNet::forward(cudaStream_t s, float* out_f32, const int* skip) {
     cudaError_t e;
     if (op >= 0) {
       if (tc_enabled && plan_ok[op]) {
-        e = conv3_forward_tc(plans[op], out_f32, skip, tc_err, pdl, s);
+        e = conv3_forward_tc(plans[op], out_f32, skip, tc_err, early, s);
       } else
-        e = conv3_forward(conv_desc(*this, op, out_f32, skip), pdl, s);
+        e = conv3_forward(conv_desc(*this, op, out_f32, skip), early, s);
     } else {
       const UnetUpSpec& u = kUnetUp[-1 - op];
       const int lc = kUnetTensor[u.in].level, lf = kUnetTensor[u.out].level;
-      e = upsample_forward(dims[lc], dims[lf], kUnetTensor[u.out].ch, act[u.in], act[u.skip], act[u.out], skip, pdl,
+      e = upsample_forward(dims[lc], dims[lf], kUnetTensor[u.out].ch, act[u.in], act[u.skip], act[u.out], skip, early,
                            s);
     }
     launches++;
     if (e != cudaSuccess) return e;
+    early = pdl;
   }
   return cudaSuccess;
 }

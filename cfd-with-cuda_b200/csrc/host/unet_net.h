@@ -90,7 +90,8 @@ struct UnetNet {
   // The layers of a forward pass start before the layer in front has finished
   // (programmatic dependent launch; CFD_PDL=0 turns it off).  The input kernel,
   // before the first layer, is launched as usual, so whatever precedes the pass
-  // (packing of the weights, an Adam step) is complete by then.
+  // (an Adam step, packing before a capture) is complete by then; after a packing
+  // by the pass itself the first layer is launched as usual too.
   bool pdl = true;
   // tensor-core path: packed weights and launch plans of the stride-1 layers
   bool tc_enabled = true;
