@@ -5,8 +5,10 @@
 // as much as one of them.  New deck to first step on a graded 30^3 mesh (27
 // Gauss points): 63 ms with an allocation per buffer, 36 ms from the pool.
 //
-// The pool belongs to its context (single-threaded use) and gives everything
-// back when the context ends.  A range returned with put() is handed out again
+// The pool belongs to its context (single-threaded use).  Blocks that hold nothing go
+// back to the driver when a context loads another deck, and when the driver has
+// no room for a new block (otherwise a deck of 70 GB after one of 60 would not fit
+// 100 GB); everything goes back when the context ends.  A range returned with put() is handed out again
 // only after the context's streams have finished what was queued on them, as
 // cudaFree would have waited.  PoolScope makes a pool current for the calling
 // thread while an entry point runs; buffers allocated meanwhile come from it.
@@ -50,7 +52,7 @@ class DevPool {
     Block b;
     b.size = std::max(bytes, std::min(kMaxBlock, std::max(kMinBlock, total_)));
     cudaError_t e = cudaMalloc((void**)&b.base, b.size);
-    if (e == cudaErrorMemoryAllocation && b.size > bytes) {
+    if (e == cudaErrorMemoryAllocation && (trim() || b.size > bytes)) {
       cudaGetLastError();
       b.size = bytes;
       e = cudaMalloc((void**)&b.base, b.size);
@@ -63,6 +65,18 @@ class DevPool {
     blocks_.push_back(std::move(b));
     return cudaSuccess;
   }
+  // Gives the blocks that hold nothing back; whether there were any.
+  bool trim() {
+    const auto first = std::partition(blocks_.begin(), blocks_.end(), [](const Block& b) { return !b.used.empty(); });
+    const bool any = first != blocks_.end();
+    for (auto it = first; it != blocks_.end(); ++it) {
+      total_ -= it->size;
+      cudaFree(it->base);
+    }
+    blocks_.erase(first, blocks_.end());
+    return any;
+  }
+  size_t held() const { return total_; }
   void put(void* p) {
     if (s_[0]) {
       cudaStreamSynchronize(cudaStreamLegacy);  // plain cudaMemset and cudaMemcpy
