@@ -113,15 +113,13 @@ struct DevBuf {
 
 }  // namespace
 
-struct cfd_ctx {
-  DevPool pool;  // first member: outlives every buffer taken from it
-  int device = 0, num_sms = 148;
-  cudaStream_t stream = nullptr;
-  cfd_options opt{};
-  std::string err;
-  HostProblem P;
-  bool loaded = false, assembled = false;
+struct PoolOwner {
+  DevPool pool;  // in the first base: outlives every buffer taken from it
+};
 
+// What a context holds of the deck that is loaded; another load starts from a new
+// one (cfd_ctx::drop_deck).
+struct DeckState {
   // mesh
   DevBuf<int> ltog, bcnodes;
   DevBuf<int> elist;           // elements colour by colour (deterministic mode)
@@ -162,19 +160,13 @@ struct cfd_ctx {
   DevBuf<int> zd_off;
   DevBuf<double> zd_coef;
   int zd_ntap = 0, zd_reach = 0, dia_grid = 0, dia_cluster = 0, dia_apply = 0;
-  DiaArgs dia() const { return DiaArgs{(int)P.NNp, zd_ntap, zd_reach, zd_off.p, zd_coef.p}; }
   DevBuf<int> nb64, nb32;  // per PCG block: [lo..., hi...] neighbour block ranges
   DevBuf<int> cg_err;
   int pcg_grid64 = 1, pcg_grid32 = 1, res_blocks = 1;
   // reductions
   DevBuf<double> upart, ppart, norms, blk;
   int nub = 1, npb = 1;
-  double* h_small = nullptr;  // pinned scratch for small readbacks (64 doubles)
-
-  // learned preconditioner: attached network, its grid and flexible-CG state
-  cfd_unet* unet = nullptr;
-  std::unique_ptr<cfd_unet> unet_owned;
-  int udims[3] = {0, 0, 0};
+  // flexible-CG state and the coarse space of the two-level preconditioners
   DevBuf<int> upmap;  // voxel -> pressure node (empty: identity)
   DevBuf<double> fcg_sc, fcg_part, fcg_work64;
   DevBuf<float> fcg_work32;
@@ -184,10 +176,56 @@ struct cfd_ctx {
   DevBuf<float> cs_zp;
   DevBuf<int> cs_wlo;
   bool cs_zp_ok = false;
-  cudaStream_t stream2 = nullptr;  // the coarse solve beside the SpMV
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   DevBuf<unsigned> fcg_cnt;
   DevBuf<int> fcg_done, fcg_err;
+  // tensor-core convection: its bounded-wait error word
+  bool convect_tc_ran = false;
+  DevBuf<int> conv_err;
+  // persistent two-level iteration
+  int fcg2l_g = 0;                  // co-resident blocks of the launch
+  int fcg2l_key[3] = {0, 0, 0};     // n, blocks, reach of the neighbour ranges in fcg2l_nb
+  DevBuf<unsigned> fcg2l_sync;      // arrival counter + per-block progress
+  DevBuf<int> fcg2l_nb;             // [lo (blocks), hi (blocks)]
+  DevBuf<double> fcg2l_part, fcg2l_time;  // time: 7 phases of block 0, then one SpMV total per block
+  DevBuf<float> fcg2l_e;                   // coarse solution in pieces
+  std::vector<int> h_zfirst, h_zlast;  // first / last column of each row of Z
+  bool coarse_ready = false;
+  int cs_fd[3] = {0, 0, 0}, cs_cd[3] = {0, 0, 0}, cs_nc = 0;
+  DevBuf<int> cs_i0[3], cs_r[3];
+  DevBuf<double> cs_f[3], cs_e64;
+  DevBuf<float> cs_c32, cs_e32;  // coarse right-hand side (both precisions), FP32 coarse solution
+  DevBuf<__half> cs_inv16;
+  DevBuf<float> zst32;  // Z in structured (125-tap) form for the FP32 inner solves, when it applies
+  bool zst_ok = false;
+  int cs_ld = 0;
+  double cs_scale = 1.0;
+};
+
+struct cfd_ctx : PoolOwner, DeckState {
+  DiaArgs dia() const { return DiaArgs{(int)P.NNp, zd_ntap, zd_reach, zd_off.p, zd_coef.p}; }
+  // Everything of the deck goes, and its memory goes back to the device.
+  void drop_deck() {
+    loaded = assembled = false;
+    reset_fcg_graphs();
+    DeckState* d = this;
+    d->~DeckState();
+    new (d) DeckState();
+    pool.trim();
+  }
+  int device = 0, num_sms = 148;
+  cudaStream_t stream = nullptr;
+  cfd_options opt{};
+  std::string err;
+  HostProblem P;
+  bool loaded = false, assembled = false;
+  double* h_small = nullptr;  // pinned scratch for small readbacks (64 doubles)
+
+  // learned preconditioner: attached network, its grid and flexible-CG state
+  cfd_unet* unet = nullptr;
+  std::unique_ptr<cfd_unet> unet_owned;
+  int udims[3] = {0, 0, 0};
+  cudaStream_t stream2 = nullptr;  // the coarse solve beside the SpMV
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int fcg_window = 25;
   bool fcg_use_graph = true;
   // CFD_FCG_SPLIT=1: the split FP32 iteration (coarse solve on a second
@@ -195,10 +233,8 @@ struct cfd_ctx {
   // 64^3 cavity (8.97 against 8.13 ms per step), so off by default
   bool fcg_split = false;
   // mixed-precision convection on the tensor cores (k_convect_tc) where it
-  // applies; conv_err is its bounded-wait error word
+  // applies
   bool convect_tc = false;
-  bool convect_tc_ran = false;
-  DevBuf<int> conv_err;
   // CFD_FCG_ANCHOR=0: with the network in the head iterations only, keep the
   // ring of the last fcg_m directions instead of anchoring the head's
   bool fcg_anchor = true;
@@ -238,12 +274,6 @@ struct cfd_ctx {
   bool l2_persist = false, l2_window = false;
   // CFD_COARSE_SPACING=<s>: coarse-lattice spacing in voxels (default 4)
   double coarse_spacing = 4.0;
-  int fcg2l_g = 0;                  // co-resident blocks of the launch
-  int fcg2l_key[3] = {0, 0, 0};     // n, blocks, reach of the neighbour ranges in fcg2l_nb
-  DevBuf<unsigned> fcg2l_sync;      // arrival counter + per-block progress
-  DevBuf<int> fcg2l_nb;             // [lo (blocks), hi (blocks)]
-  DevBuf<double> fcg2l_part, fcg2l_time;  // time: 7 phases of block 0, then one SpMV total per block
-  DevBuf<float> fcg2l_e;                   // coarse solution in pieces
   double unet_dscale = 1.0;  // median diagonal of Z (scale of the network's targets)
   double fcg_stall = 0.5;  // minimum residual reduction per window
 
@@ -251,15 +281,7 @@ struct cfd_ctx {
   // the two-level preconditioners
   bool grid_set = false;
   std::vector<int> h_pmap;  // voxel -> pressure node (empty: identity)
-  std::vector<int> h_zfirst, h_zlast;  // first / last column of each row of Z
-  bool coarse_ready = false;
   int coarse_gen = 0;  // bumped on every rebuild (captured graphs key on it)
-  int cs_fd[3] = {0, 0, 0}, cs_cd[3] = {0, 0, 0}, cs_nc = 0;
-  DevBuf<int> cs_i0[3], cs_r[3];
-  DevBuf<double> cs_f[3], cs_e64;
-  DevBuf<float> cs_c32, cs_e32;  // coarse right-hand side (both precisions), FP32 coarse solution
-  DevBuf<__half> cs_inv16;
-
   // blocks of the flexible-CG update kernel, four entries per thread:
   // 4 per SM by default (fewer partial sums for the last block to add than
   // one thread per entry; 131.5 against 127.9 steps/s on the 64^3 two-level
@@ -268,10 +290,6 @@ struct cfd_ctx {
   // CFD_HOST_PATTERNS=1: the CSR patterns are built on the host (the
   // fallback of the device build)
   bool host_patterns = false;
-  DevBuf<float> zst32;  // Z in structured (125-tap) form for the FP32 inner solves, when it applies
-  bool zst_ok = false;
-  int cs_ld = 0;
-  double cs_scale = 1.0;
   double coarse_setup_s = 0;
 
   int timeN = 0;
@@ -582,6 +600,15 @@ int find_diagonals(cfd_ctx* c);
 int upload_problem(cfd_ctx* c) {
   HostProblem& P = c->P;
   cudaStream_t s = c->stream;
+  c->drop_deck();
+  // a declared grid and a network belong to a number of pressure nodes
+  if (c->grid_set && (long long)c->udims[0] * c->udims[1] * c->udims[2] != P.NNp) {
+    c->grid_set = false;
+    c->h_pmap.clear();
+    for (int& d : c->udims) d = 0;
+    c->unet = nullptr;
+    c->unet_owned.reset();
+  }
   if (c->opt.ngp_override) P.NGP = c->opt.ngp_override;
   Basis hb;
   if (make_basis(P.NGP, hb)) return fail(c, CFD_E_BADINPUT, "unsupported NGP %d", P.NGP);
@@ -720,6 +747,7 @@ int upload_problem(cfd_ctx* c) {
   CU(c->blk.alloc(3 * NN));
   // initial condition: Un = BC values at Dirichlet nodes, zero elsewhere
   CU(launch_apply_bc((int)P.bcnode.size(), c->bcnodes.p, c->bcvals.p, c->un, s));
+  if (!c->h_pmap.empty()) CU(upload(c->upmap, c->h_pmap, s));
   CU(cudaStreamSynchronize(s));
   c->timeN = 0;
   c->timeT = P.t_ini;
@@ -1672,6 +1700,7 @@ int pressure_solve(cfd_ctx* c, const double* b, double* x, int warm, cfd_solve_s
 }
 
 int reduce_norms(cfd_ctx* c) {
+  NEED(c->loaded, "no deck is loaded");
   cudaStream_t s = c->stream;
   KL(CFD_K_OTHER, launch_reduce_norms(c->upart.p, c->nub, c->ppart.p, c->npb, c->norms.p, s));
   CU(cudaMemcpyAsync(c->h_small, c->norms.p, 5 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1826,6 +1855,7 @@ int cfd_load_inp(cfd_ctx* c, const char* path) {
   PoolScope scope(&c->pool);
   int rc = set_device(c);
   if (rc) return rc;
+  c->loaded = c->assembled = false;
   c->P = HostProblem();
   rc = read_inp(path, c->P, c->err);
   if (rc) return rc;
@@ -1842,6 +1872,7 @@ int cfd_load_mesh(cfd_ctx* c, const cfd_problem_info* info, const double* coords
   int rc = set_device(c);
   if (rc) return rc;
   HostProblem& P = c->P;
+  c->loaded = c->assembled = false;
   P = HostProblem();
   P.NE = info->NE; P.NCN = info->NCN; P.NGP = info->NGP; P.maxIter = info->maxIter;
   P.dt = info->dt; P.t_ini = info->t_ini; P.t_final = info->t_final; P.tolerance = info->tolerance;

@@ -127,7 +127,11 @@ int cfd_set_options(cfd_ctx* ctx, const cfd_options* opt);
  * DOF maps, velocity-BC nodes, monitor node, CSR patterns), the basis set-up
  * of blascoCodinaHuerta.cpp:2166-2488, the initial condition of
  * applyBC_initial (blascoCodinaHuerta.cpp:4062-4110) and the device upload of
- * initializeAndAllocateGPU (CUDAcodes.cu:161-274). */
+ * initializeAndAllocateGPU (CUDAcodes.cu:161-274).
+ * A context may load one deck after another.  The device memory of the deck
+ * before is given back first.  A declared pressure grid and an attached
+ * network stay when the number of pressure nodes is the same and are dropped
+ * otherwise.  After a load that fails, nothing is loaded. */
 int cfd_load_inp(cfd_ctx* ctx, const char* path);
 
 /* Same as cfd_load_inp from in-memory deck data (0-based ids):
