@@ -181,6 +181,10 @@ struct DeckState {
   // tensor-core convection: its bounded-wait error word
   bool convect_tc_ran = false;
   DevBuf<int> conv_err;
+  // ln of the mean residual reduction per iteration in the last solve from x0
+  // = 0 of each kind [FP32, FP64][first solve, refinement, network] (0: none
+  // yet): how many iterations to queue before the first look at a solve
+  double fcg_lnrate[2][3] = {};
   // persistent two-level iteration
   int fcg2l_g = 0;                  // co-resident blocks of the launch
   int fcg2l_key[3] = {0, 0, 0};     // n, blocks, reach of the neighbour ranges in fcg2l_nb
@@ -253,10 +257,6 @@ struct cfd_ctx : PoolOwner, DeckState {
         for (auto& gr : gq)
           for (auto& g : gr) g.reset();
   }
-  // ln of the mean residual reduction per iteration in the last solve from x0
-  // = 0 of each kind [FP32, FP64][first solve, refinement, network] (0: none
-  // yet): how many iterations to queue before the first look at a solve
-  double fcg_lnrate[2][3] = {};
   // CFD_FCG_PERSIST=1: the persistent two-level iteration (fcg_persist.cu)
   // for the FP32 inner solves on a structured grid instead of the per-kernel
   // iteration graphs; measured slower on the 64^3 cavity (about 85 against
@@ -1513,7 +1513,7 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
   // a solve from x0 = 0 is expected to take as many iterations as the last of
   // its kind, scaled to its target
   double& lnrate = c->fcg_lnrate[sizeof(VT) == 4 ? 0 : 1][use_net ? 2 : first_solve ? 0 : 1];
-  if (!warm && lnrate < 0) batch = (int)std::lround(std::log(rtol) / lnrate + 0.2) - issued;
+  if (!warm && lnrate < 0) batch = (int)std::lround(std::min(64.0, std::log(rtol) / lnrate + 0.2)) - issued;
   while (!persist) {
     batch = std::max(1, std::min({batch, 64, std::max(1, maxit - issued)}));
     if (G && G1) {
@@ -1841,6 +1841,9 @@ int cfd_set_options(cfd_ctx* c, const cfd_options* o) {
        "ngp_override must be 0, 1, 8 or 27");
   NEED(!c->loaded || o->precision == c->opt.precision, "precision must be set before cfd_load_inp");
   NEED(!c->loaded || o->ngp_override == c->opt.ngp_override, "ngp_override must be set before cfd_load_inp");
+  // another iteration: what the last solves took says nothing about it
+  if (o->precond != c->opt.precond || o->fcg_m != c->opt.fcg_m || o->fcg_net_iters != c->opt.fcg_net_iters)
+    std::memset(c->fcg_lnrate, 0, sizeof(c->fcg_lnrate));
   c->opt = *o;
   if (c->opt.inner_rtol <= 0 || c->opt.inner_rtol >= 1) c->opt.inner_rtol = 1e-4;
   if (c->opt.max_outer <= 0) c->opt.max_outer = 12;
