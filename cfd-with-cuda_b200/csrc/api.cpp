@@ -135,6 +135,10 @@ struct DeckState {
   // (CFD_MIXED) FP32 values
   DevBuf<int> ks_off, ks_col, gs_off, gs_col, gts_off, gts_col, zs_off, zs_col;
   DevBuf<double> ks_val, gs1, gs2, gs3, gts1, gts2, gts3, zs_val;
+  // the FP64 values of Z in this form: allocated and filled where something reads them
+  // (ensure_sell_z), which the form by offsets below mostly makes needless
+  bool zs_filled = false;
+  size_t zs_entries = 0;
   DevBuf<float> ks_val32, gs1_32, gs2_32, gs3_32, gts1_32, gts2_32, gts3_32, zs_val32, zdinv32;
   // velocity-sized state, double4 per node
   DevBuf<double4> vbuf[12];
@@ -287,6 +291,8 @@ struct cfd_ctx : PoolOwner, DeckState {
   // one thread per entry; 131.5 against 127.9 steps/s on the 64^3 two-level
   // line); CFD_FCG_UPDATE_BLOCKS overrides it, 0 = one thread per entry
   int upd_grid = -1;
+  // CFD_DIA=0: the pressure operator is not kept by offsets
+  bool use_dia = true;
   // CFD_HOST_PATTERNS=1: the CSR patterns are built on the host (the
   // fallback of the device build)
   bool host_patterns = false;
@@ -596,6 +602,7 @@ int klaunch(cfd_ctx* c, int cls, F&& f) {
 // initial condition (initializeAndAllocateGPU, CUDAcodes.cu:161-274, and
 // applyBC_initial, blascoCodinaHuerta.cpp:4062-4110).
 int find_diagonals(cfd_ctx* c);
+int ensure_sell_z(cfd_ctx* c);
 
 int upload_problem(cfd_ctx* c) {
   HostProblem& P = c->P;
@@ -682,7 +689,7 @@ int upload_problem(cfd_ctx* c) {
   CU(c->ks_val.alloc(sK));
   for (auto* b : {&c->gs1, &c->gs2, &c->gs3}) CU(b->alloc(sG));
   for (auto* b : {&c->gts1, &c->gts2, &c->gts3}) CU(b->alloc(sGt));
-  CU(c->zs_val.alloc(sZ));
+  c->zs_entries = sZ;
   if (c->opt.precision == CFD_MIXED) {
     CU(c->ks_val32.alloc(sK));
     for (auto* b : {&c->gs1_32, &c->gs2_32, &c->gs3_32}) CU(b->alloc(sG));
@@ -721,6 +728,7 @@ int upload_problem(cfd_ctx* c) {
   {
     int rc = find_diagonals(c);
     if (rc) return rc;
+    if (c->dia_grid == 0) CU(c->zs_val.alloc(c->zs_entries));  // the Jacobi solves read it
   }
   const int gmax = std::max({c->pcg_grid64, c->pcg_grid32, c->dia_grid});
   CU(c->cg_part.alloc(8 * (size_t)gmax));
@@ -759,12 +767,11 @@ int upload_problem(cfd_ctx* c) {
 // The diagonals of Z's pattern (column - row), kept when they are few enough
 // for the stored-by-offsets form: at most kDiaMaxTaps of them and at most 1.2
 // times the bytes of value and column (small matrices, which the latency of an
-// iteration bounds and not its bytes, at any fill).
+// iteration bounds and not its bytes, at any fill).  Without memory for it, or with
+// CFD_DIA=0, the SELL-32 form does its work.
 int find_diagonals(cfd_ctx* c) {
   const int n = (int)c->P.NNp;
-  c->zd_ntap = c->dia_grid = c->dia_cluster = c->dia_apply = 0;
-  c->zd_off.reset();
-  c->zd_coef.reset();
+  if (!c->use_dia) return CFD_OK;
   const int apply = dia_apply_grid(n, c->num_sms);
   if (apply == 0) return CFD_OK;
   DevBuf<unsigned char> mark;
@@ -780,14 +787,28 @@ int find_diagonals(cfd_ctx* c) {
   const int ntap = (int)off.size();
   if (ntap < 1 || ntap > kDiaMaxTaps) return CFD_OK;
   if (n > 4096 && 8.0 * ntap * n > 1.2 * 12.0 * (double)c->P.nnzZ) return CFD_OK;
+  const cudaError_t e = c->zd_coef.alloc(dia_elems(n, ntap));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return CFD_OK;
+  }
+  CU(e);
   CU(upload(c->zd_off, off, c->stream));
-  CU(c->zd_coef.alloc(dia_elems(n, ntap)));
   CU(cudaStreamSynchronize(c->stream));
   c->zd_ntap = ntap;
   c->zd_reach = std::max(-off.front(), off.back());
   c->dia_grid = pcg_dia_grid(n, c->device);
   c->dia_cluster = c->dia_grid > 0 ? pcg_cluster_blocks(n, c->zd_ntap) : 0;
   c->dia_apply = apply;
+  return CFD_OK;
+}
+
+// The FP64 values of Z in the SELL-32 form, for what reads them.
+int ensure_sell_z(cfd_ctx* c) {
+  if (c->zs_filled) return CFD_OK;
+  if (!c->zs_val.p) CU(c->zs_val.alloc(c->zs_entries));
+  CU(launch_csr_to_sell<double>(c->P.NNp, c->z_rp.p, c->zval.p, c->zs_off.p, c->zs_val.p, c->stream));
+  c->zs_filled = true;
   return CFD_OK;
 }
 
@@ -808,6 +829,7 @@ int run_pcg64(cfd_ctx* c, const double* b, double* x, int warm, double rtol, int
     a.timeout_ns = 2000000000ULL;
     KL(CFD_K_PCG64, launch_pcg_dia(a, c->dia_grid, c->dia_cluster, s));
   } else {
+    if (int rc = ensure_sell_z(c)) return rc;
     PcgArgs<double> a{};
     a.n = c->P.NNp;
     a.off = c->zs_off.p; a.col = c->zs_col.p; a.val = c->zs_val.p; a.dinv = c->zdinv.p;
@@ -1285,8 +1307,10 @@ int run_fcg(cfd_ctx* c, const VT* b, VT* x, int warm, double rtol, int maxit, do
     if (!c->fcg_work32.p) CU(c->fcg_work32.alloc(nwork));
     work = c->fcg_work32.p;
   } else {
-    a.val = c->zs_val.p;
     if (c->dia_apply > 0) a.dia = c->dia();
+    if (c->dia_apply == 0 || warm)  // the start kernel's residual reads the SELL-32 form
+      if (int rc = ensure_sell_z(c)) return rc;
+    a.val = c->zs_val.p;
     a.dia_grid = c->dia_apply;
     if (!c->fcg_work64.p) CU(c->fcg_work64.alloc(nwork));
     work = c->fcg_work64.p;
@@ -1572,6 +1596,8 @@ int queue_residual(cfd_ctx* c, const double* b, const double* x, double* out, co
     KL(CFD_K_RESID64,
        launch_residual_dia(c->dia(), b, x, c->ir_r.p, c->f_b.p, c->ir_part.p, c->res_blocks, when, s));
   } else {
+    if (x)
+      if (int rc = ensure_sell_z(c)) return rc;
     KL(CFD_K_RESID64, launch_residual64(c->P.NNp, c->zs_off.p, c->zs_col.p, c->zs_val.p, b, x, c->ir_r.p, c->f_b.p,
                                         c->ir_part.p, c->res_blocks, when, s));
   }
@@ -1790,6 +1816,7 @@ int cfd_create(cfd_ctx** out, int device) {
   if (const char* e = std::getenv("CFD_FCG_PERSIST")) c->fcg_persist = std::atoi(e) != 0;
   if (const char* e = std::getenv("CFD_COARSE_HOST")) c->coarse_on_host = std::atoi(e) != 0;
   if (const char* e = std::getenv("CFD_PDL")) c->pdl = std::atoi(e) != 0;
+  if (const char* e = std::getenv("CFD_DIA")) c->use_dia = std::atoi(e) != 0;
   if (const char* e = std::getenv("CFD_FCG_UPDATE_BLOCKS")) c->upd_grid = std::max(0, std::atoi(e));
   if (const char* e = std::getenv("CFD_HOST_PATTERNS")) c->host_patterns = std::atoi(e) != 0;
   if (const char* e = std::getenv("CFD_L2_PERSIST")) c->l2_persist = std::atoi(e) != 0;
@@ -1971,7 +1998,9 @@ int cfd_step0(cfd_ctx* c) {
   CU(launch_csr_to_sell<double>(P.NNp, c->gt_rp.p, c->gt1.p, c->gts_off.p, c->gts1.p, s));
   CU(launch_csr_to_sell<double>(P.NNp, c->gt_rp.p, c->gt2.p, c->gts_off.p, c->gts2.p, s));
   CU(launch_csr_to_sell<double>(P.NNp, c->gt_rp.p, c->gt3.p, c->gts_off.p, c->gts3.p, s));
-  CU(launch_csr_to_sell<double>(P.NNp, c->z_rp.p, c->zval.p, c->zs_off.p, c->zs_val.p, s));
+  c->zs_filled = false;
+  if (c->dia_grid == 0)
+    if ((rc = ensure_sell_z(c))) return rc;
   if (mixed(c)) {
     CU(launch_csr_to_sell<float>(P.NN, c->k_rp.p, c->kval.p, c->ks_off.p, c->ks_val32.p, s));
     CU(launch_csr_to_sell<float>(P.NN, c->g_rp.p, c->g1.p, c->gs_off.p, c->gs1_32.p, s));
