@@ -380,7 +380,8 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(PcgDiaArgs a, int
   post(v, 0);
   cluster_barrier();
 
-  double bnorm = 0, tol = 0, igam = 0, ialpha = 0;  // the scalars' warp
+  // the scalars' warp; the reciprocals are formed off the critical path
+  double bnorm = 0, tol = 0, gam_old = 1, igam = 0, ialpha = 0;
   int its = 0;
   for (int i = 0;; i++) {
     if (warp == kDiaWarps) {
@@ -398,7 +399,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(PcgDiaArgs a, int
         st = 0;
       else if (i >= a.maxit)
         st = 1;
-      const double beta = gam * igam, alpha = gam / (del - beta * gam * ialpha);  // i = 0: igam = 0
+      // i = 0: igam = 0; the reciprocal of a gam near the smallest numbers overflows
+      const double beta = gam_old > 1e-290 ? gam * igam : gam / gam_old;
+      const double alpha = gam / (del - beta * gam * ialpha);
       if (lane == 0) {
         sred[0] = alpha;
         sred[1] = beta;
@@ -406,6 +409,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(PcgDiaArgs a, int
         sred[3] = bnorm;
         sstat = st;
       }
+      gam_old = gam;
       igam = 1.0 / gam;
       ialpha = 1.0 / alpha;
     } else {
