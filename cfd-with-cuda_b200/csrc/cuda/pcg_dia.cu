@@ -21,7 +21,7 @@
 //   sixteenth of the loads in flight is worth more (the first form below / after /
 //   beside: 40^3, 14.5 slices, 14.5 / - / 15.2, 48^3 20.3 / 19.6 / 19.1 to 19.6, 64^3
 //   41.0 / 40.0 / 44.1 on one device).  The other warps wait only for
-//   the blocks whose rows they gather.  Every wait is bounded.
+//   the blocks whose rows they gather.  Every wait of this form is bounded.
 //
 // What bounds it: the coefficient stream on large grids; the latency of the
 // wait for the neighbours, the gathers and the block sums on small ones.  Measured
@@ -214,7 +214,9 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
 // m it gathers (double buffered) in shared memory: a block writes its rows of m
 // straight into the copies of the blocks that gather them, and its partial sums
 // into every block, and one hardware cluster barrier per iteration covers both.
-// No flag, no poll, no trip to L2.  A seventeenth warp adds the partials (in the
+// No flag, no poll, no trip to L2.  That barrier has no time limit: the blocks of a
+// cluster are on the chip together, each arrives at every barrier (all take the same
+// decisions, from the same sums in the same order), and the iterations are limited.  A seventeenth warp adds the partials (in the
 // same order in every block, so all take the same decisions) and forms alpha and
 // beta beside the product.  Bound by latency: the product's chain, the row sums,
 // the block's sums and the barrier.  us per iteration, launch included, on cavities of
