@@ -745,7 +745,7 @@ int upload_problem(cfd_ctx* c) {
   c->res_blocks = residual_blocks((int)NNp, c->num_sms);
   CU(c->ir_part.alloc(c->res_blocks));
   CU(c->ir_sum.alloc(2));
-  c->nub = mixed(c) ? step3_blocks<float>((int)NN) : step3_blocks<double>((int)NN);
+  c->nub = mixed(c) ? step3_blocks<float>((int)NN, c->num_sms) : step3_blocks<double>((int)NN, c->num_sms);
   c->npb = pupdate_blocks((int)NNp, c->num_sms);
   CU(c->upart.alloc(3 * (size_t)c->nub));
   CU(c->ppart.alloc(2 * (size_t)c->npb));
@@ -777,7 +777,7 @@ int find_diagonals(cfd_ctx* c) {
   DevBuf<unsigned char> mark;
   CU(mark.alloc(2 * (size_t)n));
   CU(cudaMemsetAsync(mark.p, 0, mark.bytes(), c->stream));
-  CU(launch_dia_mark(n, c->z_rp.p, c->z_col.p, mark.p, c->stream));
+  CU(launch_dia_mark(n, c->z_rp.p, c->z_col.p, mark.p, c->num_sms, c->stream));
   std::vector<unsigned char> h(2 * (size_t)n - 1);
   CU(cudaMemcpyAsync(h.data(), mark.p, h.size(), cudaMemcpyDeviceToHost, c->stream));
   CU(cudaStreamSynchronize(c->stream));
@@ -1194,6 +1194,7 @@ CoarseArgs<VT> coarse_args(const cfd_ctx* c, bool with_coarse) {
     a.fd[k] = c->udims[k];
     a.cd[k] = c->cs_cd[k];
   }
+  a.num_sms = c->num_sms;
   a.nc = c->cs_nc;
   a.ldinv = c->cs_ld;
   a.inv_scale = c->cs_scale;
@@ -1989,7 +1990,7 @@ int cfd_step0(cfd_ctx* c) {
   z.minv_orig = c->minv_orig.p;
   CU(launch_build_z(z, s));
   CU(launch_recip(P.NNp, c->zdiag.p, c->zdinv.p, mixed(c) ? c->zdinv32.p : nullptr, s));
-  if (c->zd_ntap > 0) CU(launch_dia_fill(c->dia(), c->z_rp.p, c->z_col.p, c->zval.p, c->zd_coef.p, s));
+  if (c->zd_ntap > 0) CU(launch_dia_fill(c->dia(), c->z_rp.p, c->z_col.p, c->zval.p, c->zd_coef.p, c->num_sms, s));
   // SELL-32 copies of the assembled operators (FP64, and FP32 in CFD_MIXED)
   CU(launch_csr_to_sell<double>(P.NN, c->k_rp.p, c->kval.p, c->ks_off.p, c->ks_val.p, s));
   CU(launch_csr_to_sell<double>(P.NN, c->g_rp.p, c->g1.p, c->gs_off.p, c->gs1.p, s));
@@ -2123,12 +2124,12 @@ int cfd_step3(cfd_ctx* c, int iter) {
     fill(a);
     a.acc_g = c->acc32;
     a.g1 = c->gs1_32.p; a.g2 = c->gs2_32.p; a.g3 = c->gs3_32.p;
-    KL(CFD_K_STEP3, launch_step3<float>(a, s));
+    KL(CFD_K_STEP3, launch_step3<float>(a, c->num_sms, s));
   } else {
     Step3Args<double> a{};
     fill(a);
     a.g1 = c->gs1.p; a.g2 = c->gs2.p; a.g3 = c->gs3.p;
-    KL(CFD_K_STEP3, launch_step3<double>(a, s));
+    KL(CFD_K_STEP3, launch_step3<double>(a, c->num_sms, s));
   }
   c->rotated = false;
   return CFD_OK;

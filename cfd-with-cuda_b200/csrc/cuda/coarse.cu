@@ -214,7 +214,7 @@ cudaError_t launch_coarse_restrict(const CoarseArgs<VT>& a, const VT* r, float* 
   // fine ranges of neighbours overlap by a support); 49 pairs of the 24 x 24 x 160
   // duct: 10.3 us in one range, 5.3 in five (each launched alone)
   const int pairs = a.cd[1] * a.cd[2];
-  const int nxs = std::max(1, std::min((2 * 148 + pairs - 1) / pairs, a.cd[0] / 8));
+  const int nxs = std::max(1, std::min((2 * a.num_sms + pairs - 1) / pairs, a.cd[0] / 8));
   const size_t sm = (size_t)std::max(kRestrictThreads, a.fd[0]) * sizeof(double);
   return launch_k(a.pdl != 0, k_restrict<VT>, dim3(pairs, nxs), dim3(kRestrictThreads), sm, s, a, r, c, done);
 }

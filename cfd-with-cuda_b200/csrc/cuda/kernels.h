@@ -154,9 +154,9 @@ struct Step3Args {
   GVec<VT>* acc_g;  // float4 copy of Acc (VT = float)
 };
 template <class VT>
-cudaError_t launch_step3(const Step3Args<VT>& a, cudaStream_t s);
+cudaError_t launch_step3(const Step3Args<VT>& a, int num_sms, cudaStream_t s);
 template <class VT>
-int step3_blocks(int NN);  // blocks of launch_step3 (its partial sums)
+int step3_blocks(int NN, int num_sms);  // blocks of launch_step3 (its partial sums)
 
 template <class VT>
 struct SpmvK3Args {
@@ -193,10 +193,10 @@ struct DiaArgs {
 inline size_t dia_elems(int n, int ntap) { return (size_t)((n + 31) / 32) * ntap * 32; }
 // mark[col - row + n - 1] = 1 for every entry (mark: 2 n - 1 bytes, zeroed by
 // the caller)
-cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, cudaStream_t s);
+cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, int num_sms, cudaStream_t s);
 // Fills coef (zeroed first) from the CSR values.
 cudaError_t launch_dia_fill(const DiaArgs& d, const int* rp, const int* col, const double* val, double* coef,
-                            cudaStream_t s);
+                            int num_sms, cudaStream_t s);
 // The pipelined Jacobi-PCG of pcg.cu on a matrix by offsets, FP64, with the
 // vectors in shared memory.  mb: 2 n work entries; part: 8 x blocks; sync: 1 +
 // blocks words, host-zeroed; result as in PcgArgs.  grid = 0 when n exceeds
@@ -323,6 +323,7 @@ template <class VT> struct CoarseArgs {
   const __half* inv16;
   double inv_scale;
   int pdl;  // 1: the coarse kernels launch with programmatic dependent launch
+  int num_sms;
 };
 // c = P^T r (FP32 coarse vector), e = Zc^-1 c
 template <class VT>

@@ -552,16 +552,16 @@ cudaError_t launch_pcg_dia(const PcgDiaArgs& a, int grid, int cluster, cudaStrea
 
 int dia_apply_grid(int n, int num_sms) { return dia_blocks(n, num_sms); }
 
-cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, cudaStream_t s) {
-  k_dia_mark<<<std::max(1, std::min((n + 255) / 256, 148 * 8)), 256, 0, s>>>(n, rp, col, mark);
+cudaError_t launch_dia_mark(int n, const int* rp, const int* col, unsigned char* mark, int num_sms, cudaStream_t s) {
+  k_dia_mark<<<std::max(1, std::min((n + 255) / 256, 8 * num_sms)), 256, 0, s>>>(n, rp, col, mark);
   return cudaGetLastError();
 }
 
 cudaError_t launch_dia_fill(const DiaArgs& d, const int* rp, const int* col, const double* val, double* coef,
-                            cudaStream_t s) {
+                            int num_sms, cudaStream_t s) {
   cudaError_t e = cudaMemsetAsync(coef, 0, dia_elems(d.n, d.ntap) * sizeof(double), s);
   if (e != cudaSuccess) return e;
-  k_dia_fill<<<std::max(1, std::min((d.n + 127) / 128, 148 * 16)), 128, 0, s>>>(d, rp, col, val, coef);
+  k_dia_fill<<<std::max(1, std::min((d.n + 127) / 128, 16 * num_sms)), 128, 0, s>>>(d, rp, col, val, coef);
   return cudaGetLastError();
 }
 

@@ -35,7 +35,7 @@ inline int rows_grid(long long rows) {
   return (int)(g < 1 ? 1 : g);
 }
 
-// Warps per slice: the largest of 1, 2, 4, 8 with at most `warps` warps over
+// Warps per slice: the largest of 1, 2, 4, 8 with at most the rule's warps per SM over
 // all slices.  Splitting pays while the chip is short of warps (a wave is 148
 // x 64) or a few long rows are its tail; it costs where the epilogue, which
 // one warp of the SPLIT runs, weighs as much as the row, and in FP32 where the
@@ -60,14 +60,13 @@ inline int rows_grid(long long rows) {
 // and k_gt in FP64 at n = 64 193 / 188 / 191 / 187, in FP32 on the duct of 24
 // x 24 x 160 (3145 slices) 78 / 63 / 63 / 53.
 struct SplitRule {
-  long long fp64, fp32;  // warps
+  int fp64, fp32;  // warps per SM
   int least32;           // least FP32 split that pays (below it: 1)
 };
-constexpr SplitRule kStep1Rule{148 * 128, 148 * 32, 2}, kSpmvK3Rule{148 * 256, 148 * 100, 2},
-    kStep3Rule{148 * 128, 148 * 50, 2}, kGtRule{148 * 512, 148 * 192, 8};
+constexpr SplitRule kStep1Rule{128, 32, 2}, kSpmvK3Rule{256, 100, 2}, kStep3Rule{128, 50, 2}, kGtRule{512, 192, 8};
 template <class VT>
-inline int row_split(long long rows, const SplitRule& rule) {
-  const long long ns = (rows + 31) / 32, warps = sizeof(VT) == 8 ? rule.fp64 : rule.fp32;
+inline int row_split(long long rows, const SplitRule& rule, int num_sms) {
+  const long long ns = (rows + 31) / 32, warps = (long long)num_sms * (sizeof(VT) == 8 ? rule.fp64 : rule.fp32);
   int sp = 1;
   while (sp < 8 && 2 * sp * ns <= warps) sp *= 2;
   return sizeof(VT) == 4 && sp < rule.least32 ? 1 : sp;
@@ -577,7 +576,7 @@ inline int ew_grid(long long n) {
 // Launches kernel<VT, SPLIT, ...> with the SPLIT of the row count.
 #define SPLIT_LAUNCH(kernel, rows, rule, ...)                                                              \
   do {                                                                                                     \
-    const int sp_ = row_split<VT>(rows, rule), g_ = split_grid(rows, sp_);                                 \
+    const int sp_ = row_split<VT>(rows, rule, num_sms), g_ = split_grid(rows, sp_);                        \
     switch (sp_) {                                                                                         \
       case 1: kernel<VT, 1 __VA_OPT__(, ) __VA_ARGS__><<<g_, kRowThreads, 0, s>>>(a); break;               \
       case 2: kernel<VT, 2 __VA_OPT__(, ) __VA_ARGS__><<<g_, block_threads(2), 0, s>>>(a); break;          \
@@ -588,28 +587,28 @@ inline int ew_grid(long long n) {
   } while (0)
 
 template <class VT>
-cudaError_t launch_step1(const Step1Args<VT>& a, int, cudaStream_t s) {
+cudaError_t launch_step1(const Step1Args<VT>& a, int num_sms, cudaStream_t s) {
   if (a.accprev) SPLIT_LAUNCH(k_step1, a.NN, kStep1Rule, true);
   SPLIT_LAUNCH(k_step1, a.NN, kStep1Rule, false);
 }
 template <class VT>
-cudaError_t launch_gt(const GtArgs<VT>& a, int, cudaStream_t s) {
+cudaError_t launch_gt(const GtArgs<VT>& a, int num_sms, cudaStream_t s) {
   SPLIT_LAUNCH(k_gt, a.NNp, kGtRule);
 }
 template <class VT>
-cudaError_t launch_step3(const Step3Args<VT>& a, cudaStream_t s) {
+cudaError_t launch_step3(const Step3Args<VT>& a, int num_sms, cudaStream_t s) {
   SPLIT_LAUNCH(k_step3, a.NN, kStep3Rule);
 }
 template <class VT>
-cudaError_t launch_spmv_k3(const SpmvK3Args<VT>& a, int, cudaStream_t s) {
+cudaError_t launch_spmv_k3(const SpmvK3Args<VT>& a, int num_sms, cudaStream_t s) {
   SPLIT_LAUNCH(k_spmv_k3, a.NN, kSpmvK3Rule);
 }
 template <class VT>
-int step3_blocks(int NN) {
-  return split_grid(NN, row_split<VT>(NN, kStep3Rule));
+int step3_blocks(int NN, int num_sms) {
+  return split_grid(NN, row_split<VT>(NN, kStep3Rule, num_sms));
 }
-template int step3_blocks<double>(int);
-template int step3_blocks<float>(int);
+template int step3_blocks<double>(int, int);
+template int step3_blocks<float>(int, int);
 int pupdate_blocks(int NNp, int num_sms) { return ew_grid(NNp) < num_sms * 4 ? ew_grid(NNp) : num_sms * 4; }
 cudaError_t launch_pressure_update(int NNp, double dt, const double* pn, const double* pdot, const double* pprev,
                                    double* pnp1, double* part, int nblocks, cudaStream_t s) {
@@ -668,8 +667,8 @@ template cudaError_t launch_step1<double>(const Step1Args<double>&, int, cudaStr
 template cudaError_t launch_step1<float>(const Step1Args<float>&, int, cudaStream_t);
 template cudaError_t launch_gt<double>(const GtArgs<double>&, int, cudaStream_t);
 template cudaError_t launch_gt<float>(const GtArgs<float>&, int, cudaStream_t);
-template cudaError_t launch_step3<double>(const Step3Args<double>&, cudaStream_t);
-template cudaError_t launch_step3<float>(const Step3Args<float>&, cudaStream_t);
+template cudaError_t launch_step3<double>(const Step3Args<double>&, int, cudaStream_t);
+template cudaError_t launch_step3<float>(const Step3Args<float>&, int, cudaStream_t);
 template cudaError_t launch_spmv_k3<double>(const SpmvK3Args<double>&, int, cudaStream_t);
 template cudaError_t launch_spmv_k3<float>(const SpmvK3Args<float>&, int, cudaStream_t);
 template cudaError_t launch_csr_to_sell<double>(int, const int*, const double*, const int*, double*, cudaStream_t);
