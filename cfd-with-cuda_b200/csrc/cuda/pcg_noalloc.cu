@@ -14,8 +14,8 @@
 // Limits and rules:
 //   - n <= CFD_NOALLOC_MAX_N (524288 rows, a 80^3 pressure grid); larger
 //     systems are rejected with CFD_E_BADARG and a message.
-//   - every GPU that loads this library holds the array (4.1 MiB) until the
-//     process exits;
+//   - every GPU that calls it holds the array (4.1 MiB; with fewer than 103 SMs 12 MiB
+//     more) until the process exits;
 //   - the first call on a device looks the array's device address up
 //     (cudaGetSymbolAddress, once per device, with that device current); make
 //     that first call before any stream capture;
@@ -33,7 +33,10 @@
 // lengths come from (r, u) and (w, u) of the same iteration, so one reduction
 // and one publication of u are the only grid-wide waits.  Everything but u
 // is used by the block that owns the rows only and stays in its shared
-// memory: r, p, s, w and x.
+// memory: r, p, s, w and x.  A device or partition whose SMs cannot hold them (fewer
+// than 103 for the largest n) keeps p, s and w in a second array (pcg_noalloc_spill.cu),
+// x in the caller's vector, and publishes r, from which u = D^-1 r is formed
+// where it is read.
 //
 // What bounds it: the matrix stream (12 bytes per non-zero; up to about 9 M
 // non-zeros it stays in L2 between iterations) and the two waits.  One block
@@ -48,13 +51,20 @@
 // read ahead.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
+#include <cstdlib>
 #include <mutex>
 
 #include "../../../include/cfdfs.h"
 #include "common.cuh"
 
 namespace cfd {
+
+// Device address of 3 CFD_NOALLOC_MAX_N doubles, placed on the device by the first
+// call (pcg_noalloc_spill.cu).
+cudaError_t noalloc_spill(double** p);
+
 namespace {
 
 constexpr int kThreads = 1024;
@@ -63,12 +73,12 @@ constexpr int kMaxBlocks = 2048;
 constexpr int kMaxDevices = 64;
 // layout of the scratch array (bytes)
 constexpr size_t kVecBytes = (size_t)kMaxN * sizeof(double);
-constexpr size_t kOffU = 0;  // u; the other vectors live in shared memory
+constexpr size_t kOffU = 0;  // u (or r); the other vectors live in shared memory
 constexpr size_t kOffPart = kVecBytes;                                    // 6 x kMaxBlocks doubles
 constexpr size_t kOffCtl = kOffPart + 6 * (size_t)kMaxBlocks * sizeof(double);  // barrier[2], err, pad
 constexpr size_t kOffRes = kOffCtl + 256;                                       // 4 doubles
 constexpr size_t kScratchBytes = kOffRes + 256;
-constexpr int kMaxDynSmem = 200 * 1024;
+constexpr size_t kMaxDynSmem = 200 * 1024;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -160,11 +170,14 @@ __device__ __forceinline__ double ldg_stream(const double* p) {
 }
 
 // w = A u on the block's rows r0 .. r0 + nr, G lanes per row (w in shared
-// memory); returns the thread's part of (w, u).  u is read with plain loads:
-// other blocks' parts of it are visible after the grid-wide wait before.
-template <int G>
+// memory, or global with SPILL); returns the thread's part of (w, u).  u, or with SPILL
+// the r of u = D^-1 r, is read with plain loads: other blocks' parts of it are visible
+// after the grid-wide wait before.
+template <int G, bool SPILL>
 __device__ __forceinline__ double spmv_rows(int r0, int nr, const int* __restrict__ rp, const int* __restrict__ col,
-                                            const double* __restrict__ val, const double* u, double* w) {
+                                            const double* __restrict__ val, const double* __restrict__ dinv,
+                                            const double* u, double* w) {
+  auto at = [&](int i) { return SPILL ? u[i] * __ldg(dinv + i) : u[i]; };
   constexpr int R = 2, STEP = kThreads / G;  // rows per group at once, rows of a pass
   const int lane = threadIdx.x % G;
   double wu = 0;
@@ -203,30 +216,35 @@ __device__ __forceinline__ double spmv_rows(int r0, int nr, const int* __restric
       s[k] = 0;
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        if (c[k][q] >= 0) s[k] += v[k][q] * u[c[k][q]];
-      for (int j = b[k] + 4 * G; j < e[k]; j += G) s[k] += ldg_stream(val + j) * u[ldg_stream(col + j)];
+        if (c[k][q] >= 0) s[k] += v[k][q] * at(c[k][q]);
+      for (int j = b[k] + 4 * G; j < e[k]; j += G) s[k] += ldg_stream(val + j) * at(ldg_stream(col + j));
       s[k] = group_sum<G>(s[k]);
       const int i = base + sub + k * STEP;
       if (i < nr && lane == 0) {
         w[i] = s[k];
-        wu += u[r0 + i] * s[k];
+        wu += at(r0 + i) * s[k];
       }
     }
   }
   return wu;
 }
 
+template <bool SPILL>
 __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* __restrict__ rp,
                                                               const int* __restrict__ col,
                                                               const double* __restrict__ val,
                                                               const double* __restrict__ dinv,
                                                               const double* __restrict__ b, double* xout, double rtol,
-                                                              int maxit, unsigned char* scratch) {
+                                                              int maxit, unsigned char* scratch, double* spill) {
   extern __shared__ double sv[];
   const int r0 = (int)((long long)n * blockIdx.x / gridDim.x);
   const int nr = (int)((long long)n * (blockIdx.x + 1) / gridDim.x) - r0;
-  double *r = sv, *p = r + nr, *s = p + nr, *w = s + nr, *x = w + nr;
   double* u = reinterpret_cast<double*>(scratch + kOffU);
+  double* const r = SPILL ? u + r0 : sv;
+  double* const p = SPILL ? spill + r0 : r + nr;
+  double* const s = SPILL ? spill + kMaxN + r0 : p + nr;
+  double* const w = SPILL ? spill + 2 * (size_t)kMaxN + r0 : s + nr;
+  double* const x = SPILL ? xout + r0 : w + nr;
   double* result = reinterpret_cast<double*>(scratch + kOffRes);
   GridSync gs{reinterpret_cast<unsigned*>(scratch + kOffCtl), reinterpret_cast<int*>(scratch + kOffCtl + 8),
               reinterpret_cast<double*>(scratch + kOffPart), 0u};
@@ -237,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* _
     const double bi = b[r0 + i], ui = bi * dinv[r0 + i];
     r[i] = bi;
     p[i] = s[i] = x[i] = 0.0;
-    u[r0 + i] = ui;
+    if (!SPILL) u[r0 + i] = ui;
     ru += bi * ui;
     rr += bi * bi;
   }
@@ -248,15 +266,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* _
     if (!alive) { status = 3; break; }
     double v[3] = {ru, 0.0, rr};
     if (mean <= 8)
-      v[1] = spmv_rows<2>(r0, nr, rp, col, val, u, w);
+      v[1] = spmv_rows<2, SPILL>(r0, nr, rp, col, val, dinv, u, w);
     else if (mean <= 16)
-      v[1] = spmv_rows<4>(r0, nr, rp, col, val, u, w);
+      v[1] = spmv_rows<4, SPILL>(r0, nr, rp, col, val, dinv, u, w);
     else if (mean <= 32)
-      v[1] = spmv_rows<8>(r0, nr, rp, col, val, u, w);
+      v[1] = spmv_rows<8, SPILL>(r0, nr, rp, col, val, dinv, u, w);
     else if (mean <= 64)
-      v[1] = spmv_rows<16>(r0, nr, rp, col, val, u, w);
+      v[1] = spmv_rows<16, SPILL>(r0, nr, rp, col, val, dinv, u, w);
     else
-      v[1] = spmv_rows<32>(r0, nr, rp, col, val, u, w);
+      v[1] = spmv_rows<32, SPILL>(r0, nr, rp, col, val, dinv, u, w);
     if (!gs.wait<3>(v)) { status = 3; break; }
     const double gamma = v[0], delta = v[1];
     rn = sqrt(v[2]);
@@ -273,20 +291,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* _
     alpha_old = alpha;
     ru = rr = 0;
     for (int i = threadIdx.x; i < nr; i += kThreads) {
-      const double pi = u[r0 + i] + beta * p[i], si = w[i] + beta * s[i];
-      const double ri = r[i] - alpha * si, ui = ri * dinv[r0 + i];
+      const double di = dinv[r0 + i];
+      const double pi = (SPILL ? r[i] * di : u[r0 + i]) + beta * p[i], si = w[i] + beta * s[i];
+      const double ri = r[i] - alpha * si, ui = ri * di;
       p[i] = pi;
       s[i] = si;
       x[i] += alpha * pi;
       r[i] = ri;
-      u[r0 + i] = ui;
+      if (!SPILL) u[r0 + i] = ui;
       ru += ri * ui;
       rr += ri * ri;
     }
     its++;
     alive = gs.wait<0>(none);
   }
-  for (int i = threadIdx.x; i < nr; i += kThreads) xout[r0 + i] = x[i];
+  if (!SPILL)
+    for (int i = threadIdx.x; i < nr; i += kThreads) xout[r0 + i] = x[i];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     result[0] = its;
     result[1] = bnorm > 0 ? rn / bnorm : 0.0;
@@ -297,6 +317,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* _
 
 std::mutex g_setup_mutex;
 void* g_scratch_addr[kMaxDevices] = {};
+double* g_spill_addr[kMaxDevices] = {};
+
+size_t block_smem(int n, long long grid) { return 5 * sizeof(double) * (size_t)((n + grid - 1) / grid); }
 
 void put_err(char* buf, int len, const char* msg) {
   if (buf && len > 0) std::snprintf(buf, (size_t)len, "%s", msg);
@@ -326,39 +349,43 @@ extern "C" int cfd_pcg_solve_noalloc(const int* rowptr, const int* col, const do
     put_err(errbuf, errlen, "cfd_pcg_solve_noalloc: no current CUDA device");
     return CFD_E_CUDA;
   }
+  int sms = 0;
+  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // CFD_NOALLOC_SMS=<k>: as on a device of k SMs
+  if (const char* lim = std::getenv("CFD_NOALLOC_SMS")) sms = std::max(1, std::min(sms, std::atoi(lim)));
+  if (e != cudaSuccess || sms < 1) {
+    put_err(errbuf, errlen, "cfd_pcg_solve_noalloc: no SM count");
+    return CFD_E_CUDA;
+  }
+  sms = std::min(sms, kMaxBlocks);
   void* scratch = nullptr;
+  double* spill = nullptr;
   {
     std::lock_guard<std::mutex> lock(g_setup_mutex);
-    if (!g_scratch_addr[dev]) {
-      void* p = nullptr;
-      e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-      if (e != cudaSuccess || !p) {
-        std::snprintf(msg, sizeof(msg), "cfd_pcg_solve_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
-        put_err(errbuf, errlen, msg);
-        return CFD_E_CUDA;
-      }
-      g_scratch_addr[dev] = p;
+    e = cudaSuccess;
+    if (!g_scratch_addr[dev]) e = cudaGetSymbolAddress(&g_scratch_addr[dev], g_noalloc_scratch);
+    if (e == cudaSuccess && !g_spill_addr[dev] && block_smem(kMaxN, sms) > kMaxDynSmem)
+      e = noalloc_spill(&g_spill_addr[dev]);
+    if (e != cudaSuccess) {
+      std::snprintf(msg, sizeof(msg), "cfd_pcg_solve_noalloc: cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
+      put_err(errbuf, errlen, msg);
+      return CFD_E_CUDA;
     }
     scratch = g_scratch_addr[dev];
+    spill = g_spill_addr[dev];
   }
   cudaStream_t s = (cudaStream_t)stream;
   // one block per SM, at least 256 rows each: a small system waits on fewer
   // arrivals, and one block on none, so up to 512 rows stay on one (512 rows
   // of 27: 6.8 us per iteration, two blocks 9.2; 8000 rows: 9.5 us on 32
   // blocks, 11.3 on 16)
-  int sms = 0;
-  long long grid = 0;
-  size_t smem = 0;
-  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) {
-    grid = n <= 512 ? 1 : ((long long)n + 255) / 256;
-    if (grid > sms) grid = sms;
-    if (grid > kMaxBlocks) grid = kMaxBlocks;
-    if (grid < 1) grid = 1;
-    smem = 5 * sizeof(double) * (size_t)((n + grid - 1) / grid);
-    e = cudaFuncSetAttribute(k_pcg_noalloc, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
-  }
-  if (e != cudaSuccess || smem > kMaxDynSmem) {
+  const long long grid = std::min<long long>(sms, n <= 512 ? 1 : (n + 255) / 256);
+  size_t smem = block_smem(n, grid);
+  const bool in_smem = smem <= kMaxDynSmem;
+  const void* kernel = in_smem ? (const void*)k_pcg_noalloc<false> : (const void*)k_pcg_noalloc<true>;
+  if (!in_smem) smem = 0;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+  if (e != cudaSuccess) {
     put_err(errbuf, errlen, "cfd_pcg_solve_noalloc: the device cannot hold the block vectors");
     return CFD_E_CUDA;
   }
@@ -368,8 +395,8 @@ extern "C" int cfd_pcg_solve_noalloc(const int* rowptr, const int* col, const do
     int nn = n, mi = maxit;
     double rt = rtol;
     unsigned char* sp = base;
-    void* params[] = {&nn, (void*)&rowptr, (void*)&col, (void*)&val, (void*)&dinv, (void*)&b, (void*)&x, &rt, &mi, &sp};
-    e = cudaLaunchCooperativeKernel((const void*)k_pcg_noalloc, dim3((unsigned)grid), dim3(kThreads), params, smem, s);
+    void* params[] = {&nn, (void*)&rowptr, (void*)&col, (void*)&val, (void*)&dinv, (void*)&b, (void*)&x, &rt, &mi, &sp, &spill};
+    e = cudaLaunchCooperativeKernel(kernel, dim3((unsigned)grid), dim3(kThreads), params, smem, s);
   }
   double res[4] = {0, 0, 0, 0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(res, base + kOffRes, sizeof(res), cudaMemcpyDeviceToHost, s);

@@ -354,13 +354,14 @@ int cfd_selftest_wait_timeout(cfd_ctx* ctx, int timeout_ms);
  * arrays -- rowptr (n+1), col and val (nnz), dinv = 1/diag (n), b (n) and the
  * output x (n) -- are DEVICE pointers owned by the caller, on the caller's
  * stream (NULL = legacy default stream) and the current device.  Work
- * vectors live in one static device array of fixed size (4.1 MiB, held by
- * every GPU that loads the library until exit), so n is limited to
+ * vectors live in a static device array of fixed size (4.1 MiB; 16.1 MiB on a
+ * device or partition of fewer than 103 SMs, whose shared memory cannot hold the
+ * rest; held by every GPU that calls it until exit), so n is limited to
  * CFD_NOALLOC_MAX_N; larger n returns CFD_E_BADARG with a message in errbuf.
  * The first call on a device looks the array up (once per device); make it
  * before any stream capture.  With CUDA's lazy module loading (the default)
  * that first call is also when the array is placed on the device, so it
- * needs 4.1 MiB free: a host that reserves device memory for its own pool
+ * needs 4.1 (16.1) MiB free: a host that reserves device memory for its own pool
  * should make one warm-up call (any small system) before it does.  Calls share the array: calls that overlap on
  * the GPU race and must not be issued.  info (may be NULL) receives
  * {iterations, ||r||/||b||, status}; returns CFD_OK, CFD_E_NOCONV,
