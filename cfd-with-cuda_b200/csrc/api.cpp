@@ -2575,6 +2575,84 @@ int cfd_coarse_matrix(int device, const int dims[3], const int* rowptr, const in
   return hb == 0 ? CFD_OK : CFD_E_BADINPUT;
 }
 
+namespace {
+
+// The give-up paths of the persistent solves: both forms of the by-offsets CG and the
+// allocation-free CG on a tridiagonal system, first with a wait whose event never
+// comes (status 3 after the time limit), then as usual (the solution).
+int selftest_solves(cfd_ctx* c, unsigned long long timeout_ns) {
+  cudaStream_t s = c->stream;
+  for (int slices : {2, 13}) {  // per block: the reductions beside the products, and after them
+    const int grid = 4, ns = grid * slices, n = 32 * ns - 5;
+    std::vector<double> coef(dia_elems(n, 3), 0.0), b(n), x(n), val;
+    std::vector<int> rp(n + 1, 0), col;
+    for (int i = 0; i < n; i++) {
+      b[i] = 1.0 + (i % 7);
+      for (int t = 0; t < 3; t++) {
+        const int j = i + t - 1;
+        if (j < 0 || j >= n) continue;
+        const double v = t == 1 ? 2.5 : -1.0;
+        coef[((size_t)(i / 32) * 3 + t) * 32 + i % 32] = v;
+        col.push_back(j);
+        val.push_back(v);
+      }
+      rp[i + 1] = (int)col.size();
+    }
+    DevBuf<double> dcoef, dval, db, dx, ddinv, work, part, res;
+    DevBuf<int> doff, drp, dcol, err;
+    DevBuf<unsigned> sync;
+    CU(upload(dcoef, coef, s));
+    CU(upload(dval, val, s));
+    CU(upload(db, b, s));
+    CU(upload(ddinv, std::vector<double>(n, 1.0 / 2.5), s));
+    CU(upload(doff, std::vector<int>{-1, 0, 1}, s));
+    CU(upload(drp, rp, s));
+    CU(upload(dcol, col, s));
+    CU(dx.alloc(n));
+    CU(work.alloc(2 * (size_t)n));
+    CU(part.alloc(8 * grid));
+    CU(sync.alloc(1 + grid));
+    CU(err.alloc(1));
+    CU(res.alloc(4));
+    auto wrong = [&]() {  // || b - A x || against || b ||
+      double r2 = 0, b2 = 0;
+      for (int i = 0; i < n; i++) {
+        const double r = b[i] - 2.5 * x[i] + (i > 0 ? x[i - 1] : 0.0) + (i + 1 < n ? x[i + 1] : 0.0);
+        r2 += r * r;
+        b2 += b[i] * b[i];
+      }
+      return !(r2 <= 1e-18 * b2);
+    };
+    for (int which = 0; which < 3; which++) {  // neighbours' phase, arrivals of the sums, neither
+      CU(cudaMemsetAsync(sync.p, 0, sync.bytes(), s));
+      CU(cudaMemsetAsync(err.p, 0, sizeof(int), s));
+      PcgDiaArgs a{};
+      a.d = DiaArgs{n, 3, 1, doff.p, dcoef.p};
+      a.dinv = ddinv.p; a.b = db.p; a.x = dx.p; a.mb = work.p; a.part = part.p; a.sync = sync.p; a.err = err.p;
+      a.rtol = 1e-10; a.maxit = 200; a.result = res.p; a.timeout_ns = timeout_ns;
+      a.nb_extra = which == 0 ? 1u << 20 : 0;
+      a.red_extra = which == 1 ? 1 : 0;
+      KL(CFD_K_PCG64, launch_pcg_dia(a, grid, 0, s));
+      CU(cudaMemcpyAsync(c->h_small, res.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
+      CU(cudaMemcpyAsync(x.data(), dx.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+      CU(cudaStreamSynchronize(s));
+      const int st = (int)c->h_small[2];
+      if (which < 2 ? st != 3 : st != 0 || wrong())
+        return fail(c, CFD_E_CUDA, "self-test: by-offsets solve (%d slices, wait %d) ended with status %d", slices,
+                    which, st);
+      double nst = -1;
+      KL(CFD_K_PCG64, noalloc_selftest(which, timeout_ns, drp.p, dcol.p, dval.p, ddinv.p, db.p, dx.p, n, &nst, s));
+      CU(cudaMemcpyAsync(x.data(), dx.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+      CU(cudaStreamSynchronize(s));
+      if (which < 2 ? nst != 3 : nst != 0 || wrong())
+        return fail(c, CFD_E_CUDA, "self-test: allocation-free solve (wait %d) ended with status %g", which, nst);
+    }
+  }
+  return CFD_OK;
+}
+
+}  // namespace
+
 int cfd_selftest_wait_timeout(cfd_ctx* c, int timeout_ms) {
   if (!c || timeout_ms <= 0 || timeout_ms > 10000) return CFD_E_BADARG;
   PoolScope scope(&c->pool);
@@ -2588,8 +2666,10 @@ int cfd_selftest_wait_timeout(cfd_ctx* c, int timeout_ms) {
   int h[2] = {0, 0};
   CU(cudaMemcpyAsync(h, flags.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
-  if (h[1]) return fail(c, CFD_E_TIMEOUT, "bounded wait gave up after %d ms (self-test)", timeout_ms);
-  return CFD_OK;
+  if (!h[1]) return CFD_OK;
+  rc = selftest_solves(c, (unsigned long long)std::min(timeout_ms, 200) * 1000000ULL);
+  if (rc) return rc;
+  return fail(c, CFD_E_TIMEOUT, "bounded wait gave up after %d ms (self-test)", timeout_ms);
 }
 
 int cfd_unet_create(cfd_unet** out, int device, unsigned long long seed) {

@@ -211,6 +211,8 @@ struct PcgDiaArgs {
   int maxit, warm;
   double* result;
   unsigned long long timeout_ns;
+  // 0; a self-test lets the waits run out: phases and arrivals beyond those that come
+  unsigned nb_extra, red_extra;
 };
 int pcg_dia_grid(int n, int device);
 // Blocks of the one-cluster form of the solve (0: the matrix does not fit the
@@ -471,6 +473,11 @@ cudaError_t launch_csr_to_sell(int nrows, const int* rp, const double* csr, cons
 cudaError_t launch_sell_widths(int nrows, const int* rp, int* width, cudaStream_t s);
 cudaError_t launch_sell_cols(int nrows, const int* rp, const int* col, const int* off, int* scol, cudaStream_t s);
 
+// The allocation-free solve (pcg_noalloc.cu) on a tridiagonal system, with arrivals that
+// never come at the wait for u (which = 0) or for the sums (1), or none (2): its status
+// word, 3 where a wait gave up.
+cudaError_t noalloc_selftest(int which, unsigned long long timeout_ns, const int* rp, const int* col, const double* val,
+                             const double* dinv, const double* b, double* x, int n, double* status, cudaStream_t s);
 cudaError_t launch_wait_selftest(const int* flag, int* err, unsigned long long timeout_ns, cudaStream_t s);
 
 // layout conversion between the reference's [u|v|w] blocks and double4 nodes

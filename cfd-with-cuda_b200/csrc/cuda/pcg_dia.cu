@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
   for (int i = 0;; i++) {
     if (rows) {
       // n_i = Z m_i  (neighbours' m_i published at phase i + 2)
-      if (alive) alive = bs.wait_nb<BESIDE ? 32 * PROD : 0>((unsigned)i + 2);
+      if (alive) alive = bs.wait_nb<BESIDE ? 32 * PROD : 0>((unsigned)i + 2 + a.nb_extra);
       if (alive)
         M.multiply(warp, lane, mb[i & 1], c);
       else if (threadIdx.x == 0)
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kDiaThreads, 1) k_pcg_dia(PcgDiaArgs a) {
     if (sums) {
       // reduction of iteration i, posted before the SpMV
       double red[4];
-      const bool ok = bs.warp_red<4>((unsigned)(i + 1) * (unsigned)G, a.part + (size_t)(i & 1) * 4 * G, red);
+      const bool ok = bs.warp_red<4>((unsigned)(i + 1) * (unsigned)G + a.red_extra, a.part + (size_t)(i & 1) * 4 * G, red);
       if (i == 0) {
         bnorm = sqrt(red[3]);
         tol = a.rtol * bnorm;

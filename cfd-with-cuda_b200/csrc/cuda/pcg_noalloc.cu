@@ -79,6 +79,7 @@ constexpr size_t kOffCtl = kOffPart + 6 * (size_t)kMaxBlocks * sizeof(double);  
 constexpr size_t kOffRes = kOffCtl + 256;                                       // 4 doubles
 constexpr size_t kScratchBytes = kOffRes + 256;
 constexpr size_t kMaxDynSmem = 200 * 1024;
+constexpr unsigned long long kTimeoutNs = 2000000000ULL;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -91,6 +92,8 @@ struct GridSync {
   unsigned* cnt;
   int* err;
   double* part;
+  unsigned long long timeout_ns;
+  unsigned extra[2];  // 0; a self-test's arrivals that never come [wait<0>, wait<3>]
   unsigned k;
   template <int NV>
   __device__ __forceinline__ bool wait(double (&v)[NV > 0 ? NV : 1]) {
@@ -124,12 +127,12 @@ struct GridSync {
         red_add_release_u32(cnt, 1u);
       }
       __syncwarp();
-      const unsigned target = k * (unsigned)G;
+      const unsigned target = k * (unsigned)G + extra[NV > 0];
       int ok = 1;
       if (ld_acquire_u32(cnt) < target) {
         const unsigned long long t0 = global_ns();
         while (ld_acquire_u32(cnt) < target) {
-          if (ld_volatile_i32(err) || global_ns() - t0 > 2000000000ULL) {
+          if (ld_volatile_i32(err) || global_ns() - t0 > timeout_ns) {
             ok = 0;
             break;
           }
@@ -235,7 +238,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* _
                                                               const double* __restrict__ val,
                                                               const double* __restrict__ dinv,
                                                               const double* __restrict__ b, double* xout, double rtol,
-                                                              int maxit, unsigned char* scratch, double* spill) {
+                                                              int maxit, unsigned char* scratch, double* spill,
+                                                              unsigned long long timeout_ns, unsigned extra0,
+                                                              unsigned extra1) {
   extern __shared__ double sv[];
   const int r0 = (int)((long long)n * blockIdx.x / gridDim.x);
   const int nr = (int)((long long)n * (blockIdx.x + 1) / gridDim.x) - r0;
@@ -247,7 +252,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(int n, const int* _
   double* const x = SPILL ? xout + r0 : w + nr;
   double* result = reinterpret_cast<double*>(scratch + kOffRes);
   GridSync gs{reinterpret_cast<unsigned*>(scratch + kOffCtl), reinterpret_cast<int*>(scratch + kOffCtl + 8),
-              reinterpret_cast<double*>(scratch + kOffPart), 0u};
+              reinterpret_cast<double*>(scratch + kOffPart), timeout_ns, {extra0, extra1}, 0u};
   // lanes per row: about four loads per lane for a row of the mean length
   const int mean = (int)(((long long)__ldg(rp + n) - __ldg(rp)) / n);
   double ru = 0, rr = 0, none[1];
@@ -326,6 +331,32 @@ void put_err(char* buf, int len, const char* msg) {
 }
 
 }  // namespace
+
+cudaError_t noalloc_selftest(int which, unsigned long long timeout_ns, const int* rp, const int* col, const double* val,
+                             const double* dinv, const double* b, double* x, int n, double* status, cudaStream_t s) {
+  void* p = nullptr;
+  cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+  if (e != cudaSuccess) return e;
+  unsigned char* base = static_cast<unsigned char*>(p);
+  const int grid = 4;
+  double rtol = 1e-10;
+  int maxit = 200;
+  double* spill = nullptr;
+  unsigned extra[2] = {which == 0 ? 1u : 0u, which == 1 ? 1u : 0u};
+  void* params[] = {&n, (void*)&rp, (void*)&col, (void*)&val, (void*)&dinv, (void*)&b, (void*)&x,
+                    &rtol, &maxit, &base, &spill, &timeout_ns, &extra[0], &extra[1]};
+  e = cudaFuncSetAttribute(k_pcg_noalloc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem);
+  if (e == cudaSuccess) e = cudaMemsetAsync(base + kOffCtl, 0, 256, s);
+  if (e == cudaSuccess)
+    e = cudaLaunchCooperativeKernel((const void*)k_pcg_noalloc<false>, dim3(grid), dim3(kThreads), params,
+                                    block_smem(n, grid), s);
+  double res[4] = {0, 0, -1, 0};
+  if (e == cudaSuccess) e = cudaMemcpyAsync(res, base + kOffRes, sizeof(res), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  *status = res[2];
+  return e;
+}
+
 }  // namespace cfd
 
 extern "C" int cfd_pcg_solve_noalloc(const int* rowptr, const int* col, const double* val, const double* dinv,
@@ -395,7 +426,10 @@ extern "C" int cfd_pcg_solve_noalloc(const int* rowptr, const int* col, const do
     int nn = n, mi = maxit;
     double rt = rtol;
     unsigned char* sp = base;
-    void* params[] = {&nn, (void*)&rowptr, (void*)&col, (void*)&val, (void*)&dinv, (void*)&b, (void*)&x, &rt, &mi, &sp, &spill};
+    unsigned long long timeout_ns = kTimeoutNs;
+    unsigned none = 0;
+    void* params[] = {&nn, (void*)&rowptr, (void*)&col, (void*)&val, (void*)&dinv, (void*)&b, (void*)&x,
+                      &rt, &mi, &sp, &spill, &timeout_ns, &none, &none};
     e = cudaLaunchCooperativeKernel(kernel, dim3((unsigned)grid), dim3(kThreads), params, smem, s);
   }
   double res[4] = {0, 0, 0, 0};

@@ -342,8 +342,12 @@ int cfd_coarse_matrix(int device, const int dims[3], const int* rowptr, const in
                       double spacing, int* cd, double* zc);
 
 /* Runs one small kernel whose bounded wait watches a flag nothing sets, with
- * the given limit in milliseconds.  Returns CFD_E_TIMEOUT when the wait gave
- * up as designed (the context stays usable), CFD_OK otherwise. */
+ * the given limit in milliseconds, then the persistent pressure solves and the
+ * allocation-free solve on a small system with events that never come (limit
+ * at most 200 ms each) and again as usual.  Returns CFD_E_TIMEOUT when every
+ * wait gave up as designed (the context stays usable), CFD_OK when the first
+ * did not, CFD_E_CUDA with a message when a solve ended in another way.  Not to be
+ * called while cfd_pcg_solve_noalloc runs on the device. */
 int cfd_selftest_wait_timeout(cfd_ctx* ctx, int timeout_ms);
 
 /* ---- pressure solve that allocates nothing ----------------------------------
