@@ -525,7 +525,9 @@ size_t stencil_elems(int n) { return (size_t)((n + 31) >> 5) * 125 * 32; }
 // of the matrix.  us per SpMV at 0 / 0.1 / 0.2 / 0.4 / 0.6: 24.6 / 23.6 / 24.0 /
 // 25.2 / 26.6 on the 65^3 grid (137 MB, inverse 48 MB), 16.0 / 16.0 / 14.7 /
 // 14.7 / 14.3 on 161 x 25 x 25 (50 MB, 8 MB), 16.1 / 16.1 / 14.9 / 14.6 / 14.7
-// on 49^3 (59 MB, 10 MB).
+// on 49^3 (59 MB, 10 MB): kernel times of the run, one kernel starting while the
+// one before it drains.  With events around every launch, as cfd_profile takes them,
+// nothing overlaps and the events count too: 32.7 on the 65^3 grid.
 float stencil_keep_fraction(int n, double inv_bytes) {
   const double bytes = (double)stencil_elems(n) * sizeof(float);
   return (float)std::max(0.0, std::min(0.6, (70e6 - inv_bytes) / bytes));

@@ -43,25 +43,26 @@ inline int rows_grid(long long rows) {
 // cavities of n^3 elements (velocity slices: 154, 1123, 3676, 8582, 16 600,
 // 22 000 and 67 000 for n = 8, 16, 24, 32, 40, 44, 64; pressure slices: 23,
 // 154, 489, 1124, 2154, 2848, 8583):
-//              n = 8                n = 16           n = 24           n = 32 (40 FP32)    n = 44 (64 FP32)
+//                n = 8                n = 16              n = 24              n = 32 (40 FP32)    n = 44 (64 FP32)
 //   FP64
-//   k_step1    31 / 28 / 17 / 10    74/62/34/21      81/70/45/50      97 / 89 / 93 / 107  205/217/230/273
-//   k_spmv_k3  32 / 18 / 10 / 6.3   71/37/20/14      74/43/30/30      89 / 61 / 59 / 63   144/144/146/152
-//   k_step3    7.6/ 7.1/ 5.2/ 4.3   23/13/7.9/6.5    30/19/15/20      32 / 32 / 34 / 46   72/70/80/107
-//   k_gt       57 / 30 / 17 / 9.6   114/59/31/17     146/72/38/22     142 / 73 / 41 / 28  148/84/87/72
+//   k_step1      23 / 17 / 11 / 7.1   47 / 36 / 21 / 15   59 / 48 / 39 / 41   80 / 82 / 80 / 93   185/200/204/237
+//   with K Acc   36 / 20 / 12 / 9.4   54 / 43 / 29 / 23   85 / 69 / 59 / 62   114/132/126/142     280/326/315/356
+//   k_spmv_k3    18 / 18 / 10 / 6.3   38 / 37 / 20 / 14   45 / 42 / 30 / 30   63 / 62 / 60 / 63   137/143/146/152
+//   k_step3      9.1/ 7.0/ 5.1/ 4.4   19 / 13 / 8.1/ 6.7  24 / 18 / 15 / 20   36 / 32 / 35 / 46   70/ 71/ 81/108
+//   k_gt         44 / 22 / 12 / 7.2   81 / 41 / 22 / 12   103/ 50 / 28 / 17   104/ 55 / 33 / 26   109/ 67/ 73/ 62
 //   FP32
-//   k_step1    18 / 16 / 11 / 8.2   37/33/20/21      43/43/47/67      93 / 163 / 192 / 297
-//   k_spmv_k3  16 / 14 / 9.2 / 7.0  36/30/17/13      39/33/29/40      59 / 108 / 118 / 170
-//   k_step3    8.7/ 6.1/ 4.8/ 4.3   17/9.8/7.0/10    20/14/18/25      40 / 52 / 67 / 107
-//   k_gt       30 / 24 / 13 / 8.3   60/46/25/14      72/55/30/17      75 / 58 / 37 / 37   114/130/122/131
-// (taken before the loads were ordered as at for_entries, which moved both sides
-// of each line alike: at the chosen split, FP64 n = 8 step 1 10 -> 7.2, n = 32
-// k_gt 28 -> 26, FP32 n = 24 k_spmv_k3 29 -> 24)
-// and k_gt in FP64 at n = 64 193 / 188 / 191 / 187, in FP32 on the duct of 24
-// x 24 x 160 (3145 slices) 78 / 63 / 63 / 53.
+//   k_step1      20 / 11 / 8.1/ 7.5   39 / 21 / 15 / 16   45 / 33 / 35 / 51   95 /126/144/227     373/495/583/929
+//   with K Acc   19 / 16 / 11 / 10    37 / 30 / 22 / 22   46 / 52 / 54 / 68   118/197/218/297     474/758/850/1190
+//   k_spmv_k3    16 / 9.9/ 7.3/ 6.2   35 / 19 / 12 / 11   39 / 26 / 24 / 33   60 / 92 / 96 /140   223/346/373/556
+//   k_step3      8.4/ 6.2/ 4.9/ 4.4   15 / 9.7/ 7.2/ 11   19 / 14 / 18 / 26   39 / 51 / 67 /107   160/197/257/424
+//   k_gt         26 / 23 / 13 / 7.8   55 / 46 / 24 / 14   65 / 52 / 28 / 16   67 / 57 / 36 / 37   112/126/127/129
+// and k_gt in FP64 at n = 64 180 / 174 / 173 / 172, in FP32 on the duct of 24
+// x 24 x 160 (3145 slices) 70 / 60 / 61 / 52.  One rule serves step 1 with and without K
+// Acc_prev; with it the FP64 line would lie a little lower (n = 32: 114 unsplit, 132
+// as chosen).
 struct SplitRule {
   int fp64, fp32;  // warps per SM
-  int least32;           // least FP32 split that pays (below it: 1)
+  int least32;     // least FP32 split that pays (below it: 1)
 };
 constexpr SplitRule kStep1Rule{128, 32, 2}, kSpmvK3Rule{256, 100, 2}, kStep3Rule{128, 50, 2}, kGtRule{512, 192, 8};
 template <class VT>
