@@ -79,7 +79,10 @@ typedef struct {
                         a node) with plain adds instead of FP64 atomics, so
                         repeated runs are bitwise identical, as the
                         reference's coloured assembly (CUDAcodes.cu:915-936);
-                        0 (default): one launch over all elements, atomics */
+                        0 (default): one launch over all elements, atomics:
+                        FP64 results repeat to rounding; CFD_MIXED adds the
+                        convection term in FP32 and its pressures repeat to
+                        about 1e-6 (one inner iteration more or less) */
 } cfd_options;
 
 typedef struct {
